@@ -244,6 +244,8 @@ static uint64_t wait_timeout_ns() {
 
 // ---- planner ----------------------------------------------------------------
 
+constexpr uint64_t kWalkMinBytes = 16ull << 20;
+
 enum class Method { Auto, BS, Pttwac, Stash, TwoPass, Cycles, Staged, Resident };
 
 TuneParams &tune_params() {
@@ -417,6 +419,19 @@ static bool do_0100(cudaStream_t s, void *buf, int e, uint64_t T, uint64_t a,
                   "memory (or the stream is being captured)",
                   (unsigned long long)T, (unsigned long long)a,
                   (unsigned long long)B, (unsigned long long)b);
+  }
+  // longer cycles of units of 64 bytes and more, cut into segments
+  if (m == Method::Auto && T * a * B * U >= kWalkMinBytes &&
+      !getenv("LM_NO_WALK") && walk_applies(buf, T, a, B, U)) {
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    cudaStreamIsCapturing(s, &cs);
+    Scratch sc, list;
+    if (try_scratch(sc, walk_scratch_bytes(buf, T, a, B, U), s) &&
+        try_scratch(list, cycle_scratch_bytes(a, B), s))
+      return check_launch(
+          launch_walk100(s, buf, T, a, B, U, sc.p, list.p,
+                         cs == cudaStreamCaptureStatusNone),
+          "walk launch");
   }
   // the stash wavefront spreads rows over all CTAs: with too few rows per
   // SM its steps are too small to keep HBM busy

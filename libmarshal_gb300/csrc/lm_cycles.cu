@@ -179,8 +179,9 @@ cudaError_t launch_move(cudaStream_t s, char *base, uint64_t T,
   return cudaGetLastError();
 }
 
-// Cycle leaders depend only on (a, B): lists computed outside stream capture
-// are kept per device (the first kCacheEntries shapes, kCacheBytes in all,
+// Cycle leaders depend only on (a, B) and which cycles they stand for (kind:
+// 0 for all of them, k > 0 for those that hold no start of lm_walk.cu's
+// blocks of 2^k positions): lists computed outside stream capture are kept per device (the first kCacheEntries shapes, kCacheBytes in all,
 // until lm_marshal_finalize) and reused; a later call on another stream
 // waits for the producing kernel.
 constexpr int kCacheEntries = 16;
@@ -191,7 +192,7 @@ struct CycEntry {
   cudaEvent_t ready = nullptr;
 };
 std::mutex g_cyc_mu;
-std::map<std::tuple<int, uint64_t, uint64_t>, CycEntry> g_cyc;
+std::map<std::tuple<int, uint64_t, uint64_t, uint32_t>, CycEntry> g_cyc;
 
 }  // namespace
 
@@ -215,11 +216,8 @@ size_t cycle_scratch_bytes(uint64_t A, uint64_t B) {
 }
 
 static cudaError_t run_leaders(cudaStream_t s, uint32_t a, const ModM &m,
-                               uint32_t L, bool w32, void *mem) {
-  uint32_t *count = reinterpret_cast<uint32_t *>(mem);
-  uint32_t *list = reinterpret_cast<uint32_t *>((char *)mem + 256);
-  cudaError_t err = cudaMemsetAsync(count, 0, sizeof(uint32_t), s);
-  if (err != cudaSuccess) return err;
+                               uint32_t L, bool w32, uint32_t *list,
+                               uint32_t *count) {
   const DeviceInfo &di = device_info();
   const uint64_t want = (m.M + kCycThreads - 1) / kCycThreads;
   const unsigned grid =
@@ -232,20 +230,25 @@ static cudaError_t run_leaders(cudaStream_t s, uint32_t a, const ModM &m,
   return cudaGetLastError();
 }
 
-// The leader list of 100(a, B): from the cache, or computed into a new
-// cache entry, or (during stream capture, or with the cache full) computed
-// into `scratch`.
-static cudaError_t leaders_for(cudaStream_t s, uint32_t a, uint32_t B,
-                               const ModM &m, uint32_t L, bool w32,
-                               void *scratch, bool may_cache, void **mem) {
+// See lm_internal.h.
+cudaError_t cycle_list_for(
+    cudaStream_t s, uint64_t a, uint64_t B, uint32_t kind, void *scratch,
+    bool may_cache, void **mem,
+    const std::function<cudaError_t(uint32_t *, uint32_t *)> &find) {
+  auto find_into = [&](void *p) {
+    uint32_t *count = reinterpret_cast<uint32_t *>(p);
+    const cudaError_t err = cudaMemsetAsync(count, 0, sizeof(uint32_t), s);
+    if (err != cudaSuccess) return err;
+    return find(reinterpret_cast<uint32_t *>((char *)p + 256), count);
+  };
   auto into_scratch = [&]() {
     *mem = scratch;
-    return run_leaders(s, a, m, L, w32, scratch);
+    return find_into(scratch);
   };
   if (!may_cache) return into_scratch();
   int dev = 0;
   cudaGetDevice(&dev);
-  const auto key = std::make_tuple(dev, (uint64_t)a, (uint64_t)B);
+  const auto key = std::make_tuple(dev, a, B, kind);
   std::lock_guard<std::mutex> lock(g_cyc_mu);
   auto it = g_cyc.find(key);
   if (it != g_cyc.end()) {
@@ -273,7 +276,7 @@ static cudaError_t leaders_for(cudaStream_t s, uint32_t a, uint32_t B,
     cudaFreeAsync(en.mem, s);
     return err;
   }
-  if ((err = run_leaders(s, a, m, L, w32, en.mem)) != cudaSuccess ||
+  if ((err = find_into(en.mem)) != cudaSuccess ||
       (err = cudaEventRecord(en.ready, s)) != cudaSuccess) {
     cudaFreeAsync(en.mem, s);
     cudaEventDestroy(en.ready);
@@ -313,7 +316,11 @@ cudaError_t launch_cycles100(cudaStream_t s, void *buf, int e, uint64_t T,
   const uint32_t U = b * (uint32_t)e;
   const bool w32 = (uint64_t)a * (M - 1) < (1ull << 32);
   void *mem = nullptr;
-  cudaError_t err = leaders_for(s, a, B, m, L, w32, scratch, may_cache, &mem);
+  cudaError_t err = cycle_list_for(
+      s, a, B, 0, scratch, may_cache, &mem,
+      [&](uint32_t *list, uint32_t *count) {
+        return run_leaders(s, a, m, L, w32, list, count);
+      });
   if (err != cudaSuccess) return err;
   const uint32_t *count = reinterpret_cast<const uint32_t *>(mem);
   const uint32_t *list =
