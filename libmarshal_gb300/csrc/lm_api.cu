@@ -87,7 +87,8 @@ int prepare_launch(const void *kern, LaunchCache &c, size_t smem, int threads,
   cudaGetDevice(&dev);
   const int d = dev & 7;
   const int need = (int)smem + 1;
-  if (need > 48 * 1024 + 1 && c.smem_set[d].load(std::memory_order_acquire) < need) {
+  // (the 48 KB that need no attribute hold the static shared memory too)
+  if (need > 40 * 1024 && c.smem_set[d].load(std::memory_order_acquire) < need) {
     if ((*err = cudaFuncSetAttribute(kern,
                                      cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      (int)smem)) != cudaSuccess)

@@ -88,6 +88,14 @@ struct BJob {
   // 8-byte elements) the output rows allow (store_b1_vecc), 0 for none; vrw = staged rows per output vector
   // of either store (their groups are shifted in the stage), 0 for none
   uint32_t vb1, vbc, vrw;
+  // 1- and 2-byte elements whose output rows start anywhere: ragged 1 =
+  // store_b1_ragged (blocks stage `extra` rows more than S), 2 =
+  // store_b1_flat (blocks of whole columns), 0 = none; contig = blocks of
+  // whole rows staged as the one range that they are, row r at r * row
+  // bytes; tab = words of a block's table of row offsets
+  uint8_t ragged, contig;
+  uint16_t extra;
+  uint32_t tab;
 };
 
 struct BItem {
@@ -714,6 +722,179 @@ __device__ __forceinline__ void store_b1_vecc(const unsigned char *buf,
   }
 }
 
+// store_b1 for 1- and 2-byte elements whose output rows start anywhere.
+// Element by element this is bound by write requests (one per 8 elements of a
+// column), and gathered byte by byte by instructions.  So an output run goes
+// out in whole 16-byte vectors of its own alignment: a block stages RW - 1
+// rows (RW = 16/E) more than its S, and its share of a column are the rows
+// from the first vector boundary at or after its first row to the first one
+// at or after its last; only the first and the last rows of the matrix leave
+// partial vectors, element by element.  A lane reads the 32-bit words of its
+// 4/E columns in the 2 RW rows from a group's first one on (two shared words
+// and a funnel shift each, as rows start on any byte), transposes them in
+// registers, and takes each column's vector out of its 32 bytes.  Eight
+// lanes take consecutive groups of rows (128 bytes of an output row), four
+// lanes consecutive words.
+// tab holds each row's offset in the stage, rounded down to words, RW rows and
+// 4 words of padding per group (the eight lanes' reads fall in distinct
+// banks), 0 for rows that are not there; its first word of padding holds the
+// first row's offset within 16.
+__device__ __forceinline__ uint32_t rag_index(uint32_t r, uint32_t e) {
+  return r + 4 * (r >> (5 - e));  // 2^(5-e) = RW for 1- and 2-byte elements
+}
+
+template <int E, bool CONTIG>
+__device__ __forceinline__ void store_b1_ragged(
+    const unsigned char *buf, const uint32_t *tab, uint32_t S, uint32_t nrows,
+    bool first, uint32_t ncols, typename Elem<E>::T *dst, uint32_t ostride,
+    uint32_t warp, uint32_t nwarps, uint32_t pitch, uint32_t rb) {
+  static_assert(E == 1 || E == 2, "narrow elements only");
+  using T = typename Elem<E>::T;
+  constexpr uint32_t RW = 16 / E, TW = RW + 4, CW = 4 / E;
+  const uint32_t lane = threadIdx.x & 31;
+  const uint32_t ng = S / RW;
+  const uint32_t nwc = (ncols + CW - 1) / CW;
+  // eight lanes on consecutive groups (four where there are no more)
+  const uint32_t lg = ng > 4 ? 3 : 2;
+  const uint32_t ngc = (ng + (1 << lg) - 1) >> lg;
+  const uint32_t nwd = (nwc + (32 >> lg) - 1) >> (5 - lg);
+  // bits of a row's first element past a word: the same every fourth row
+  const uint32_t m0 = CONTIG ? tab[0] : tab[RW];
+  const uint32_t sh0 = m0 * 8, sh1 = (m0 + rb) * 8, sh2 = (m0 + 2 * rb) * 8,
+                 sh3 = (m0 + 3 * rb) * 8;
+  for (uint32_t u = warp; u < ngc * nwd; u += nwarps) {
+    const uint32_t d = u / ngc, gc = u - d * ngc;
+    const uint32_t g = (gc << lg) + (lane & ((1 << lg) - 1));
+    const uint32_t wc = (d << (5 - lg)) + (lane >> lg);
+    if (g >= ng || wc >= nwc || g * RW >= nrows) continue;
+    uint32_t w[CW][8];  // 2 RW rows of each column
+    const uint32_t *tg = tab + g * TW;
+    const unsigned char *bw = buf + wc * 4;
+    auto word = [&](uint32_t off, uint32_t sh) {
+      const uint32_t *q = reinterpret_cast<const uint32_t *>(bw + off);
+      return __funnelshift_r(q[0], q[1], sh);
+    };
+    // rows without a table: the words of rows 0..3 of the group, a multiple
+    // of 4 bytes further on for each four rows
+    const uint32_t o0 = m0 + g * RW * pitch;
+    const uint32_t c0 = o0 & ~3u, c1 = (o0 + pitch) & ~3u,
+                   c2 = (o0 + 2 * pitch) & ~3u, c3 = (o0 + 3 * pitch) & ~3u;
+#pragma unroll
+    for (uint32_t q = 0; q < 8; ++q) {
+      if constexpr (E == 1) {
+        uint4 t;
+        if constexpr (CONTIG) {
+          const uint32_t st = q * 4 * pitch;
+          t = make_uint4(c0 + st, c1 + st, c2 + st, c3 + st);
+        } else {
+          t = *reinterpret_cast<const uint4 *>(tg + (q / 4) * TW + (q % 4) * 4);
+        }
+        const uint32_t a0 = word(t.x, sh0), a1 = word(t.y, sh1),
+                       a2 = word(t.z, sh2), a3 = word(t.w, sh3);
+        const uint32_t lo01 = __byte_perm(a0, a1, 0x5140);
+        const uint32_t hi01 = __byte_perm(a0, a1, 0x7362);
+        const uint32_t lo23 = __byte_perm(a2, a3, 0x5140);
+        const uint32_t hi23 = __byte_perm(a2, a3, 0x7362);
+        w[0][q] = __byte_perm(lo01, lo23, 0x5410);
+        w[1][q] = __byte_perm(lo01, lo23, 0x7632);
+        w[2][q] = __byte_perm(hi01, hi23, 0x5410);
+        w[3][q] = __byte_perm(hi01, hi23, 0x7632);
+      } else {
+        uint2 t;
+        if constexpr (CONTIG) {
+          const uint32_t st = (q / 2) * 4 * pitch;
+          t = q % 2 ? make_uint2(c2 + st, c3 + st) : make_uint2(c0 + st, c1 + st);
+        } else {
+          t = *reinterpret_cast<const uint2 *>(tg + (q / 4) * TW + (q % 4) * 2);
+        }
+        const uint32_t a0 = word(t.x, q % 2 ? sh2 : sh0),
+                       a1 = word(t.y, q % 2 ? sh3 : sh1);
+        w[0][q] = __byte_perm(a0, a1, 0x5410);
+        w[1][q] = __byte_perm(a0, a1, 0x7632);
+      }
+    }
+    unsigned char *run =
+        reinterpret_cast<unsigned char *>(dst + (uint64_t)(wc * CW) * ostride);
+#pragma unroll
+    for (uint32_t c = 0; c < CW; ++c, run += (uint64_t)ostride * E) {
+      const uint32_t h = (16 - ((uintptr_t)run & 15)) & 15;  // bytes
+      uint32_t x[6], y[5];
+#pragma unroll
+      for (int i = 0; i < 6; ++i) x[i] = h & 8 ? w[c][i + 2] : w[c][i];
+#pragma unroll
+      for (int i = 0; i < 5; ++i) y[i] = h & 4 ? x[i + 1] : x[i];
+      if (wc * CW + c < ncols && g * 16 + h + 16 <= nrows * E)
+        __stcg(reinterpret_cast<uint4 *>(run + g * 16 + h),
+               make_uint4(__funnelshift_r(y[0], y[1], h * 8),
+                          __funnelshift_r(y[1], y[2], h * 8),
+                          __funnelshift_r(y[2], y[3], h * 8),
+                          __funnelshift_r(y[3], y[4], h * 8)));
+    }
+  }
+  // the rows of the matrix before the first boundary and after the last
+  // (a block that stages fewer rows than S + RW - 1 ends with the matrix)
+  const bool end = nrows < S + RW - 1;
+  if (!first && !end) return;
+  for (uint32_t x = warp * 32 + lane; x < ncols * RW; x += nwarps * 32) {
+    const uint32_t jj = x / RW, k = x % RW;
+    T *run = dst + (uint64_t)jj * ostride;
+    const uint32_t h = (16 - (uint32_t)((uintptr_t)run & 15)) / E % RW;
+    auto put = [&](uint32_t r) {
+      const uint32_t off = CONTIG ? m0 + r * pitch
+                                  : tab[rag_index(r, E)] + ((m0 + r * rb) & 3);
+      __stcg(run + r, *reinterpret_cast<const T *>(buf + off + jj * E));
+    };
+    if (first && k < min(h, nrows)) put(k);
+    if (end && nrows > h) {
+      const uint32_t r = h + (nrows - h) / RW * RW + k;
+      if (r < nrows && r < S + h) put(r);
+    }
+  }
+}
+
+// For blocks of whole columns (S = a) the block's output is one
+// contiguous range of n = a * ncols elements, written in the 16-byte vectors
+// of its alignment whatever the column length; a vector's elements run down
+// a column and on into the next.
+template <int E>
+__device__ __forceinline__ void store_b1_flat(
+    const unsigned char *buf, uint32_t a, const FastDiv &div_a, uint32_t n,
+    typename Elem<E>::T *dst, uint32_t t, uint32_t nt, uint32_t pitch,
+    uint32_t rb, uint32_t m0) {
+  using T = typename Elem<E>::T;
+  constexpr uint32_t RW = 16 / E;
+  const uint32_t p = (uint32_t)((uintptr_t)dst & 15) / E;
+  const uint32_t np = (n + p + RW - 1) / RW;
+  for (uint32_t x = t; x < np; x += nt) {
+    const uint32_t o0 = x == 0 ? 0 : x * RW - p;  // first element
+    uint32_t jj = fdiv(o0, div_a);
+    uint32_t i = o0 - jj * a;
+    uint32_t off = i * pitch + 16 * (i / RW), m = m0 + i * rb;
+    auto next = [&]() {
+      const T v = *reinterpret_cast<const T *>(buf + off + (m & 15) + jj * E);
+      ++i;
+      off += pitch + (i % RW == 0 ? 16 : 0);
+      m += rb;
+      if (i == a) {
+        i = 0;
+        off = 0;
+        m = m0;
+        ++jj;
+      }
+      return v;
+    };
+    const uint32_t o1 = min(n, (x + 1) * RW - p);
+    if (o1 - o0 == RW) {
+      T v[RW];
+#pragma unroll
+      for (uint32_t k = 0; k < RW; ++k) v[k] = next();
+      __stcg(reinterpret_cast<uint4 *>(dst + o0), pack16<E>(v));
+    } else {
+      for (uint32_t o = o0; o < o1; ++o) __stcg(dst + o, next());
+    }
+  }
+}
+
 // Tiles larger than one CTA's shared memory, processed by persistent
 // clusters: rank 0 claims items and shares them through distributed shared
 // memory; each CTA stages a column band of the tile with bulk copies
@@ -940,6 +1121,7 @@ __global__ void __launch_bounds__(kBatchThreads, 2) k_batch_band(BatchArgs g) {
 constexpr int kStageThreads = 256;
 constexpr uint32_t kStageTileBytes = 32 * 1024;  // staged bytes per block
 constexpr uint32_t kStageMaxS = 256;             // rows per block
+constexpr uint32_t kRowTable = (kStageMaxS / 8 + 1) * 12;  // most words of a BJob::tab
 constexpr uint32_t kStageBlocksPerItem = 4;   // fine-grained: balanced tails
 constexpr uint64_t kCopyVecsPerItem = 16384;     // 256 KB
 // staged jobs in this range copy back with a kernel that drops each scratch
@@ -955,6 +1137,7 @@ struct GBlock {
   uint32_t t, i0, j0, si, sj;
 };
 
+template <bool RAG>
 __device__ __forceinline__ GBlock gather_decode(const BJob &j, uint32_t q) {
   GBlock k;
   k.t = fdiv(q, j.div_nIJ);
@@ -963,7 +1146,7 @@ __device__ __forceinline__ GBlock gather_decode(const BJob &j, uint32_t q) {
   const uint32_t bj = r - bi * j.nJ;
   k.i0 = bi * j.S;
   k.j0 = bj * j.Sj;
-  k.si = min(j.S, j.a - k.i0);
+  k.si = min(RAG ? j.S + j.extra : j.S, j.a - k.i0);
   k.sj = min(j.Sj, j.B - k.j0);
   return k;
 }
@@ -981,11 +1164,37 @@ struct RowCopy {
   uint32_t dst;    // offset in the stage
 };
 
+template <int NT, bool RAG>
 __device__ __forceinline__ RowCopy gather_row_plan(const BJob &j, uint32_t q,
                                                    uint32_t *rowoff) {
   RowCopy c{0, 0, 0};
-  const GBlock k = gather_decode(j, q);
-  const uint32_t r = (threadIdx.x & 31) * (kStageThreads / 32) + (threadIdx.x >> 5);
+  const GBlock k = gather_decode<RAG>(j, q);
+  if (RAG && j.contig) {
+    // one piece per warp of the block's range (its 16-byte superset)
+    const uintptr_t src = (uintptr_t)(j.base + ((uint64_t)k.t * j.tile_elems +
+                                                (uint64_t)k.i0 * j.row_elems) *
+                                                   j.e);
+    const uint32_t m0 = (uint32_t)(src & 15);
+    const uint32_t all = (m0 + k.si * j.pitch + 15) & ~15u;
+    const uint32_t piece = (all + NT / 2 - 1) / (NT / 2) * 16;
+    if (j.ragged == 1) {
+      if (threadIdx.x == 0) rowoff[0] = m0;
+    } else {
+      for (uint32_t r = threadIdx.x; r < k.si; r += NT)
+        rowoff[r] = m0 + r * j.pitch;
+    }
+    const uint32_t o = (threadIdx.x >> 5) * piece;
+    if ((threadIdx.x & 31) || o >= all) return c;
+    c.src = src - m0 + o;
+    c.bytes = min(piece, all - o);
+    c.dst = o;
+    return c;
+  }
+  const uint32_t r = (threadIdx.x & 31) * (NT / 32) + (threadIdx.x >> 5);
+  const uint32_t tr = RAG && j.ragged == 1 ? rag_index(r, j.e) : r;
+  if (RAG && j.ragged == 1) {
+    if (r >= k.si && tr < j.tab) rowoff[tr] = 0;
+  }
   if (r >= k.si) return c;
   const uint32_t len = k.sj * j.b * j.e;
   const uintptr_t src = (uintptr_t)(j.base + ((uint64_t)k.t * j.tile_elems +
@@ -997,7 +1206,9 @@ __device__ __forceinline__ RowCopy gather_row_plan(const BJob &j, uint32_t q,
   // per group (the shifts only grow, so rows never overlap), so the eight
   // consecutive groups a warp reads at once fall in distinct bank groups
   c.dst = r * j.pitch + (j.vrw ? 16 * (r / j.vrw) : 0);
-  rowoff[r] = c.dst + (uint32_t)(src - c.src);
+  const uint32_t m = (uint32_t)(src - c.src);
+  rowoff[tr] = c.dst + (RAG && j.ragged == 1 ? m & ~3u : m);
+  if (RAG && j.ragged == 1 && r == 0) rowoff[16 / j.e] = m;
   return c;
 }
 
@@ -1011,11 +1222,11 @@ __device__ __forceinline__ void gather_row_issue(const RowCopy &c,
 
 // All threads: output rows j0..j0+sj-1 of the block, each si*b elements
 // long, from the staged rows.
-template <int E>
+template <int E, int NT, bool RAG>
 __device__ void gather_store(const BJob &j, uint32_t q, const unsigned char *buf,
                              const uint32_t *rowoff) {
   using T = typename Elem<E>::T;
-  const GBlock k = gather_decode(j, q);
+  const GBlock k = gather_decode<RAG>(j, q);
   T *dst = reinterpret_cast<T *>(j.scratch) + (uint64_t)k.t * j.tile_elems +
            ((uint64_t)k.j0 * j.a + k.i0) * j.b;
   if (j.nv16) {
@@ -1026,7 +1237,7 @@ __device__ void gather_store(const BJob &j, uint32_t q, const unsigned char *buf
     const FastDiv dsi = k.si == j.S ? j.div_S : make_fastdiv(k.si);
     unsigned char *d = reinterpret_cast<unsigned char *>(dst);
     const uint64_t ostride = (uint64_t)j.a * U;  // bytes between output rows
-    for (uint32_t x = threadIdx.x; x < n; x += kStageThreads) {
+    for (uint32_t x = threadIdx.x; x < n; x += NT) {
       uint32_t u = x, sv = 0;
       if (NS != 1) {
         u = fdiv(x, j.div_nv16);
@@ -1043,11 +1254,28 @@ __device__ void gather_store(const BJob &j, uint32_t q, const unsigned char *buf
     return;
   }
   if (j.b == 1) {
-    const uint32_t w = threadIdx.x >> 5, nw = kStageThreads / 32;
+    const uint32_t w = threadIdx.x >> 5, nw = NT / 32;
     const uint32_t rb = (j.row_elems * E) & 15;  // row length mod 16
     if constexpr (E <= 2) {
       if (j.vb1 && k.si % (16 / E) == 0 && k.sj % (4 / E) == 0) {
         store_b1_vec<E>(buf, rowoff, k.si, k.sj, dst, j.a, w, nw, j.pitch, rb);
+        return;
+      }
+    }
+    if constexpr (RAG && E <= 2) {
+      if (j.ragged == 2) {
+        store_b1_flat<E>(buf, j.a, j.div_a, k.sj * j.a, dst, threadIdx.x,
+                         NT, j.pitch, rb, rowoff[0] & 15);
+        return;
+      }
+      if (j.ragged) {
+        const uint32_t w = threadIdx.x >> 5;
+        if (j.contig)
+          store_b1_ragged<E, true>(buf, rowoff, j.S, k.si, k.i0 == 0, k.sj, dst,
+                                   j.a, w, NT / 32, j.pitch, rb);
+        else
+          store_b1_ragged<E, false>(buf, rowoff, j.S, k.si, k.i0 == 0, k.sj,
+                                    dst, j.a, w, NT / 32, j.pitch, rb);
         return;
       }
     }
@@ -1066,18 +1294,18 @@ __device__ void gather_store(const BJob &j, uint32_t q, const unsigned char *buf
       return;
     }
     store_b1<E>(buf, rowoff, k.si, k.sj, j.ng8, j.div_ng8, dst, j.a,
-                threadIdx.x >> 5, kStageThreads / 32);
+                threadIdx.x >> 5, NT / 32);
     return;
   }
   const uint32_t ob = k.si * j.b;  // elements per output row segment
   const uint32_t n = k.sj * ob;
   const FastDiv div_ob = k.si == j.S ? j.div_Sb : make_fastdiv(ob);
   const uint64_t ostride = (uint64_t)j.a * j.b;
-  for (uint32_t base = threadIdx.x; base < n; base += kStageThreads * 4) {
+  for (uint32_t base = threadIdx.x; base < n; base += NT * 4) {
     T v[4];
 #pragma unroll
     for (int u = 0; u < 4; ++u) {
-      const uint32_t o = base + u * kStageThreads;
+      const uint32_t o = base + u * NT;
       if (o < n) {
         const uint32_t jj = fdiv(o, div_ob);
         const uint32_t rem = o - jj * ob;
@@ -1092,7 +1320,7 @@ __device__ void gather_store(const BJob &j, uint32_t q, const unsigned char *buf
     }
 #pragma unroll
     for (int u = 0; u < 4; ++u) {
-      const uint32_t o = base + u * kStageThreads;
+      const uint32_t o = base + u * NT;
       if (o < n) {
         const uint32_t jj = fdiv(o, div_ob);
         __stcg(dst + jj * ostride + (o - jj * ob), v[u]);
@@ -1109,11 +1337,13 @@ __device__ void gather_store(const BJob &j, uint32_t q, const unsigned char *buf
 // the registers of two (staged 100s of 2-byte elements, 4096 x 32768:
 // gather 0.0933 vs 0.0963 ms; 500 x 268435: 0.161 vs 0.167 ms; 1-byte
 // 16384 x 16384 the other way: 0.126 vs 0.121 ms).
-template <int MB>
+// RAG: with the code of ragged blocks and of rows staged as one range (in a
+// kernel of its own: it takes 128 registers).
+template <int MB, bool RAG>
 __global__ void __launch_bounds__(kStageThreads, MB) k_batch_gather(BatchArgs g) {
   extern __shared__ __align__(128) unsigned char smem[];
   __shared__ __align__(8) uint64_t bar[2];
-  __shared__ uint32_t rowoff[2][kStageMaxS];
+  __shared__ __align__(16) uint32_t rowoff[2][RAG ? kRowTable : kStageMaxS];
   __shared__ uint32_t s_job[2], s_q[2], s_valid[2];
   __shared__ int s_dead;
   __shared__ __align__(16) BJob s_jobs[2];  // job of the block in each stage
@@ -1157,7 +1387,7 @@ __global__ void __launch_bounds__(kStageThreads, MB) k_batch_gather(BatchArgs g)
   uint32_t cq = s_q[0];
   {
     if (warp == 0) copy_job(&s_jobs[0], &jobs[s_job[0]]);
-    const RowCopy rc = gather_row_plan(jobs[s_job[0]], cq, rowoff[0]);
+    const RowCopy rc = gather_row_plan<kStageThreads, RAG>(jobs[s_job[0]], cq, rowoff[0]);
     gather_arrive(&bar[0], rc.bytes);
     __syncthreads();  // every warp's expected bytes before any copy
     gather_row_issue(rc, smem, &bar[0]);
@@ -1173,7 +1403,7 @@ __global__ void __launch_bounds__(kStageThreads, MB) k_batch_gather(BatchArgs g)
     const uint32_t nj = s_job[nx], nq = s_q[nx];
     if (more) {
       if (warp == 0) copy_job(&s_jobs[nx], &jobs[nj]);
-      const RowCopy rc = gather_row_plan(jobs[nj], nq, rowoff[nx]);
+      const RowCopy rc = gather_row_plan<kStageThreads, RAG>(jobs[nj], nq, rowoff[nx]);
       gather_arrive(&bar[nx], rc.bytes);
       __syncthreads();  // every warp's expected bytes before any copy
       gather_row_issue(rc, smem + (size_t)nx * g.stage_bytes, &bar[nx]);
@@ -1193,10 +1423,10 @@ __global__ void __launch_bounds__(kStageThreads, MB) k_batch_gather(BatchArgs g)
       const BJob &j = s_jobs[st];
       const unsigned char *buf = smem + (size_t)st * g.stage_bytes;
       switch (j.e) {
-        case 1: gather_store<1>(j, cq, buf, rowoff[st]); break;
-        case 2: gather_store<2>(j, cq, buf, rowoff[st]); break;
-        case 4: gather_store<4>(j, cq, buf, rowoff[st]); break;
-        default: gather_store<8>(j, cq, buf, rowoff[st]); break;
+        case 1: gather_store<1, kStageThreads, RAG>(j, cq, buf, rowoff[st]); break;
+        case 2: gather_store<2, kStageThreads, RAG>(j, cq, buf, rowoff[st]); break;
+        case 4: gather_store<4, kStageThreads, RAG>(j, cq, buf, rowoff[st]); break;
+        default: gather_store<8, kStageThreads, RAG>(j, cq, buf, rowoff[st]); break;
       }
     } else {
       s_dead = 1;
@@ -1611,8 +1841,9 @@ static void fill_job(BJob &j, const lm_job &jb, const Normalized &nz,
 // aligned supersets at an odd number of 16-byte words, at most
 // kStageTileBytes per block: whole rows when a row is short (tall, narrow
 // matrices), whole columns when the rows are few (short, wide ones), else
-// S x S with S the largest power of two up to 128 that fits.  False when a
-// unit exceeds kStageTileBytes or the job has 2^32 blocks or more.
+// S x S with S the largest power of two up to 128 that fits (and other
+// heights and widths for 1- and 2-byte elements, below).  False when a unit
+// exceeds kStageTileBytes or the job has 2^32 blocks or more.
 // `scratch` is left for the caller.
 static bool staged_job(BJob &j, const lm_job &jb, const Normalized &nz,
                        uint64_t *nblk, size_t *stage_bytes) {
@@ -1648,9 +1879,63 @@ static bool staged_job(BJob &j, const lm_job &jb, const Normalized &nz,
   }
   Si = std::min<uint64_t>(Si, nz.a);
   Sj = std::min<uint64_t>(Sj, nz.B);
+  j.ragged = j.extra = j.contig = 0;
+  const uint64_t row = nz.B * unit;
+  const bool narrow = nz.b == 1 && nz.e <= 2 && !tune_params().staged_plain;
+  const uint64_t RW = 16 / std::min(nz.e, 2);
+  // narrow elements whose output rows are not whole 16-byte vectors on an
+  // aligned buffer (8-byte ones of 2-byte elements are as fast by
+  // store_b1_vecc: 5004 x 20003 157 us, 160 by store_b1_ragged; with 4-byte
+  // vectors 184 and 161, and bytes in 4- and 8-byte ones 104 and 90)
+  const uint64_t W = nz.e == 2 ? 8 : 16;
+  const bool off =
+      narrow && ((uintptr_t)jb.buf % W || (nz.a * nz.e) % W);
+  if (narrow && row % 4 && 8 * RW * row <= kStageTileBytes * 3 / 4 &&
+      nz.a > 8 * RW) {
+    // short rows, staged as the one range that they are: a bulk copy for
+    // each few dozen bytes is bound by the number of copies (10^7 x 3 bytes
+    // 302 us, 48 this way; 245 tiles of 23673 x 15 half-words 313 and 126).
+    // Rows of whole words would share banks.
+    Sj = nz.B;
+    Si = kStageTileBytes * 3 / 4 / row / (8 * RW) * (8 * RW);
+    j.contig = 1;
+  } else if (off && Si < nz.a) {
+    // 128 columns and the rows that fill the block (64 columns of 2-byte
+    // elements in blocks under 32 KB), unless whole rows leave eight vectors
+    // to an output run
+    if (Sj < nz.B || Si < 9 * RW) {
+      Sj = nz.e == 2 && kStageTileBytes < (32u << 10) ? 64 : 128;
+      if (tune_params().staged_wide > 1) Sj *= tune_params().staged_wide;
+      Sj = std::min<uint64_t>(Sj, nz.B);
+      Si = kStageTileBytes / (Sj * nz.e);
+    }
+    Si = std::max<uint64_t>(std::min<uint64_t>(Si, kStageMaxS) / RW, 2) * RW - RW;
+  }
+  if (j.contig || (off && Si < nz.a)) {
+    // blocks that take RW - 1 rows beyond theirs (store_b1_ragged): as many
+    // down the rows as this height takes, of even height
+    const uint64_t n = (nz.a + Si - 1) / Si;
+    Si = ((nz.a + n - 1) / n + RW - 1) / RW * RW;
+    j.ragged = 1;
+    j.extra = (uint16_t)(RW - 1);
+  } else if (off) {
+    // blocks of whole columns, written as one range (columns of whole words
+    // of bytes go 3-12 % faster by store_b1_vecc's 4- and 8-byte vectors, at
+    // 100 and 200 rows)
+    Si = nz.a;
+    if (nz.e == 2 || nz.a % 4 || (uintptr_t)jb.buf % 4) {
+      j.ragged = 2;
+      if (Sj > RW && Sj < nz.B) Sj = Sj / RW * RW;
+    }
+  } else if (nz.b == 1 && nz.e == 4 && Sj == nz.B && nz.B % 2 &&
+             !tune_params().staged_plain) {
+    // (rows of an odd number of words: their reads share no banks;
+    // 10^7 x 17 floats 724 us with a copy per row, 518 as one range)
+    j.contig = 1;
+  }
   const uint64_t nI = (nz.a + Si - 1) / Si, nJ = (nz.B + Sj - 1) / Sj;
   if (nz.T * nI * nJ >= 0xffffffffull) return false;
-  const uint32_t sp = (uint32_t)pitch_of(Sj);
+  const uint32_t sp = (uint32_t)(j.contig ? row : pitch_of(Sj));
   const uint32_t S = (uint32_t)Si;
   fill_job(j, jb, nz, sp);
   j.S = S;
@@ -1661,7 +1946,7 @@ static bool staged_job(BJob &j, const lm_job &jb, const Normalized &nz,
   // staged rows on 32-bit words (row length, buffer and block columns) and
   // output vectors on 16 bytes (output row length and block rows; the
   // scratch sits at the buffer's address modulo 16)
-  j.vb1 = (nz.b == 1 && nz.e <= 2 && ((uintptr_t)jb.buf & 15) == 0 &&
+  j.vb1 = (nz.b == 1 && !j.contig && nz.e <= 2 && ((uintptr_t)jb.buf & 15) == 0 &&
            (nz.B * nz.e) % 4 == 0 && (Sj * nz.e) % 4 == 0 &&
            (nz.a * nz.e) % 16 == 0 && (S * nz.e) % 16 == 0)
               ? 1u : 0u;
@@ -1674,7 +1959,10 @@ static bool staged_job(BJob &j, const lm_job &jb, const Normalized &nz,
         j.vbc = w;
         break;
       }
-  j.vrw = j.vb1 ? 16 / nz.e : j.vbc / nz.e;
+  j.tab = S;  // (kRowTable words at most)
+  if (j.ragged == 1 && j.contig) j.tab = 4;
+  else if (j.ragged == 1) j.tab = (S * nz.e / 16 + 1) * (16 / nz.e + 4);
+  j.vrw = j.contig ? 0 : j.vb1 || j.ragged ? 16 / nz.e : j.vbc / nz.e;
   j.div_nv16 = make_fastdiv(j.nv16 ? j.nv16 : 1);
   j.ng8 = (S + 7) / 8;
   j.div_ng8 = make_fastdiv(j.ng8);
@@ -1688,8 +1976,11 @@ static bool staged_job(BJob &j, const lm_job &jb, const Normalized &nz,
   // (rows shifted by 16 bytes per group of vrw rows for the vectorized
   // narrow stores)
   *stage_bytes =
-      ((size_t)S * sp + (j.vrw ? 16 * ((S + j.vrw - 1) / j.vrw) : 0) + 127) /
-      128 * 128;
+      ((size_t)(S + j.extra + j.contig) * sp +
+       (j.vrw ? 16 * ((S + j.extra + j.vrw - 1) / j.vrw) : 0) +
+       // (reads whole words past the last row; up to 15 bytes before the first)
+       (j.ragged == 1 || j.contig ? 48 : 0) +
+       127) / 128 * 128;
   return true;
 }
 
@@ -1885,7 +2176,12 @@ static bool plan_batch(lm_batch_t bt, const lm_job *jobs, int n,
           BJob j;
           uint64_t nblk = 0;
           size_t stage = 0;
-          if (!staged_job(j, jb, nz, &nblk, &stage)) goto planner;
+          // (the waves' kernel holds no code for ragged blocks: its mixed
+          // items ran 3 % slower with the registers that these take)
+          tune_params().staged_plain = 1;
+          const bool fits = staged_job(j, jb, nz, &nblk, &stage);
+          tune_params().staged_plain = 0;
+          if (!fits) goto planner;
           // same address modulo 16 as the buffer (see k_batch_copyback);
           // the arena base is set when the wave is enqueued
           j.scratch = (char *)(uintptr_t)(wave_used + ((uintptr_t)jb.buf & 15));
@@ -2005,23 +2301,23 @@ static bool launch_band(cudaStream_t s, const BJob *d_jobs,
   return false;
 }
 
+// (one for both launchers: a kernel's shared-memory limit only grows)
+static LaunchCache g_gather3_cache;
+
 static bool launch_staged(cudaStream_t s, const BJob *d_jobs,
                           const BItem *d_items, uint32_t nitems,
                           uint32_t *counter, size_t smem, bool copyback) {
   if (nitems == 0) return false;
   const DeviceInfo &di = device_info();
-  auto kern = copyback ? k_batch_copyback : k_batch_gather<3>;
+  auto kern = copyback ? k_batch_copyback : k_batch_gather<3, false>;
   // the gather keeps two stages of `smem` bytes
   const size_t dyn = copyback ? 0 : 2 * smem;
-  if (dyn > 48 * 1024 &&
-      cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           (int)dyn) != cudaSuccess)
-    return set_error("batch: smem attribute");
-  int occ = 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, kStageThreads,
-                                                    dyn) != cudaSuccess ||
-      occ < 1)
-    return set_error("batch: occupancy");
+  static LaunchCache copy_cache;
+  cudaError_t err = cudaSuccess;
+  const int occ = prepare_launch((const void *)kern,
+                                 copyback ? copy_cache : g_gather3_cache, dyn,
+                                 kStageThreads, &err);
+  if (err != cudaSuccess || occ < 1) return set_error("batch: occupancy");
   const uint32_t grid =
       (uint32_t)std::min<uint64_t>((uint64_t)di.sms * occ, nitems);
   BatchArgs g;
@@ -2078,18 +2374,18 @@ cudaError_t launch_staged0100(cudaStream_t s, void *buf, int e, uint64_t T,
   size_t stage = 0;
   if (!staged_job(g.single, jb, nz, &nblk, &stage)) return cudaErrorInvalidValue;
   g.single.scratch = reinterpret_cast<char *>(scratch);
-  auto gather = e == 2 ? k_batch_gather<2> : k_batch_gather<3>;
+  const bool rag = g.single.ragged || g.single.contig, two = e == 2;
+  auto gather = rag   ? k_batch_gather<2, true>
+                : two ? k_batch_gather<2, false>
+                      : k_batch_gather<3, false>;
   const size_t dyn = 2 * stage;
   cudaError_t err = cudaSuccess;
-  if (dyn > 48 * 1024 &&
-      (err = cudaFuncSetAttribute(gather,
-                                  cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)dyn)) != cudaSuccess)
-    return err;
-  int occ = 0;
-  if ((err = cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-           &occ, gather, kStageThreads, dyn)) != cudaSuccess)
-    return err;
+  static LaunchCache rag_cache, two_cache;
+  const int occ = prepare_launch(
+      (const void *)gather,
+      rag ? rag_cache : two ? two_cache : g_gather3_cache, dyn, kStageThreads,
+      &err);
+  if (err != cudaSuccess) return err;
   const DeviceInfo &di = device_info();
   const uint32_t grid = (uint32_t)std::min<uint64_t>(
       (uint64_t)di.sms * std::max(occ, 1), nblk);
@@ -2132,6 +2428,10 @@ cudaError_t launch_staged0100(cudaStream_t s, void *buf, int e, uint64_t T,
 // reset (and a captured launch, whose count would be stale on replay, takes
 // the staged form instead).
 constexpr uint32_t kResMaxBlocks = 16;  // blocks one CTA holds
+// 16 warps: the stores are bound by the latency of shared reads (with 8: 894
+// x 5393 half-words 22.6 us instead of 17.8, 260 x 51932 bytes 26.3 instead
+// of 21.1; 32, at 64 registers, spill)
+constexpr int kResThreads = 512;
 constexpr uint32_t kResSlots = 1024;
 __device__ uint32_t g_res_arrivals[kResSlots];
 
@@ -2145,12 +2445,12 @@ struct ResArgs {
   uint64_t timeout_ns;
 };
 
-__global__ void __launch_bounds__(kStageThreads, 1) k_resident(ResArgs g) {
+__global__ void __launch_bounds__(kResThreads, 1) k_resident(ResArgs g) {
   extern __shared__ __align__(128) unsigned char smem[];
   __shared__ __align__(8) uint64_t bar;
   __shared__ __align__(16) BJob s_job;
   __shared__ int s_ok;
-  const uint32_t warp = threadIdx.x >> 5, nw = kStageThreads / 32;
+  const uint32_t warp = threadIdx.x >> 5, nw = kResThreads / 32;
   const uint32_t nmine =
       g.nblk > blockIdx.x ? (g.nblk - blockIdx.x + gridDim.x - 1) / gridDim.x
                           : 0;
@@ -2170,8 +2470,8 @@ __global__ void __launch_bounds__(kStageThreads, 1) k_resident(ResArgs g) {
 #pragma unroll
   for (uint32_t k = 0; k < kResMaxBlocks; ++k)
     if (k < nmine) {
-      rc[k] = gather_row_plan(s_job, blockIdx.x + k * gridDim.x,
-                              rowoff + k * s_job.S);
+      rc[k] = gather_row_plan<kResThreads, true>(s_job, blockIdx.x + k * gridDim.x,
+                              rowoff + k * s_job.tab);
       bytes += rc[k].bytes;
     }
   gather_arrive(&bar, bytes);
@@ -2210,12 +2510,12 @@ __global__ void __launch_bounds__(kStageThreads, 1) k_resident(ResArgs g) {
     for (uint32_t k = 0; k < nmine; ++k) {
       const uint32_t q = blockIdx.x + k * gridDim.x;
       const unsigned char *buf = smem + (size_t)k * g.stage_bytes;
-      const uint32_t *ro = rowoff + k * s_job.S;
+      const uint32_t *ro = rowoff + k * s_job.tab;
       switch (s_job.e) {
-        case 1: gather_store<1>(s_job, q, buf, ro); break;
-        case 2: gather_store<2>(s_job, q, buf, ro); break;
-        case 4: gather_store<4>(s_job, q, buf, ro); break;
-        default: gather_store<8>(s_job, q, buf, ro); break;
+        case 1: gather_store<1, kResThreads, true>(s_job, q, buf, ro); break;
+        case 2: gather_store<2, kResThreads, true>(s_job, q, buf, ro); break;
+        case 4: gather_store<4, kResThreads, true>(s_job, q, buf, ro); break;
+        default: gather_store<8, kResThreads, true>(s_job, q, buf, ro); break;
       }
     }
     return;
@@ -2264,31 +2564,41 @@ bool plan_resident(ResArgs &g, uint32_t *grid, size_t *dyn, void *buf,
   const TuneParams saved = tune_params();
   double best_cost = 0;
   bool ok = false;
-  for (uint32_t wide : {1u, 2u, 4u}) {
-    for (uint32_t tb : {32u << 10, 16u << 10, 8u << 10}) {
-      tune_params().staged_block_bytes = tb;
-      tune_params().staged_wide = wide;
-      BJob j;
-      uint64_t nblk = 0;
-      size_t stage = 0;
-      if (!staged_job(j, jb, nz, &nblk, &stage)) continue;
-      const uint64_t G = std::min<uint64_t>((uint64_t)di.sms, nblk);
-      const uint64_t nper = (nblk + G - 1) / G;
-      const size_t need = nper * stage + (nper * j.S * 4 + 15) / 16 * 16;
-      if (nper > kResMaxBlocks || need > max_dyn) continue;
-      const double cost = 7.6 * (double)(nper * j.S) +
-                          12.5 * (double)(nper * stage) / 1024.0;
-      if (!ok || cost < best_cost) {
-        best_cost = cost;
-        g.job = j;
-        g.nblk = (uint32_t)nblk;
-        g.nper = (uint32_t)nper;
-        g.stage_bytes = (uint32_t)stage;
-        *grid = (uint32_t)G;
-        *dyn = need;
-        ok = true;
+  // (plain: blocks without the extra rows of unaligned narrow ones, whose
+  // shared memory a payload near the limit does not have)
+  for (uint32_t plain = 0; plain < 2 && !ok; ++plain) {
+    tune_params().staged_plain = plain;
+    for (uint32_t wide : {1u, 2u, 4u}) {
+      for (uint32_t tb : {32u << 10, 16u << 10, 8u << 10}) {
+        tune_params().staged_block_bytes = tb;
+        tune_params().staged_wide = wide;
+        BJob j;
+        uint64_t nblk = 0;
+        size_t stage = 0;
+        if (!staged_job(j, jb, nz, &nblk, &stage)) continue;
+        const uint64_t G = std::min<uint64_t>((uint64_t)di.sms, nblk);
+        const uint64_t nper = (nblk + G - 1) / G;
+        const size_t need = nper * stage + (nper * j.tab * 4 + 15) / 16 * 16;
+        if (nper > kResMaxBlocks || need > max_dyn) continue;
+        double cost = 7.6 * (double)(nper * (j.contig ? 16 : j.S + j.extra)) +
+                      12.5 * (double)(nper * stage) / 1024.0;
+        // store_b1_ragged: the steps of a warp in a block, about 120 ns of the
+        // CTA's time each
+        if (j.ragged == 1)
+          cost += 120.0 * (double)nper * ((j.S * e / 16 + 7) / 8) *
+                  ((j.Sj * e + 15) / 16);
+        if (!ok || cost < best_cost) {
+          best_cost = cost;
+          g.job = j;
+          g.nblk = (uint32_t)nblk;
+          g.nper = (uint32_t)nper;
+          g.stage_bytes = (uint32_t)stage;
+          *grid = (uint32_t)G;
+          *dyn = need;
+          ok = true;
+        }
+        break;  // the largest block of this width that fits
       }
-      break;  // the largest block of this width that fits
     }
   }
   tune_params() = saved;
@@ -2406,7 +2716,7 @@ cudaError_t launch_resident0100(cudaStream_t s, void *buf, int e, uint64_t T,
   void *args[] = {&g};
   ProfScope ps(s, "resident");
   err = cudaLaunchCooperativeKernel((const void *)k_resident, dim3(grid),
-                                    dim3(kStageThreads), args, dyn, s);
+                                    dim3(kResThreads), args, dyn, s);
   if (err != cudaSuccess) {
     // no CTA arrives: the slot keeps the count it had
     std::lock_guard<std::mutex> lock(g_res_mu);

@@ -84,6 +84,8 @@ struct TuneParams {
   // staged form: square blocks of S x S units get S * staged_wide columns
   // (0 or 1: square)
   uint32_t staged_wide = 0;
+  // staged form: no extra rows for unaligned narrow blocks (lm_batch.cu)
+  uint32_t staged_plain = 0;
 };
 TuneParams &tune_params();
 
