@@ -21,6 +21,7 @@
 #include <mutex>
 #include <string>
 #include <tuple>
+#include <vector>
 
 #include "lm_core.cuh"
 #include "lm_internal.h"
@@ -182,6 +183,42 @@ uint32_t *device_status_word() {
   }
   return words[dev];
 }
+
+// A zeroed word of pinned host memory for one call's kernel, from a page
+// kept for the process (as many words as calls ever wait at once).
+struct HostWord {
+  static std::mutex &mu() {
+    static std::mutex m;
+    return m;
+  }
+  static std::vector<uint32_t *> &pool() {
+    static std::vector<uint32_t *> v;
+    return v;
+  }
+  uint32_t *p = nullptr;
+  bool lost = false;  // not to be given back
+  HostWord() {
+    std::lock_guard<std::mutex> lock(mu());
+    if (pool().empty()) {
+      void *page = nullptr;
+      constexpr int kWords = 64;
+      if (cudaHostAlloc(&page, kWords * 64, cudaHostAllocPortable) != cudaSuccess) {
+        cudaGetLastError();
+        return;
+      }
+      for (int i = 0; i < kWords; ++i)
+        pool().push_back((uint32_t *)((char *)page + 64 * i));
+    }
+    p = pool().back();
+    pool().pop_back();
+    *(volatile uint32_t *)p = 0;
+  }
+  ~HostWord() {
+    if (!p || lost) return;
+    std::lock_guard<std::mutex> lock(mu());
+    pool().push_back(p);
+  }
+};
 
 // Reads and clears the status word after the stream's work has finished.
 static bool check_status(cudaStream_t s, const char *what) {
@@ -681,19 +718,26 @@ static bool do_pad(cudaStream_t s, void *buf, int e, int64_t x, int64_t y,
   if ((y == 0 || pad == x) && stall_block < 0) return false;
   if (buf == nullptr) return fail("null buffer");
   if (misaligned(buf, e)) return fail("buffer must be aligned to the element size");
-  Scratch sc, st;
-  if (get_zeroed(sc, pad_scratch_bytes(x, y, pad), s)) return true;
-  if (get_zeroed(st, 4, s)) return true;
+  Scratch sc;
+  const size_t flags = stall_block >= 0
+                           ? std::max<size_t>(pad_scratch_bytes(buf, e, y, pad), 16)
+                           : pad_scratch_bytes(buf, e, y, pad);
+  if (flags && get_zeroed(sc, flags, s)) return true;
+  // (a word of host memory, so that no copy follows the kernel)
+  HostWord st;
+  if (!st.p) return fail("padding: no status word");
   cudaError_t err =
-      padding ? launch_padding(s, buf, e, x, y, pad, (uint32_t *)sc.p,
-                               (uint32_t *)st.p, timeout_ns, stall_block)
-              : launch_unpadding(s, buf, e, x, y, pad, (uint32_t *)sc.p,
-                                 (uint32_t *)st.p, timeout_ns, stall_block);
+      padding ? launch_padding(s, buf, e, x, y, pad, (uint32_t *)sc.p, st.p,
+                               timeout_ns, stall_block)
+              : launch_unpadding(s, buf, e, x, y, pad, (uint32_t *)sc.p, st.p,
+                                 timeout_ns, stall_block);
   if (err != cudaSuccess) return cuda_fail(err, padding ? "padding" : "unpadding");
-  uint32_t status = 0;
-  err = cudaMemcpyAsync(&status, st.p, 4, cudaMemcpyDeviceToHost, s);
-  if (err == cudaSuccess) err = cudaStreamSynchronize(s);
-  if (err != cudaSuccess) return cuda_fail(err, "padding status");
+  err = cudaStreamSynchronize(s);
+  if (err != cudaSuccess) {
+    st.lost = true;  // the kernel may still write it
+    return cuda_fail(err, "padding status");
+  }
+  const uint32_t status = *(volatile uint32_t *)st.p;
   if (status != kStatusOk)
     return fail("%s: an inter-CTA wait timed out (status %u)",
                 padding ? "padding" : "unpadding", status);

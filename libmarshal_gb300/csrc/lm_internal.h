@@ -262,11 +262,12 @@ uint32_t *device_status_word();
 // ---- row padding / unpadding with bounded inter-CTA waits ----------------
 // padding:   [y][x] -> [y][pad] (new columns zero)
 // unpadding: [y][pad] -> [y][x], tail y*x..y*pad-1 zero.
-// `scratch` must hold pad_scratch_bytes(...) zeroed bytes; `status` one
-// zeroed word that the kernel sets to kStatusWaitTimeout when a wait runs
-// out.  stall_block >= 0 makes that block wait on a flag nothing sets
-// (failure-detection test hook).
-size_t pad_scratch_bytes(uint64_t x, uint64_t y, uint64_t pad);
+// `scratch` must hold pad_scratch_bytes(...) zeroed bytes (0 and nullptr: one
+// task, which waits for nothing); `status` one zeroed word of pinned host
+// memory that the kernel sets to kStatusWaitTimeout when a wait runs out.
+// stall_block >= 0 makes that task wait on a flag nothing sets
+// (failure-detection test hook; it needs the scratch of two tasks).
+size_t pad_scratch_bytes(const void *buf, int e, uint64_t y, uint64_t pad);
 cudaError_t launch_padding(cudaStream_t s, void *buf, int e, uint64_t x,
                            uint64_t y, uint64_t pad, uint32_t *scratch,
                            uint32_t *status, uint64_t timeout_ns,

@@ -8,35 +8,50 @@
 // unbounded spin, until its predecessor has stored (cl_aos_asta.cl:855-858,
 // 914-917), so the stores of the whole buffer are serialised.
 //
-// GB300 design: each CTA takes a task id from a ticket counter (tasks are
-// handed out in start order), loads its outputs' sources into registers,
-// publishes "loaded" with a release store, then waits -- with an acquire
-// load, a backoff and a time limit -- only for the tasks whose SOURCES lie in
-// its own destination range.  Those tasks always have smaller ids, and a task
-// never waits before publishing its own flag, so the waits cannot form a
-// cycle and the stores of independent tasks overlap.  A wait that runs out
-// sets a status word (the host reports an error) and the CTA skips its
-// stores; nothing spins forever.
+// GB300 design: a task is a range of the padded layout (24 KB, less where the
+// buffer is small), cut at 16-byte addresses, and the compact bytes that
+// belong to it, one range too.  A CTA takes a task from a ticket counter
+// (padding from the back, unpadding from the front), brings its source into
+// shared memory with bulk copies, publishes "loaded" with a release store,
+// then waits -- with an acquire load, a backoff and a time limit -- only for
+// the tasks whose SOURCES lie where it writes.  Those tasks always have
+// smaller tickets, and a task never waits before publishing its own flag, so
+// the waits cannot form a cycle and the stores of independent tasks overlap.
+// A wait that runs out sets a status word (the host reports an error) and the
+// CTA skips its stores; nothing spins forever.
+//
+// Output is written in the 16-byte vectors of its address: inside a row,
+// which is a shift by a constant, four words from five shared ones; across a
+// row's end, element by element into the vector.  Bound by DRAM for rows of
+// some hundred bytes: 8192 x 12289 floats to 12320 columns (806 MB moved)
+// 173 us = 4.7 TB/s (313 us with tasks of single elements in registers),
+// 7382 x 30496 bytes back to 30484 columns 103 us (596).
+#include <algorithm>
+
 #include "lm_core.cuh"
 #include "lm_internal.h"
 
 namespace lm {
 
-constexpr int kPadThreads = 512;
-constexpr int kPadPer = 8;
-constexpr uint64_t kPadTask = (uint64_t)kPadThreads * kPadPer;
+constexpr int kPadThreads = 128;
+constexpr uint64_t kPadTask = 16 * 1024;
+constexpr uint64_t kPadMinTask = 2 * 1024;
 
 struct PadArgs {
   char *buf;
-  uint64_t x, y, pad;
-  uint64_t O;        // outputs = y * pad
+  uint64_t x, pad;   // row bytes, compact and padded
+  uint64_t yx, O;    // bytes of all rows, compact and padded
   uint64_t ntasks;
+  uint32_t P;        // buf modulo 16; task k: padded bytes k*task - P and on
+  uint32_t task;     // bytes of a task, a multiple of 16
+  uint32_t rows;     // unpadding: 1 = copy the rows of a task one by one
   uint32_t *ticket;  // scratch[0]
   uint32_t *loaded;  // scratch[1 .. ntasks]
   uint32_t *never;   // scratch[ntasks + 1], never set
-  uint32_t *status;
+  uint32_t *status;  // host memory, read when the stream has finished
   uint64_t timeout_ns;
   int64_t stall_block;
+  FastDiv div_x, div_pad;  // where rows are no longer than a task
 };
 
 __device__ __forceinline__ bool wait_flag(const uint32_t *f, uint64_t t0,
@@ -50,117 +65,238 @@ __device__ __forceinline__ bool wait_flag(const uint32_t *f, uint64_t t0,
   return true;
 }
 
-// Waits (thread 0) for tasks [k_lo, k_hi] except `self`; returns false on
-// timeout.  Result is broadcast through shared memory.
-__device__ bool wait_range(const PadArgs &g, int64_t k_lo, int64_t k_hi,
-                           uint64_t self, bool stall) {
-  __shared__ int ok;
-  if (threadIdx.x == 0) {
-    const uint64_t t0 = global_timer_ns();
+// Bytes before padded byte o of the rows' own, and their number up to it.
+__device__ __forceinline__ uint64_t pad_compact(uint64_t o, const PadArgs &g) {
+  const uint64_t r = o / g.pad, c = o - r * g.pad;
+  return r * g.x + min64(c, g.x);
+}
+
+// Rows that byte t lies past the row at whose start t counts from zero (t <
+// row + task bytes).
+__device__ __forceinline__ uint32_t pad_rows(uint64_t t, uint64_t row,
+                                             uint32_t task,
+                                             const FastDiv &div) {
+  return row > task ? (t >= row ? 1u : 0u) : fdiv((uint32_t)t, div);
+}
+
+// 16 bytes of shared memory at any byte offset.
+__device__ __forceinline__ uint4 pad_read16(const unsigned char *p,
+                                            uint32_t off) {
+  const uint32_t *q = reinterpret_cast<const uint32_t *>(p + (off & ~3u));
+  const uint32_t a = q[0], b = q[1], c = q[2], d = q[3], e = q[4];
+  const uint32_t s = off * 8;
+  return make_uint4(__funnelshift_r(a, b, s), __funnelshift_r(b, c, s),
+                    __funnelshift_r(c, d, s), __funnelshift_r(d, e, s));
+}
+
+// A task: padded bytes [lo, hi), compact bytes [c0, c1), the rows of lo and
+// c0; its source bytes are [s0, s1), byte s at stage + s - base.
+struct PadTask {
+  uint64_t k, lo, hi, c0, c1, lo_row, c0_row, s0, s1;
+  int64_t base;
+};
+
+template <bool PAD>
+__device__ __forceinline__ void pad_claim(const PadArgs &g, PadTask &t) {
+  // (a single task has no one to wait for and no flags)
+  const uint64_t n = g.ticket ? atomicAdd(g.ticket, 1u) : 0;
+  const uint64_t k = t.k = PAD ? g.ntasks - 1 - n : n;
+  t.lo = k * g.task > g.P ? k * g.task - g.P : 0;
+  t.hi = min64(g.O, (k + 1) * g.task - g.P);
+  t.lo_row = t.lo / g.pad;
+  t.c0 = t.lo_row * g.x + min64(t.lo - t.lo_row * g.pad, g.x);
+  t.c1 = pad_compact(t.hi, g);
+  t.c0_row = t.lo_row;  // (c0 starts the next row where lo is in padding)
+  if (t.lo - t.lo_row * g.pad >= g.x) t.c0_row += 1;
+  t.s0 = PAD ? t.c0 : t.lo;
+  t.s1 = PAD ? t.c1 : t.hi;
+  t.base = (int64_t)((t.s0 + g.P) & ~(uint64_t)15) - g.P;
+}
+
+// One warp: the task's source into `stage`, completion on `bar`.
+template <bool PAD>
+__device__ __forceinline__ void pad_load(const PadArgs &g, const PadTask &t,
+                                         unsigned char *stage, uint64_t *bar) {
+  const uint32_t lane = threadIdx.x & 31;
+  if (PAD || !g.rows) {
+    if (lane) return;
+    const uint32_t bytes =
+        t.s1 > t.s0 ? (uint32_t)((t.s1 - t.base + 15) & ~(uint64_t)15) : 0u;
+    mbar_arrive_expect_tx(bar, bytes);
+    if (bytes) {
+      fence_proxy_async_smem();
+      bulk_g2s(stage, g.buf + t.base, bytes, bar);
+    }
+    return;
+  }
+  // one copy for each row's own bytes (long rows, much padding)
+  const uint64_t r1 = (t.hi - 1) / g.pad;
+  uint32_t bytes = 0;
+  for (int pass = 0; pass < 2; ++pass) {
+    for (uint64_t r = t.lo_row + lane; r <= r1; r += 32) {
+      const uint64_t a = max(t.lo, r * g.pad), b = min64(t.hi, r * g.pad + g.x);
+      if (a >= b) continue;
+      const uint64_t a0 = (a + g.P) & ~(uint64_t)15;
+      const uint64_t b0 = (b + g.P + 15) & ~(uint64_t)15;
+      if (pass == 0)
+        bytes += (uint32_t)(b0 - a0);
+      else
+        bulk_g2s(stage + (a0 - g.P - t.base), g.buf + a0 - g.P,
+                 (uint32_t)(b0 - a0), bar);
+    }
+    if (pass == 0) {
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) bytes += __shfl_xor_sync(kFull, bytes, o);
+      if (lane == 0) mbar_arrive_expect_tx(bar, bytes);
+      __syncwarp();
+      fence_proxy_async_smem();
+    }
+  }
+}
+
+// One task per CTA.  (Persistent CTAs that load their next task's source
+// meanwhile publish it only after the current task, so the waits of all
+// others grow into a convoy: 420 us where this form takes 175.)
+template <int E, bool PAD>
+__global__ void __launch_bounds__(kPadThreads) k_pad(PadArgs g) {
+  using T = typename Elem<E>::T;
+  extern __shared__ __align__(128) unsigned char smem[];
+  __shared__ __align__(8) uint64_t bar;
+  __shared__ PadTask tk;
+  __shared__ int s_ok;
+  const uint32_t tid = threadIdx.x;
+  if (tid == 0) {
+    mbar_init(&bar, 1);
+    fence_mbar_init();
+    s_ok = 1;
+    pad_claim<PAD>(g, tk);
+  }
+  __syncthreads();
+  if (tid < 32) pad_load<PAD>(g, tk, smem, &bar);
+  const uint64_t k = tk.k;
+  const uint64_t lo = tk.lo, hi = tk.hi, c0 = tk.c0, c1 = tk.c1;
+  const int64_t base = tk.base;
+  const uint64_t t0 = global_timer_ns();
+  while (!mbar_try_wait(&bar, 0))
+    if (global_timer_ns() - t0 > g.timeout_ns) {
+      s_ok = 0;
+      break;
+    }
+  __syncthreads();
+  if (tid == 0 && s_ok && g.ticket) st_release_gpu(g.loaded + k, 1u);
+
+  // ---- wait for the tasks whose sources lie where this one writes
+  if (tid < 32) {
+    int64_t k0 = 0, k1 = -1;
+    if (PAD) {
+      const uint64_t e1 = min64(hi, g.yx);
+      if (lo < e1) {
+        const uint64_t o0 = (lo / g.x) * g.pad + lo % g.x;
+        const uint64_t o1 = ((e1 - 1) / g.x) * g.pad + (e1 - 1) % g.x;
+        k0 = (int64_t)((o0 + g.P) / g.task);
+        k1 = (int64_t)((o1 + g.P) / g.task);
+      }
+    } else if (c0 < c1) {
+      // compact bytes [c0, c1) hold the padded bytes of the same numbers
+      k0 = (int64_t)((c0 + g.P) / g.task);
+      k1 = (int64_t)((c1 - 1 + g.P) / g.task);
+    }
+    const uint64_t t1 = global_timer_ns();
     bool good = true;
-    if (stall) good = wait_flag(g.never, t0, g.timeout_ns);
-    for (int64_t k = k_lo; good && k <= k_hi; ++k) {
-      if ((uint64_t)k == self) continue;
-      good = wait_flag(g.loaded + k, t0, g.timeout_ns);
-    }
-    if (!good) atomicOr(g.status, kStatusWaitTimeout);
-    ok = good;
+    if ((int64_t)k == g.stall_block) good = wait_flag(g.never, t1, g.timeout_ns);
+    for (int64_t w = k0 + tid; good && w <= k1; w += 32)
+      if (w != (int64_t)k) good = wait_flag(g.loaded + w, t1, g.timeout_ns);
+    if (!good) s_ok = 0;
   }
   __syncthreads();
-  return ok != 0;
-}
+  if (!s_ok) {
+    if (tid == 0) {
+      *reinterpret_cast<volatile uint32_t *>(g.status) = kStatusWaitTimeout;
+      // nothing may still be landing in shared memory when the CTA exits
+      const uint64_t t2 = global_timer_ns();
+      while (!mbar_try_wait(&bar, 0) && global_timer_ns() - t2 < g.timeout_ns) {
+      }
+    }
+    return;
+  }
 
-template <int E>
-__global__ void __launch_bounds__(kPadThreads) k_padding(PadArgs g) {
-  using T = typename Elem<E>::T;
-  __shared__ uint64_t task_s;
-  if (threadIdx.x == 0) task_s = atomicAdd(g.ticket, 1u);
-  __syncthreads();
-  const uint64_t k = task_s;
-  if (k >= g.ntasks) return;
-  T *b = reinterpret_cast<T *>(g.buf);
-  // outputs of task k: [lo, hi), counted from the back
-  const uint64_t hi = g.O - k * kPadTask;
-  const uint64_t lo = hi > kPadTask ? hi - kPadTask : 0;
-  T v[kPadPer];
+  // ---- write: padded bytes [lo, hi), or compact ones [c0, c1) and zeros
+  const uint64_t d0 = PAD ? lo : c0, d1 = PAD ? hi : c1;
+  const uint64_t row = PAD ? g.pad : g.x;    // of the written layout
+  const uint64_t from = PAD ? g.x : g.pad;   // of the source
+  const uint64_t row0 = PAD ? tk.lo_row : tk.c0_row;
+  const FastDiv &div = PAD ? g.div_pad : g.div_x;
+  const uint64_t in_row = d0 - row0 * row;   // d0's place in its row
+  // source byte of column c, row0 + r: smem[r*from + c + at0]
+  const int64_t at0 = (int64_t)(row0 * from) - base;
+  const int64_t v0 = (int64_t)((d0 + g.P) & ~(uint64_t)15) - g.P;
+  const uint32_t nv = d1 > d0 ? (uint32_t)((d1 - v0 + 15) / 16) : 0u;
+  for (uint32_t v = tid; v < nv; v += kPadThreads) {
+    const int64_t o = v0 + (int64_t)v * 16;
+    const bool whole = o >= (int64_t)d0 && o + 16 <= (int64_t)d1;
+    const uint64_t ob = whole ? (uint64_t)o : max((uint64_t)max(o, (int64_t)0), d0);
+    const uint64_t t = ob - d0 + in_row;
+    uint32_t r = pad_rows(t, row, g.task, div);
+    uint64_t c = t - r * row;
+    if (whole && c + 16 <= g.x) {
+      *reinterpret_cast<uint4 *>(g.buf + o) =
+          pad_read16(smem, (uint32_t)(at0 + (int64_t)(r * from + c)));
+      continue;
+    }
+    if (PAD && whole && c >= g.x && c + 16 <= g.pad) {
+      *reinterpret_cast<uint4 *>(g.buf + o) = make_uint4(0, 0, 0, 0);
+      continue;
+    }
+    // across a row's end, or at an end of the task: element by element
+    T e[16 / E];
+    const uint64_t oe = min64((uint64_t)(o + 16), d1);
+    uint32_t n = (uint32_t)((oe - ob) / E);
 #pragma unroll
-  for (int u = 0; u < kPadPer; ++u) {
-    const uint64_t o = lo + (uint64_t)u * kPadThreads + threadIdx.x;
-    v[u] = T(0);
-    if (o < hi) {
-      const uint64_t r = o / g.pad, c = o - r * g.pad;
-      if (c < g.x) v[u] = __ldcg(b + r * g.x + c);
+    for (uint32_t i = 0; i < 16 / E; ++i) {
+      e[i] = T(0);
+      if (i < n) {
+        if (!PAD || c < g.x)
+          e[i] = *reinterpret_cast<const T *>(
+              smem + (at0 + (int64_t)(r * from + c)));
+        c += E;
+        if (c >= row) {
+          c = 0;
+          ++r;
+        }
+      }
+    }
+    if (whole) {
+      *reinterpret_cast<uint4 *>(g.buf + o) = pack16<E>(e);
+    } else {
+#pragma unroll
+      for (uint32_t i = 0; i < 16 / E; ++i)
+        if (i < n) *reinterpret_cast<T *>(g.buf + ob + i * E) = e[i];
     }
   }
-  __syncthreads();
-  if (threadIdx.x == 0) st_release_gpu(g.loaded + k, 1u);
-  // sources located in [lo, hi) are read by outputs g(s) = (s/x)*pad + s%x
-  int64_t k_lo = 0, k_hi = -1;
-  const uint64_t yx = g.y * g.x;
-  if (lo < yx && g.x > 0) {
-    const uint64_t s0 = lo, s1 = (hi < yx ? hi : yx) - 1;
-    const uint64_t o_min = (s0 / g.x) * g.pad + s0 % g.x;
-    const uint64_t o_max = (s1 / g.x) * g.pad + s1 % g.x;
-    k_lo = (int64_t)((g.O - 1 - o_max) / kPadTask);
-    k_hi = (int64_t)((g.O - 1 - o_min) / kPadTask);
-  }
-  if (!wait_range(g, k_lo, k_hi, k, (int64_t)k == g.stall_block)) return;
-#pragma unroll
-  for (int u = 0; u < kPadPer; ++u) {
-    const uint64_t o = lo + (uint64_t)u * kPadThreads + threadIdx.x;
-    if (o < hi) __stcg(b + o, v[u]);
-  }
-}
-
-template <int E>
-__global__ void __launch_bounds__(kPadThreads) k_unpadding(PadArgs g) {
-  using T = typename Elem<E>::T;
-  __shared__ uint64_t task_s;
-  if (threadIdx.x == 0) task_s = atomicAdd(g.ticket, 1u);
-  __syncthreads();
-  const uint64_t k = task_s;
-  if (k >= g.ntasks) return;
-  T *b = reinterpret_cast<T *>(g.buf);
-  const uint64_t lo = k * kPadTask;
-  const uint64_t hi = (lo + kPadTask < g.O) ? lo + kPadTask : g.O;
-  const uint64_t yx = g.y * g.x;
-  T v[kPadPer];
-#pragma unroll
-  for (int u = 0; u < kPadPer; ++u) {
-    const uint64_t o = lo + (uint64_t)u * kPadThreads + threadIdx.x;
-    v[u] = T(0);
-    if (o < hi && o < yx) {
-      const uint64_t r = o / g.x, c = o - r * g.x;
-      v[u] = __ldcg(b + r * g.pad + c);
-    }
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) st_release_gpu(g.loaded + k, 1u);
-  // sources in [lo, hi) belong to outputs [hinv(lo), hinv(hi)) where
-  // hinv(s) = (s/pad)*x + min(s%pad, x)
-  auto hinv = [&](uint64_t s) {
-    const uint64_t r = s / g.pad, c = s - r * g.pad;
-    return r * g.x + (c < g.x ? c : g.x);
-  };
-  int64_t k_lo = 0, k_hi = -1;
-  uint64_t a0 = hinv(lo), a1 = hinv(hi);
-  if (a1 > yx) a1 = yx;
-  if (a0 < a1) {
-    k_lo = (int64_t)(a0 / kPadTask);
-    k_hi = (int64_t)((a1 - 1) / kPadTask);
-  }
-  if (!wait_range(g, k_lo, k_hi, k, (int64_t)k == g.stall_block)) return;
-#pragma unroll
-  for (int u = 0; u < kPadPer; ++u) {
-    const uint64_t o = lo + (uint64_t)u * kPadThreads + threadIdx.x;
-    if (o < hi) __stcg(b + o, v[u]);
+  if (!PAD && hi > g.yx) {
+    // zeros behind the rows, where this task's own source was: elements up
+    // to a vector boundary, vectors (hi is one, or the buffer's end)
+    const uint64_t z0 = max(lo, g.yx);
+    const uint64_t za = min64(((z0 + g.P + 15) & ~(uint64_t)15) - g.P, hi);
+    const uint64_t zb = za + (hi - za) / 16 * 16;
+    const uint32_t nh = (uint32_t)(za - z0) / E, nt = (uint32_t)(hi - zb) / E;
+    if (tid < nh) *reinterpret_cast<T *>(g.buf + z0 + tid * E) = T(0);
+    if (tid < nt) *reinterpret_cast<T *>(g.buf + zb + tid * E) = T(0);
+    for (uint64_t z = za + tid * 16; z < zb; z += kPadThreads * 16)
+      *reinterpret_cast<uint4 *>(g.buf + z) = make_uint4(0, 0, 0, 0);
   }
 }
 
-size_t pad_scratch_bytes(uint64_t x, uint64_t y, uint64_t pad) {
-  const uint64_t O = y * pad;
-  const uint64_t ntasks = (O + kPadTask - 1) / kPadTask;
-  return (size_t)(ntasks + 2) * 4;
+// Bytes of a task: at least two tasks per SM where the buffer has them.
+static uint32_t pad_task_bytes(uint64_t bytes) {
+  const uint64_t per = bytes / (2 * (uint64_t)device_info().sms);
+  return (uint32_t)(std::max(kPadMinTask, std::min(kPadTask, per)) / 128 * 128);
+}
+
+size_t pad_scratch_bytes(const void *buf, int e, uint64_t y, uint64_t pad) {
+  const uint64_t O = y * pad * e, task = pad_task_bytes(O);
+  const uint64_t n = (O + ((uintptr_t)buf & 15) + task - 1) / task;
+  return n > 1 ? (size_t)(n + 2) * 4 : 0;
 }
 
 template <bool PAD>
@@ -169,33 +305,38 @@ static cudaError_t run_pad(cudaStream_t s, void *buf, int e, uint64_t x,
                            uint32_t *status, uint64_t timeout_ns,
                            int64_t stall_block) {
   if (pad < x) return cudaErrorInvalidValue;
-  const uint64_t O = y * pad;
-  if (O == 0 || (pad == x && stall_block < 0)) return cudaSuccess;
   PadArgs g;
   g.buf = reinterpret_cast<char *>(buf);
-  g.x = x;
-  g.y = y;
-  g.pad = pad;
-  g.O = O;
-  g.ntasks = (O + kPadTask - 1) / kPadTask;
-  if (g.ntasks >= 0xffffffffull) return cudaErrorInvalidValue;
+  g.x = x * e;
+  g.pad = pad * e;
+  g.yx = y * g.x;
+  g.O = y * g.pad;
+  if (g.O == 0 || (pad == x && stall_block < 0)) return cudaSuccess;
+  g.P = (uint32_t)((uintptr_t)buf & 15);
+  g.task = pad_task_bytes(g.O);
+  g.ntasks = (g.O + g.P + g.task - 1) / g.task;
+  if (g.ntasks >= 0x7fffffffull) return cudaErrorInvalidValue;
+  // rows of 1 KB and more with an eighth or more of padding
+  g.rows = g.x >= 1024 && (g.pad - g.x) * 8 >= g.pad ? 1u : 0u;
+  if (g.ntasks > 1 && !scratch) return cudaErrorInvalidValue;
   g.ticket = scratch;
   g.loaded = scratch + 1;
   g.never = scratch + 1 + g.ntasks;
   g.status = status;
   g.timeout_ns = timeout_ns;
   g.stall_block = stall_block;
+  g.div_x = make_fastdiv((uint32_t)std::min<uint64_t>(g.x ? g.x : 1, 1u << 30));
+  g.div_pad = make_fastdiv((uint32_t)std::min<uint64_t>(g.pad, 1u << 30));
+  // the task's bytes, the rest of its first and last 16, and the word that
+  // the last unaligned read runs over
+  const size_t smem = g.task + 64;
   const unsigned grid = (unsigned)g.ntasks;
   ProfScope ps(s, PAD ? "padding" : "unpadding");
   switch (e) {
-    case 1: PAD ? k_padding<1><<<grid, kPadThreads, 0, s>>>(g)
-                : k_unpadding<1><<<grid, kPadThreads, 0, s>>>(g); break;
-    case 2: PAD ? k_padding<2><<<grid, kPadThreads, 0, s>>>(g)
-                : k_unpadding<2><<<grid, kPadThreads, 0, s>>>(g); break;
-    case 4: PAD ? k_padding<4><<<grid, kPadThreads, 0, s>>>(g)
-                : k_unpadding<4><<<grid, kPadThreads, 0, s>>>(g); break;
-    case 8: PAD ? k_padding<8><<<grid, kPadThreads, 0, s>>>(g)
-                : k_unpadding<8><<<grid, kPadThreads, 0, s>>>(g); break;
+    case 1: k_pad<1, PAD><<<grid, kPadThreads, smem, s>>>(g); break;
+    case 2: k_pad<2, PAD><<<grid, kPadThreads, smem, s>>>(g); break;
+    case 4: k_pad<4, PAD><<<grid, kPadThreads, smem, s>>>(g); break;
+    case 8: k_pad<8, PAD><<<grid, kPadThreads, smem, s>>>(g); break;
     default: return cudaErrorInvalidValue;
   }
   return cudaGetLastError();

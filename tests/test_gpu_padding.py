@@ -1,0 +1,57 @@
+"""Row padding and unpadding by tasks of byte ranges (lm_pad.cu), at the edges
+of tasks, rows and vectors and on buffers at every alignment."""
+import pytest
+
+torch = pytest.importorskip("torch")
+
+from libmarshal_gb300 import lm
+
+pytestmark = pytest.mark.gpu
+
+DT = {1: torch.uint8, 2: torch.int16, 4: torch.int32, 8: torch.int64}
+
+
+def _check(e, x, y, pad, offset=0):
+    n = y * pad * e
+    g = torch.Generator(device="cuda").manual_seed(n + x + offset)
+    raw = torch.randint(1, 256, (n + 64,), dtype=torch.uint8, device="cuda",
+                        generator=g)
+    before = raw.clone()
+    data = before[offset:offset + n].clone().view(DT[e])
+    ptr = raw.data_ptr() + offset
+    want = torch.zeros_like(data)
+    want.view(y, pad)[:, :x] = data[:y * x].view(y, x)
+    lm.padding(ptr, x, y, pad, elem_bytes=e)
+    assert torch.equal(raw[offset:offset + n], want.view(torch.uint8))
+    data = torch.randint(1, 100, (y * pad,), device="cuda", generator=g).to(DT[e])
+    raw[offset:offset + n] = data.view(torch.uint8)
+    want.zero_()
+    want[:y * x] = data.view(y, pad)[:, :x].reshape(-1)
+    lm.unpadding(ptr, x, y, pad, elem_bytes=e)
+    assert torch.equal(raw[offset:offset + n], want.view(torch.uint8))
+    assert torch.equal(raw[:offset], before[:offset])
+    assert torch.equal(raw[offset + n:], before[offset + n:])
+
+
+@pytest.mark.parametrize("e", [1, 2, 4, 8])
+def test_shapes(e):
+    for x, y, pad in ((1, 1, 2), (0, 7, 5), (3, 100, 4), (15, 70, 16),
+                      (16, 4000, 17), (1, 3000, 129), (17, 2049, 32),
+                      (2047, 33, 2048), (2049, 33, 3000), (1024, 600, 1200),
+                      (33000, 5, 33001), (5000, 101, 40000), (100003, 9, 100016),
+                      (661, 16, 672), (4, 100000, 5)):
+        _check(e, x, y, pad)
+
+
+@pytest.mark.parametrize("e", [1, 2, 4, 8])
+def test_alignments(e):
+    for off in range(0, 16, e):
+        for x, y, pad in ((37, 501, 40), (3001, 21, 3100), (2000, 61, 2500)):
+            _check(e, x, y, pad, off)
+
+
+@pytest.mark.parametrize("e,x,y,pad", [(4, 12289, 1024, 12320),
+                                       (1, 30484, 2000, 30496),
+                                       (2, 663, 50001, 672), (8, 25, 200000, 28)])
+def test_large(e, x, y, pad):
+    _check(e, x, y, pad)
