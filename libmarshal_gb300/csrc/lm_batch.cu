@@ -92,7 +92,7 @@ struct BJob {
   // store_b1_ragged (blocks stage `extra` rows more than S), 2 =
   // store_b1_flat (blocks of whole columns), 0 = none; contig = blocks of
   // whole rows staged as the one range that they are, row r at r * row
-  // bytes; tab = words of a block's table of row offsets
+  // bytes (2: with 16 bytes after each 16/e rows); tab = words of a block's table of row offsets
   uint8_t ragged, contig;
   uint16_t extra;
   uint32_t tab;
@@ -747,7 +747,7 @@ template <int E, bool CONTIG>
 __device__ __forceinline__ void store_b1_ragged(
     const unsigned char *buf, const uint32_t *tab, uint32_t S, uint32_t nrows,
     bool first, uint32_t ncols, typename Elem<E>::T *dst, uint32_t ostride,
-    uint32_t warp, uint32_t nwarps, uint32_t pitch, uint32_t rb) {
+    uint32_t warp, uint32_t nwarps, uint32_t pitch, uint32_t rb, uint32_t gp) {
   static_assert(E == 1 || E == 2, "narrow elements only");
   using T = typename Elem<E>::T;
   constexpr uint32_t RW = 16 / E, TW = RW + 4, CW = 4 / E;
@@ -776,7 +776,7 @@ __device__ __forceinline__ void store_b1_ragged(
     };
     // rows without a table: the words of rows 0..3 of the group, a multiple
     // of 4 bytes further on for each four rows
-    const uint32_t o0 = m0 + g * RW * pitch;
+    const uint32_t o0 = m0 + g * (RW * pitch + gp);
     const uint32_t c0 = o0 & ~3u, c1 = (o0 + pitch) & ~3u,
                    c2 = (o0 + 2 * pitch) & ~3u, c3 = (o0 + 3 * pitch) & ~3u;
 #pragma unroll
@@ -784,7 +784,7 @@ __device__ __forceinline__ void store_b1_ragged(
       if constexpr (E == 1) {
         uint4 t;
         if constexpr (CONTIG) {
-          const uint32_t st = q * 4 * pitch;
+          const uint32_t st = q * 4 * pitch + (q / 4) * gp;
           t = make_uint4(c0 + st, c1 + st, c2 + st, c3 + st);
         } else {
           t = *reinterpret_cast<const uint4 *>(tg + (q / 4) * TW + (q % 4) * 4);
@@ -802,7 +802,7 @@ __device__ __forceinline__ void store_b1_ragged(
       } else {
         uint2 t;
         if constexpr (CONTIG) {
-          const uint32_t st = (q / 2) * 4 * pitch;
+          const uint32_t st = (q / 2) * 4 * pitch + (q / 4) * gp;
           t = q % 2 ? make_uint2(c2 + st, c3 + st) : make_uint2(c0 + st, c1 + st);
         } else {
           t = *reinterpret_cast<const uint2 *>(tg + (q / 4) * TW + (q % 4) * 2);
@@ -840,7 +840,7 @@ __device__ __forceinline__ void store_b1_ragged(
     T *run = dst + (uint64_t)jj * ostride;
     const uint32_t h = (16 - (uint32_t)((uintptr_t)run & 15)) / E % RW;
     auto put = [&](uint32_t r) {
-      const uint32_t off = CONTIG ? m0 + r * pitch
+      const uint32_t off = CONTIG ? m0 + r * pitch + r / RW * gp
                                   : tab[rag_index(r, E)] + ((m0 + r * rb) & 3);
       __stcg(run + r, *reinterpret_cast<const T *>(buf + off + jj * E));
     };
@@ -1183,6 +1183,16 @@ __device__ __forceinline__ RowCopy gather_row_plan(const BJob &j, uint32_t q,
       for (uint32_t r = threadIdx.x; r < k.si; r += NT)
         rowoff[r] = m0 + r * j.pitch;
     }
+    if (j.contig == 2) {
+      // a copy per group of RW rows (16 B bytes), 16 bytes between groups
+      const uint32_t gb = j.pitch * (16 / j.e);
+      const uint32_t g = (threadIdx.x & 31) * (NT / 32) + (threadIdx.x >> 5);
+      if (g * gb >= k.si * j.pitch) return c;
+      c.src = src - m0 + (uint64_t)g * gb;
+      c.bytes = min((m0 + gb + 15) & ~15u, all - g * gb);
+      c.dst = g * (gb + 16);
+      return c;
+    }
     const uint32_t o = (threadIdx.x >> 5) * piece;
     if ((threadIdx.x & 31) || o >= all) return c;
     c.src = src - m0 + o;
@@ -1272,10 +1282,11 @@ __device__ void gather_store(const BJob &j, uint32_t q, const unsigned char *buf
         const uint32_t w = threadIdx.x >> 5;
         if (j.contig)
           store_b1_ragged<E, true>(buf, rowoff, j.S, k.si, k.i0 == 0, k.sj, dst,
-                                   j.a, w, NT / 32, j.pitch, rb);
+                                   j.a, w, NT / 32, j.pitch, rb,
+                                   j.contig == 2 ? 16 : 0);
         else
           store_b1_ragged<E, false>(buf, rowoff, j.S, k.si, k.i0 == 0, k.sj,
-                                    dst, j.a, w, NT / 32, j.pitch, rb);
+                                    dst, j.a, w, NT / 32, j.pitch, rb, 0);
         return;
       }
     }
@@ -1890,15 +1901,19 @@ static bool staged_job(BJob &j, const lm_job &jb, const Normalized &nz,
   const uint64_t W = nz.e == 2 ? 8 : 16;
   const bool off =
       narrow && ((uintptr_t)jb.buf % W || (nz.a * nz.e) % W);
-  if (narrow && row % 4 && 8 * RW * row <= kStageTileBytes * 3 / 4 &&
-      nz.a > 8 * RW) {
+  if (narrow && 8 * RW * row <= kStageTileBytes * 3 / 4 && nz.a > 8 * RW &&
+      (off || row % 4)) {
     // short rows, staged as the one range that they are: a bulk copy for
     // each few dozen bytes is bound by the number of copies (10^7 x 3 bytes
     // 302 us, 48 this way; 245 tiles of 23673 x 15 half-words 313 and 126).
-    // Rows of whole words would share banks.
+    // A copy per RW rows where B is a multiple of 4, whose groups of rows
+    // would share banks if nothing lay between them.
     Sj = nz.B;
     Si = kStageTileBytes * 3 / 4 / row / (8 * RW) * (8 * RW);
-    j.contig = 1;
+    j.contig = nz.B % 4 ? 1 : 2;
+    // (a thread per copy of the smallest CTA, and the rows beyond)
+    if (j.contig == 2)
+      Si = std::min<uint64_t>(Si, (kStageThreads - 8) * RW);
   } else if (off && Si < nz.a) {
     // 128 columns and the rows that fill the block (64 columns of 2-byte
     // elements in blocks under 32 KB), unless whole rows leave eight vectors
@@ -1976,7 +1991,8 @@ static bool staged_job(BJob &j, const lm_job &jb, const Normalized &nz,
   // (rows shifted by 16 bytes per group of vrw rows for the vectorized
   // narrow stores)
   *stage_bytes =
-      ((size_t)(S + j.extra + j.contig) * sp +
+      ((size_t)(S + j.extra + (j.contig ? 1 : 0)) * sp +
+       (j.contig == 2 ? 16 * ((size_t)S / (16 / nz.e) + 1) : 0) +
        (j.vrw ? 16 * ((S + j.extra + j.vrw - 1) / j.vrw) : 0) +
        // (reads whole words past the last row; up to 15 bytes before the first)
        (j.ragged == 1 || j.contig ? 48 : 0) +

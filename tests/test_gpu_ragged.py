@@ -53,7 +53,8 @@ def test_buffer_alignment(e, offsets):
 
 
 @pytest.mark.parametrize("e", [1, 2, 4])
-@pytest.mark.parametrize("B", [2, 3, 5, 9, 16, 17, 63, 95, 119, 191, 193])
+@pytest.mark.parametrize("B", [2, 3, 4, 5, 8, 9, 12, 16, 17, 30, 63, 64, 95, 119, 124,
+                               191, 193])
 def test_short_rows(B, e):
     """Rows staged as one range, and the widths just past it."""
     for T, a in ((1, 4099), (3, 1000), (2, 1537), (5, 257)):
