@@ -1181,7 +1181,8 @@ __device__ __forceinline__ RowCopy gather_row_plan(const BJob &j, uint32_t q,
       if (threadIdx.x == 0) rowoff[0] = m0;
     } else {
       for (uint32_t r = threadIdx.x; r < k.si; r += NT)
-        rowoff[r] = m0 + r * j.pitch;
+        rowoff[r] = m0 + r * j.pitch +
+                    (j.contig == 2 ? r / (16 / j.e) * 16 : 0);
     }
     if (j.contig == 2) {
       // a copy per group of RW rows (16 B bytes), 16 bytes between groups
@@ -1902,10 +1903,12 @@ static bool staged_job(BJob &j, const lm_job &jb, const Normalized &nz,
   const bool off =
       narrow && ((uintptr_t)jb.buf % W || (nz.a * nz.e) % W);
   if (narrow && 8 * RW * row <= kStageTileBytes * 3 / 4 && nz.a > 8 * RW &&
-      (off || row % 4)) {
+      (off || row % 4 || row <= 128)) {
     // short rows, staged as the one range that they are: a bulk copy for
     // each few dozen bytes is bound by the number of copies (10^7 x 3 bytes
-    // 302 us, 48 this way; 245 tiles of 23673 x 15 half-words 313 and 126).
+    // 302 us, 48 this way; 245 tiles of 23673 x 15 half-words 313 and 126; with
+    // output rows of whole vectors, 10^7 x 16 bytes 356 and 123, 3 10^6 x 64
+    // half-words 472 and 270, but x 128 538 and 583).
     // A copy per RW rows where B is a multiple of 4, whose groups of rows
     // would share banks if nothing lay between them.
     Sj = nz.B;
@@ -1942,11 +1945,12 @@ static bool staged_job(BJob &j, const lm_job &jb, const Normalized &nz,
       j.ragged = 2;
       if (Sj > RW && Sj < nz.B) Sj = Sj / RW * RW;
     }
-  } else if (nz.b == 1 && nz.e == 4 && Sj == nz.B && nz.B % 2 &&
-             !tune_params().staged_plain) {
-    // (rows of an odd number of words: their reads share no banks;
-    // 10^7 x 17 floats 724 us with a copy per row, 518 as one range)
-    j.contig = 1;
+  } else if (nz.b == 1 && nz.e >= 4 && Sj == nz.B &&
+             (nz.B % 2 || row <= 256) && !tune_params().staged_plain) {
+    // the same for wider elements: 10^7 x 17 floats 724 us with a copy per
+    // row, 513 as one range; 6 10^6 x 20 429 and 336, 3 10^6 x 64 512 and
+    // 473, 6 10^6 x 4 doubles 266 and 243
+    j.contig = nz.B % 2 ? 1 : 2;
   }
   const uint64_t nI = (nz.a + Si - 1) / Si, nJ = (nz.B + Sj - 1) / Sj;
   if (nz.T * nI * nJ >= 0xffffffffull) return false;

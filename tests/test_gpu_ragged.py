@@ -52,7 +52,7 @@ def test_buffer_alignment(e, offsets):
             _check(1, a, B, e, RESIDENT, off)
 
 
-@pytest.mark.parametrize("e", [1, 2, 4])
+@pytest.mark.parametrize("e", [1, 2, 4, 8])
 @pytest.mark.parametrize("B", [2, 3, 4, 5, 8, 9, 12, 16, 17, 30, 63, 64, 95, 119, 124,
                                191, 193])
 def test_short_rows(B, e):
