@@ -381,6 +381,13 @@ static bool do_0100(cudaStream_t s, void *buf, int e, uint64_t T, uint64_t a,
   if (misaligned(buf, e)) return fail("buffer must be aligned to the element size");
   if (a * B >= 0xffffffffull) return fail("a*B must be < 2^32");
   widen_units(buf, &e, &b);
+  if (m == Method::Auto && a == B && !getenv("LM_NO_SQUARE") &&
+      square0100_applies(buf, T, a, B, b, e)) {
+    uint32_t *status = device_status_word();
+    return check_launch(launch_square0100(s, buf, e, T, a, b, status,
+                                          wait_timeout_ns()),
+                        "square launch");
+  }
   if (m == Method::Auto || m == Method::BS) {
     BsPlan p = plan_bs0100(T, (uint32_t)a, (uint32_t)B, (uint32_t)b, e);
     // a megabyte or more in fewer tile chunks (or clusters) than SMs leaves

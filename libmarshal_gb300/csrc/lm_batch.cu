@@ -1121,6 +1121,7 @@ __global__ void __launch_bounds__(kBatchThreads, 2) k_batch_band(BatchArgs g) {
 constexpr int kStageThreads = 256;
 constexpr uint32_t kStageTileBytes = 32 * 1024;  // staged bytes per block
 constexpr uint32_t kStageMaxS = 256;             // rows per block
+constexpr uint32_t kSquareMaxS = 128;             // rows of a square's block
 constexpr uint32_t kRowTable = (kStageMaxS / 8 + 1) * 12;  // most words of a BJob::tab
 constexpr uint32_t kStageBlocksPerItem = 4;   // fine-grained: balanced tails
 constexpr uint64_t kCopyVecsPerItem = 16384;     // 256 KB
@@ -1889,6 +1890,7 @@ static bool staged_job(BJob &j, const lm_job &jb, const Normalized &nz,
     Si = Sj = S;
     if (tune_params().staged_wide > 1) Sj = S * tune_params().staged_wide;
   }
+  if (tune_params().square) Si = Sj = tune_params().square;
   Si = std::min<uint64_t>(Si, nz.a);
   Sj = std::min<uint64_t>(Sj, nz.B);
   j.ragged = j.extra = j.contig = 0;
@@ -2433,6 +2435,209 @@ cudaError_t launch_staged0100(cudaStream_t s, void *buf, int e, uint64_t T,
   k_stage_copyback<<<cgrid, kStageThreads, 0, s>>>(
       reinterpret_cast<char *>(buf), reinterpret_cast<const char *>(scratch),
       g.single.bytes);
+  return cudaGetLastError();
+}
+
+// ---- square 0100s ------------------------------------------------------------
+// A square matrix of units is transposed in place block pair by block pair:
+// blocks (I, J) and (J, I) are both staged, then each is written transposed
+// over the other, so no CTA waits for another, no scratch is needed and the
+// payload moves once in and once out.  Two pairs per CTA: the next pair's
+// rows (bulk copies spread over all threads) land while the current one is
+// written.
+struct SqArgs {
+  BJob job;              // S x S blocks, written over themselves
+  uint32_t nitems;       // pairs (and blocks of the diagonal) of all tiles
+  uint32_t nb;           // block rows of a tile
+  uint32_t stage_bytes;  // shared-memory bytes of one block
+  uint32_t *status;
+  uint64_t timeout_ns;
+  FastDiv div_pairs, div_w;
+};
+
+// Pair x: blocks q[0] = (I, J) and q[1] = (J, I), I <= J.  The triangle is
+// folded into a rectangle of w columns: row r holds block row r's pairs and
+// those of the block row that fills it up.
+__device__ __forceinline__ void square_pair(const SqArgs &g, uint32_t x,
+                                            uint32_t q[2]) {
+  const uint32_t t = fdiv(x, g.div_pairs);
+  x -= t * g.div_pairs.d;
+  const uint32_t r = fdiv(x, g.div_w), c = x - r * g.div_w.d;
+  const uint32_t even = (g.nb & 1) ^ 1;
+  uint32_t I, J;
+  if (c >= r + even) {
+    I = r;
+    J = c - even;
+  } else {
+    I = g.nb - even - r;
+    J = g.nb - 1 - c;
+  }
+  q[0] = t * g.job.nIJ + I * g.nb + J;
+  q[1] = t * g.job.nIJ + J * g.nb + I;
+}
+
+__global__ void __launch_bounds__(kStageThreads, 3) k_square(SqArgs g) {
+  extern __shared__ __align__(128) unsigned char smem[];
+  __shared__ __align__(8) uint64_t bar[2];
+  __shared__ __align__(16) uint32_t rowoff[2][2][kSquareMaxS];
+  __shared__ __align__(16) BJob s_job;
+  __shared__ int s_dead;
+  const uint32_t warp = threadIdx.x >> 5;
+  if (threadIdx.x == 0) {
+    mbar_init(&bar[0], kStageThreads / 32);
+    mbar_init(&bar[1], kStageThreads / 32);
+    fence_mbar_init();
+    s_dead = 0;
+  }
+  if (warp == 0) copy_job(&s_job, &g.job);
+  __syncthreads();
+  // the copies of pair x into stage st
+  auto issue = [&](uint32_t x, uint32_t st) {
+    uint32_t q[2];
+    square_pair(g, x, q);
+    unsigned char *buf = smem + st * 2 * (size_t)g.stage_bytes;
+    const RowCopy a =
+        gather_row_plan<kStageThreads, false>(s_job, q[0], rowoff[st][0]);
+    RowCopy b{0, 0, 0};
+    if (q[1] != q[0])
+      b = gather_row_plan<kStageThreads, false>(s_job, q[1], rowoff[st][1]);
+    gather_arrive(&bar[st], a.bytes + b.bytes);
+    __syncthreads();  // every warp's expected bytes before any copy
+    gather_row_issue(a, buf, &bar[st]);
+    gather_row_issue(b, buf + g.stage_bytes, &bar[st]);
+  };
+  if (blockIdx.x >= g.nitems) return;
+  issue(blockIdx.x, 0);
+  uint32_t n = 0;
+  bool ahead = false;  // the other stage's copies are in flight
+  for (uint32_t x = blockIdx.x;; x += gridDim.x, ++n) {
+    const uint32_t st = n & 1;
+    ahead = g.nitems - x > gridDim.x;
+    if (ahead) issue(x + gridDim.x, st ^ 1);
+    const uint64_t t0 = global_timer_ns();
+    while (!mbar_try_wait(&bar[st], (n >> 1) & 1))
+      if (global_timer_ns() - t0 > g.timeout_ns) {
+        s_dead = 1;
+        break;
+      }
+    __syncthreads();  // both blocks are staged for everyone
+    if (s_dead) break;
+    uint32_t q[2];
+    square_pair(g, x, q);
+    const unsigned char *buf = smem + st * 2 * (size_t)g.stage_bytes;
+    for (uint32_t h = 0; h < (q[0] == q[1] ? 1u : 2u); ++h) {
+      const unsigned char *b = buf + h * g.stage_bytes;
+      const uint32_t *ro = rowoff[st][h];
+      switch (s_job.e) {
+        case 1: gather_store<1, kStageThreads, false>(s_job, q[h], b, ro); break;
+        case 2: gather_store<2, kStageThreads, false>(s_job, q[h], b, ro); break;
+        case 4: gather_store<4, kStageThreads, false>(s_job, q[h], b, ro); break;
+        default: gather_store<8, kStageThreads, false>(s_job, q[h], b, ro);
+      }
+    }
+    __syncthreads();  // stage st is free
+    if (!ahead) return;
+  }
+  // a copy that never landed: report it, wait once more (bounded) for what
+  // may still be landing
+  if (threadIdx.x == 0 && g.status) atomicExch(g.status, kStatusWaitTimeout);
+  for (uint32_t m = n; m < n + (ahead ? 2u : 1u); ++m) {
+    const uint64_t t1 = global_timer_ns();
+    while (!mbar_try_wait(&bar[m & 1], (m >> 1) & 1) &&
+           global_timer_ns() - t1 < g.timeout_ns) {
+    }
+  }
+}
+
+// Blocks of a square 0100; false where it is not one or its stores would go
+// element by element (narrow elements whose rows are no whole 8-byte
+// vectors: the staged form's ragged blocks are faster).
+static bool plan_square(SqArgs &g, void *buf, uint64_t T, uint64_t a,
+                        uint64_t B, uint64_t b, int e) {
+  const uint64_t unit = b * (uint64_t)e;
+  // (units of 64 bytes and more move as cycles of two; matrices of up to 128
+  // units as whole tiles: 1000 x 100^2 floats 21.1 us, 30.5 as squares)
+  if (T == 0 || a != B || a <= (T > 4 ? 255u : 128u) || unit > 32) return false;
+  lm_job jb{};
+  jb.buf = buf;
+  jb.elem_bytes = e;
+  Normalized nz;
+  nz.ok = true;
+  nz.e = e;
+  nz.T = T;
+  nz.a = nz.B = a;
+  nz.b = b;
+  // blocks of 16 to 32 KB with rows of 128 bytes and more (16384^2 half-words
+  // 209 us with 128 rows, 267 with 64; 8192^2 floats 98 with 64, 215 with
+  // 32; 8192^2 doubles 202 with 64, 240 with 32), of even size, and smaller
+  // where they are fewer than SMs (333^2 floats 10.6 us with 64 rows, 10.0
+  // with 32)
+  uint64_t S = unit <= 2 ? 128 : unit <= 8 ? 64 : 32;
+  auto pairs = [&](uint64_t s) {
+    const uint64_t n = (a + s - 1) / s;
+    return T * (n * (n + 1) / 2);
+  };
+  // where the CTAs take few pairs each, halves may fill the last round better
+  // (they cost 20 % more per byte, twice as much with rows under 256 bytes):
+  // 7 x 700^2 doubles 19.9 us with 64 rows, 18.5 with 32
+  auto rounds = [&](uint64_t s) {
+    const uint64_t pitch = (s * unit + 15) / 16 * 16 + 32;
+    const uint64_t occ = std::max<uint64_t>(
+        1, std::min<uint64_t>(3, (220u << 10) / (4 * s * pitch)));
+    const uint64_t ctas = occ * (uint64_t)device_info().sms;
+    return (double)((pairs(s) + ctas - 1) / ctas * occ * s * s);
+  };
+  while (S > 32 && (pairs(S) < (uint64_t)device_info().sms ||
+                    rounds(S / 2) * (S / 2 * unit >= 256 ? 1.2 : 2.2) <
+                        rounds(S)))
+    S /= 2;
+  const uint64_t nb = (a + S - 1) / S, RW = 16 / (uint64_t)e;
+  S = ((a + nb - 1) / nb + RW - 1) / RW * RW;
+  const TuneParams saved = tune_params();
+  tune_params() = TuneParams();
+  tune_params().square = (uint32_t)S;
+  tune_params().staged_plain = 1;
+  uint64_t nblk = 0;
+  size_t stage = 0;
+  const bool ok = staged_job(g.job, jb, nz, &nblk, &stage);
+  tune_params() = saved;
+  if (!ok || pairs(S) >= 0xffffffffull ||
+      4 * stage + 4096 > (size_t)device_info().max_smem_optin)
+    return false;
+  if (e <= 2 && b == 1 && !g.job.vb1 && g.job.vbc < 8) return false;
+  g.job.scratch = g.job.base;
+  g.nb = g.job.nJ;
+  const uint32_t per = g.nb * (g.nb + 1) / 2;
+  g.nitems = (uint32_t)(T * per);
+  g.stage_bytes = (uint32_t)stage;
+  g.div_pairs = make_fastdiv(per);
+  g.div_w = make_fastdiv(g.nb | 1);
+  return true;
+}
+
+bool square0100_applies(const void *buf, uint64_t T, uint64_t a, uint64_t B,
+                        uint64_t b, int e) {
+  SqArgs g{};
+  return plan_square(g, const_cast<void *>(buf), T, a, B, b, e);
+}
+
+cudaError_t launch_square0100(cudaStream_t s, void *buf, int e, uint64_t T,
+                              uint64_t a, uint64_t b, uint32_t *status,
+                              uint64_t timeout_ns) {
+  SqArgs g{};
+  if (!plan_square(g, buf, T, a, a, b, e)) return cudaErrorInvalidValue;
+  g.status = status;
+  g.timeout_ns = timeout_ns;
+  const size_t dyn = 4 * (size_t)g.stage_bytes;
+  static LaunchCache cache;
+  cudaError_t err = cudaSuccess;
+  const int occ =
+      prepare_launch((const void *)k_square, cache, dyn, kStageThreads, &err);
+  if (err != cudaSuccess) return err;
+  const uint32_t grid = (uint32_t)std::min<uint64_t>(
+      g.nitems, (uint64_t)device_info().sms * std::max(occ, 1));
+  ProfScope ps(s, "square");
+  k_square<<<grid, kStageThreads, dyn, s>>>(g);
   return cudaGetLastError();
 }
 

@@ -86,6 +86,8 @@ struct TuneParams {
   uint32_t staged_wide = 0;
   // staged form: no extra rows for unaligned narrow blocks (lm_batch.cu)
   uint32_t staged_plain = 0;
+  // staged form's blocks for a square: this many rows and columns
+  uint32_t square = 0;
 };
 TuneParams &tune_params();
 
@@ -210,6 +212,15 @@ bool staged0100_applies(uint64_t T, uint64_t a, uint64_t B, uint64_t b, int e);
 cudaError_t launch_staged0100(cudaStream_t s, void *buf, int e, uint64_t T,
                               uint64_t a, uint64_t B, uint64_t b,
                               void *scratch);
+
+// ---- square 0100s (lm_batch.cu) ----------------------------------------------
+// T squares of a x a units, block pairs exchanged through shared memory: 2 x
+// payload, no scratch, nothing waits for another CTA.
+bool square0100_applies(const void *buf, uint64_t T, uint64_t a, uint64_t B,
+                        uint64_t b, int e);
+cudaError_t launch_square0100(cudaStream_t s, void *buf, int e, uint64_t T,
+                              uint64_t a, uint64_t b, uint32_t *status,
+                              uint64_t timeout_ns);
 
 // ---- 0100 held whole in shared memory (lm_batch.cu) -------------------------
 // Payloads that fit the shared memory of all SMs (about 30 MB on GB300): the
