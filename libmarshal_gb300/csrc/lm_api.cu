@@ -283,6 +283,9 @@ static uint64_t wait_timeout_ns() {
 // ---- planner ----------------------------------------------------------------
 
 constexpr uint64_t kWalkMinBytes = 16ull << 20;
+// (what is smaller is held in shared memory, or, under capture, leaves too
+// few steps)
+constexpr uint64_t kWaveMinBytes = 32ull << 20;
 
 enum class Method { Auto, BS, Pttwac, Stash, TwoPass, Cycles, Staged, Resident };
 
@@ -478,38 +481,17 @@ static bool do_0100(cudaStream_t s, void *buf, int e, uint64_t T, uint64_t a,
                          cs == cudaStreamCaptureStatusNone),
           "walk launch");
   }
-  // the stash wavefront spreads rows over all CTAs: with too few rows per
-  // SM its steps are too small to keep HBM busy
-  const uint64_t stash_min_rows = kStashRowsPerSm * (uint64_t)device_info().sms;
-  const bool want_stash =
-      m == Method::Stash ||
-      (m == Method::Auto && T == 1 && U < 128 && a * B >= (1ull << 20) &&
-       a >= stash_min_rows && !getenv("LM_NO_STASH"));
-  if (want_stash) {
-    // 100 on small units: the 3 x payload streaming plan (lm_stash.cu).
-    StashPlan sp = T == 1 ? plan_stash(a, B, (uint32_t)b, e) : StashPlan();
-    // very tall matrices leave each CTA short strips (a step's rows x strip
-    // must fit shared memory); below 384-byte strips the staged form moves
-    // units of 4 bytes and more faster (fp64 32768 x 16000: 3.06 TB/s by
-    // the stash with 256-byte strips, 3.24 TB/s staged)
-    if (m == Method::Auto && sp.feasible && U >= 4 && sp.g * U < 384 &&
-        staged0100_applies(T, a, B, b, e))
-      sp = StashPlan();
-    uint32_t *status = sp.feasible ? device_status_word() : nullptr;
-    if (sp.feasible && status) {
-      // the stash (about half the payload) may not be available: then the
-      // plans below, which need less scratch, take over
-      Scratch sc;
-      if (try_scratch(sc, stash_scratch_bytes(sp), s))
-        return check_launch(launch_stash100(s, buf, e, a, B, (uint32_t)b, sp,
-                                            sc.p, status, wait_timeout_ns()),
-                            "stash launch");
-      if (m == Method::Stash) return fail("stash: no scratch for this size");
-    }
-    if (m == Method::Stash)
-      return fail("stash plan not applicable to 0100(%llu, %llu, %llu, %llu)",
-                  (unsigned long long)T, (unsigned long long)a,
-                  (unsigned long long)B, (unsigned long long)b);
+  // a large matrix at 3 x payload: half of its blocks in place, the others
+  // through scratch (lm_batch.cu, k_wave)
+  if (m == Method::Auto && T == 1 && U < kStagedMaxUnit &&
+      a * B * U >= kWaveMinBytes && !getenv("LM_NO_WAVE")) {
+    const size_t need = wave0100_scratch(buf, a, B, b, e);
+    uint32_t *status = need ? device_status_word() : nullptr;
+    Scratch sc;
+    if (need && status && try_scratch(sc, need, s))
+      return check_launch(launch_wave0100(s, buf, e, a, B, b, sc.p, status,
+                                          wait_timeout_ns()),
+                          "wave launch");
   }
   // any shape through scratch: block transposes out of place, then a copy
   // back (4 x payload, but every access in whole sectors); falls through
@@ -537,6 +519,33 @@ static bool do_0100(cudaStream_t s, void *buf, int e, uint64_t T, uint64_t a,
     } else if (m == Method::Staged) {
       return fail("staged: units above 32 KB or too many blocks");
     }
+  }
+  // the stash plan moves 3 x payload with half the scratch, where the forms
+  // above could not have theirs.  Its wavefront spreads rows over all CTAs:
+  // with too few rows per SM its steps are too small to keep HBM busy
+  const uint64_t stash_min_rows = kStashRowsPerSm * (uint64_t)device_info().sms;
+  const bool want_stash =
+      m == Method::Stash ||
+      (m == Method::Auto && T == 1 && U < 128 && a * B >= (1ull << 20) &&
+       a >= stash_min_rows && !getenv("LM_NO_STASH"));
+  if (want_stash) {
+    // 100 on small units: the 3 x payload streaming plan (lm_stash.cu).
+    StashPlan sp = T == 1 ? plan_stash(a, B, (uint32_t)b, e) : StashPlan();
+    uint32_t *status = sp.feasible ? device_status_word() : nullptr;
+    if (sp.feasible && status) {
+      // the stash (about half the payload) may not be available: then the
+      // plans below, which need less scratch, take over
+      Scratch sc;
+      if (try_scratch(sc, stash_scratch_bytes(sp), s))
+        return check_launch(launch_stash100(s, buf, e, a, B, (uint32_t)b, sp,
+                                            sc.p, status, wait_timeout_ns()),
+                            "stash launch");
+      if (m == Method::Stash) return fail("stash: no scratch for this size");
+    }
+    if (m == Method::Stash)
+      return fail("stash plan not applicable to 0100(%llu, %llu, %llu, %llu)",
+                  (unsigned long long)T, (unsigned long long)a,
+                  (unsigned long long)B, (unsigned long long)b);
   }
   if ((m == Method::Auto && U < 128) || m == Method::TwoPass) {
     // Aggregate small super-elements into >=128-byte units first so the

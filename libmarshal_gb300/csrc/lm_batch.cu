@@ -852,6 +852,50 @@ __device__ __forceinline__ void store_b1_ragged(
   }
 }
 
+// store_b1_ragged for 4- and 8-byte elements: a lane gathers the RW = 16/E
+// rows of its vector from its column, wherever they start.
+template <int E>
+__device__ __forceinline__ void store_b1_ragw(
+    const unsigned char *buf, const uint32_t *rowoff, uint32_t S,
+    uint32_t nrows, bool first, uint32_t ncols, typename Elem<E>::T *dst,
+    uint32_t ostride, uint32_t warp, uint32_t nwarps) {
+  static_assert(E == 4 || E == 8, "wide elements only");
+  using T = typename Elem<E>::T;
+  constexpr uint32_t RW = 16 / E;
+  const uint32_t lane = threadIdx.x & 31;
+  const uint32_t ng = S / RW, ngc = (ng + 7) / 8, nd = (ncols + 3) / 4;
+  for (uint32_t u = warp; u < ngc * nd; u += nwarps) {
+    const uint32_t d = u / ngc, gc = u - d * ngc;
+    const uint32_t g = gc * 8 + (lane & 7), jj = d * 4 + (lane >> 3);
+    if (g >= ng || jj >= ncols) continue;
+    T *run = dst + (uint64_t)jj * ostride;
+    const uint32_t h = (16 - (uint32_t)((uintptr_t)run & 15)) / E % RW;
+    const uint32_t r0 = g * RW + h;
+    if (r0 + RW > nrows) continue;
+    const unsigned char *col = buf + jj * E;
+    T v[RW];
+#pragma unroll
+    for (uint32_t k = 0; k < RW; ++k)
+      v[k] = *reinterpret_cast<const T *>(col + rowoff[r0 + k]);
+    __stcg(reinterpret_cast<uint4 *>(run + r0), pack16<E>(v));
+  }
+  const bool end = nrows < S + RW - 1;
+  if (!first && !end) return;
+  for (uint32_t x = warp * 32 + lane; x < ncols * RW; x += nwarps * 32) {
+    const uint32_t jj = x / RW, k = x % RW;
+    T *run = dst + (uint64_t)jj * ostride;
+    const uint32_t h = (16 - (uint32_t)((uintptr_t)run & 15)) / E % RW;
+    auto put = [&](uint32_t r) {
+      __stcg(run + r, *reinterpret_cast<const T *>(buf + rowoff[r] + jj * E));
+    };
+    if (first && k < min(h, nrows)) put(k);
+    if (end && nrows > h) {
+      const uint32_t r = h + (nrows - h) / RW * RW + k;
+      if (r < nrows && r < S + h) put(r);
+    }
+  }
+}
+
 // For blocks of whole columns (S = a) the block's output is one
 // contiguous range of n = a * ncols elements, written in the 16-byte vectors
 // of its alignment whatever the column length; a vector's elements run down
@@ -1138,7 +1182,7 @@ struct GBlock {
   uint32_t t, i0, j0, si, sj;
 };
 
-template <bool RAG>
+template <int RAG>
 __device__ __forceinline__ GBlock gather_decode(const BJob &j, uint32_t q) {
   GBlock k;
   k.t = fdiv(q, j.div_nIJ);
@@ -1165,9 +1209,10 @@ struct RowCopy {
   uint32_t dst;    // offset in the stage
 };
 
-template <int NT, bool RAG>
+template <int NT, int RAG>
 __device__ __forceinline__ RowCopy gather_row_plan(const BJob &j, uint32_t q,
-                                                   uint32_t *rowoff) {
+                                                   uint32_t *rowoff,
+                                                   uint32_t lim = 0) {
   RowCopy c{0, 0, 0};
   const GBlock k = gather_decode<RAG>(j, q);
   if (RAG && j.contig) {
@@ -1178,7 +1223,7 @@ __device__ __forceinline__ RowCopy gather_row_plan(const BJob &j, uint32_t q,
     const uint32_t m0 = (uint32_t)(src & 15);
     const uint32_t all = (m0 + k.si * j.pitch + 15) & ~15u;
     const uint32_t piece = (all + NT / 2 - 1) / (NT / 2) * 16;
-    if (j.ragged == 1) {
+    if (j.ragged == 1 && j.e <= 2) {
       if (threadIdx.x == 0) rowoff[0] = m0;
     } else {
       for (uint32_t r = threadIdx.x; r < k.si; r += NT)
@@ -1203,15 +1248,18 @@ __device__ __forceinline__ RowCopy gather_row_plan(const BJob &j, uint32_t q,
     return c;
   }
   const uint32_t r = (threadIdx.x & 31) * (NT / 32) + (threadIdx.x >> 5);
-  const uint32_t tr = RAG && j.ragged == 1 ? rag_index(r, j.e) : r;
-  if (RAG && j.ragged == 1) {
+  const bool rag = (RAG & 1) && j.ragged == 1 && j.e <= 2;
+  const uint32_t tr = rag ? rag_index(r, j.e) : r;
+  if (rag) {
     if (r >= k.si && tr < j.tab) rowoff[tr] = 0;
   }
   if (r >= k.si) return c;
   const uint32_t len = k.sj * j.b * j.e;
-  const uintptr_t src = (uintptr_t)(j.base + ((uint64_t)k.t * j.tile_elems +
-                                              (uint64_t)(k.i0 + r) * j.row_elems +
-                                              (uint64_t)k.j0 * j.b) * j.e);
+  // (rows of the job below `lim` come from the scratch)
+  const char *base = k.i0 + r < lim ? j.scratch : j.base;
+  const uintptr_t src = (uintptr_t)(base + ((uint64_t)k.t * j.tile_elems +
+                                            (uint64_t)(k.i0 + r) * j.row_elems +
+                                            (uint64_t)k.j0 * j.b) * j.e);
   c.src = src & ~(uintptr_t)15;
   c.bytes = (uint32_t)(((src + len + 15) & ~(uintptr_t)15) - c.src);
   // vectorized narrow stores: the rows of group r / vrw shifted by 16 bytes
@@ -1219,8 +1267,8 @@ __device__ __forceinline__ RowCopy gather_row_plan(const BJob &j, uint32_t q,
   // consecutive groups a warp reads at once fall in distinct bank groups
   c.dst = r * j.pitch + (j.vrw ? 16 * (r / j.vrw) : 0);
   const uint32_t m = (uint32_t)(src - c.src);
-  rowoff[tr] = c.dst + (RAG && j.ragged == 1 ? m & ~3u : m);
-  if (RAG && j.ragged == 1 && r == 0) rowoff[16 / j.e] = m;
+  rowoff[tr] = c.dst + (rag ? m & ~3u : m);
+  if (rag && r == 0) rowoff[16 / j.e] = m;
   return c;
 }
 
@@ -1234,12 +1282,14 @@ __device__ __forceinline__ void gather_row_issue(const RowCopy &c,
 
 // All threads: output rows j0..j0+sj-1 of the block, each si*b elements
 // long, from the staged rows.
-template <int E, int NT, bool RAG>
-__device__ void gather_store(const BJob &j, uint32_t q, const unsigned char *buf,
-                             const uint32_t *rowoff) {
+// (block k, written to `out`, which is laid out as the buffer)
+template <int E, int NT, int RAG>
+__device__ __forceinline__ void gather_store_at(const BJob &j, const GBlock &k,
+                                                char *out,
+                                                const unsigned char *buf,
+                                                const uint32_t *rowoff) {
   using T = typename Elem<E>::T;
-  const GBlock k = gather_decode<RAG>(j, q);
-  T *dst = reinterpret_cast<T *>(j.scratch) + (uint64_t)k.t * j.tile_elems +
+  T *dst = reinterpret_cast<T *>(out) + (uint64_t)k.t * j.tile_elems +
            ((uint64_t)k.j0 * j.a + k.i0) * j.b;
   if (j.nv16) {
     // whole 16-byte vectors: lanes on consecutive vectors of a column's
@@ -1274,7 +1324,7 @@ __device__ void gather_store(const BJob &j, uint32_t q, const unsigned char *buf
         return;
       }
     }
-    if constexpr (RAG && E <= 2) {
+    if constexpr ((RAG & 1) && E <= 2) {
       if (j.ragged == 2) {
         store_b1_flat<E>(buf, j.a, j.div_a, k.sj * j.a, dst, threadIdx.x,
                          NT, j.pitch, rb, rowoff[0] & 15);
@@ -1289,6 +1339,13 @@ __device__ void gather_store(const BJob &j, uint32_t q, const unsigned char *buf
         else
           store_b1_ragged<E, false>(buf, rowoff, j.S, k.si, k.i0 == 0, k.sj,
                                     dst, j.a, w, NT / 32, j.pitch, rb, 0);
+        return;
+      }
+    }
+    if constexpr ((RAG & 2) && E >= 4) {
+      if (j.ragged) {
+        store_b1_ragw<E>(buf, rowoff, j.S, k.si, k.i0 == 0, k.sj, dst, j.a,
+                         threadIdx.x >> 5, NT / 32);
         return;
       }
     }
@@ -1342,6 +1399,13 @@ __device__ void gather_store(const BJob &j, uint32_t q, const unsigned char *buf
   }
 }
 
+template <int E, int NT, int RAG>
+__device__ void gather_store(const BJob &j, uint32_t q, const unsigned char *buf,
+                             const uint32_t *rowoff) {
+  gather_store_at<E, NT, RAG>(j, gather_decode<RAG>(j, q), j.scratch, buf,
+                              rowoff);
+}
+
 // Persistent: every CTA walks blocks (claimed item by item from the work
 // counter) with two shared-memory stages, loading block n+1 by bulk copies
 // (issued by all warps) while it writes block n.
@@ -1352,11 +1416,11 @@ __device__ void gather_store(const BJob &j, uint32_t q, const unsigned char *buf
 // 16384 x 16384 the other way: 0.126 vs 0.121 ms).
 // RAG: with the code of ragged blocks and of rows staged as one range (in a
 // kernel of its own: it takes 128 registers).
-template <int MB, bool RAG>
+template <int MB, int RAG>
 __global__ void __launch_bounds__(kStageThreads, MB) k_batch_gather(BatchArgs g) {
   extern __shared__ __align__(128) unsigned char smem[];
   __shared__ __align__(8) uint64_t bar[2];
-  __shared__ __align__(16) uint32_t rowoff[2][RAG ? kRowTable : kStageMaxS];
+  __shared__ __align__(16) uint32_t rowoff[2][RAG & 1 ? kRowTable : kStageMaxS];
   __shared__ uint32_t s_job[2], s_q[2], s_valid[2];
   __shared__ int s_dead;
   __shared__ __align__(16) BJob s_jobs[2];  // job of the block in each stage
@@ -1889,6 +1953,8 @@ static bool staged_job(BJob &j, const lm_job &jb, const Normalized &nz,
     while (S > 1 && S * S * unit > kStageTileBytes) S >>= 1;
     Si = Sj = S;
     if (tune_params().staged_wide > 1) Sj = S * tune_params().staged_wide;
+    if (!tune_params().staged_wide && 2 * S * S * unit <= kStageTileBytes)
+      Si = 2 * S;
   }
   if (tune_params().square) Si = Sj = tune_params().square;
   Si = std::min<uint64_t>(Si, nz.a);
@@ -1947,12 +2013,23 @@ static bool staged_job(BJob &j, const lm_job &jb, const Normalized &nz,
       j.ragged = 2;
       if (Sj > RW && Sj < nz.B) Sj = Sj / RW * RW;
     }
-  } else if (nz.b == 1 && nz.e >= 4 && Sj == nz.B &&
-             (nz.B % 2 || row <= 256) && !tune_params().staged_plain) {
+  } else if (nz.b == 1 && nz.e >= 4 && !tune_params().staged_plain &&
+             Sj == nz.B && (nz.B % 2 || row <= 256)) {
     // the same for wider elements: 10^7 x 17 floats 724 us with a copy per
     // row, 513 as one range; 6 10^6 x 20 429 and 336, 3 10^6 x 64 512 and
     // 473, 6 10^6 x 4 doubles 266 and 243
     j.contig = nz.B % 2 ? 1 : 2;
+  }
+  if (nz.b == 1 && nz.e >= 4 && !tune_params().staged_plain && Si < nz.a &&
+      (((uintptr_t)jb.buf & 15) || (nz.a * nz.e) % 16)) {
+    // 4- and 8-byte elements whose output rows are not whole vectors
+    // (store_b1_ragw)
+    const uint64_t R = 16 / nz.e;
+    Si = std::min<uint64_t>(Si, kStageMaxS - R) / R * R;
+    if (Si >= 8 * R) {
+      j.ragged = 1;
+      j.extra = (uint16_t)(R - 1);
+    }
   }
   const uint64_t nI = (nz.a + Si - 1) / Si, nJ = (nz.B + Sj - 1) / Sj;
   if (nz.T * nI * nJ >= 0xffffffffull) return false;
@@ -1981,7 +2058,8 @@ static bool staged_job(BJob &j, const lm_job &jb, const Normalized &nz,
         break;
       }
   j.tab = S;  // (kRowTable words at most)
-  if (j.ragged == 1 && j.contig) j.tab = 4;
+  if (j.ragged && nz.e >= 4) j.tab = S + j.extra;
+  else if (j.ragged == 1 && j.contig) j.tab = 4;
   else if (j.ragged == 1) j.tab = (S * nz.e / 16 + 1) * (16 / nz.e + 4);
   j.vrw = j.contig ? 0 : j.vb1 || j.ragged ? 16 / nz.e : j.vbc / nz.e;
   j.div_nv16 = make_fastdiv(j.nv16 ? j.nv16 : 1);
@@ -2331,7 +2409,7 @@ static bool launch_staged(cudaStream_t s, const BJob *d_jobs,
                           uint32_t *counter, size_t smem, bool copyback) {
   if (nitems == 0) return false;
   const DeviceInfo &di = device_info();
-  auto kern = copyback ? k_batch_copyback : k_batch_gather<3, false>;
+  auto kern = copyback ? k_batch_copyback : k_batch_gather<3, 0>;
   // the gather keeps two stages of `smem` bytes
   const size_t dyn = copyback ? 0 : 2 * smem;
   static LaunchCache copy_cache;
@@ -2397,15 +2475,15 @@ cudaError_t launch_staged0100(cudaStream_t s, void *buf, int e, uint64_t T,
   if (!staged_job(g.single, jb, nz, &nblk, &stage)) return cudaErrorInvalidValue;
   g.single.scratch = reinterpret_cast<char *>(scratch);
   const bool rag = g.single.ragged || g.single.contig, two = e == 2;
-  auto gather = rag   ? k_batch_gather<2, true>
-                : two ? k_batch_gather<2, false>
-                      : k_batch_gather<3, false>;
+  auto gather = rag   ? e <= 2 ? k_batch_gather<2, 1> : k_batch_gather<3, 2>
+                : two ? k_batch_gather<2, 0>
+                      : k_batch_gather<3, 0>;
   const size_t dyn = 2 * stage;
   cudaError_t err = cudaSuccess;
-  static LaunchCache rag_cache, two_cache;
+  static LaunchCache rag_cache[2], two_cache;
   const int occ = prepare_launch(
       (const void *)gather,
-      rag ? rag_cache : two ? two_cache : g_gather3_cache, dyn, kStageThreads,
+      rag ? rag_cache[e <= 2] : two ? two_cache : g_gather3_cache, dyn, kStageThreads,
       &err);
   if (err != cudaSuccess) return err;
   const DeviceInfo &di = device_info();
@@ -2436,6 +2514,367 @@ cudaError_t launch_staged0100(cudaStream_t s, void *buf, int e, uint64_t T,
       reinterpret_cast<char *>(buf), reinterpret_cast<const char *>(scratch),
       g.single.bytes);
   return cudaGetLastError();
+}
+
+// ---- one large 0100 at 3 x payload -------------------------------------------
+// The staged form transposes every block into scratch and copies all of it
+// back.  In an order of blocks, half of that is not needed:
+//  * backward (tall matrices): block rows from the last to the first.  A
+//    block's output whose place lies in rows that have been read goes
+//    straight there, the rest to scratch (laid out as the buffer).  The place
+//    of output row j, position i is source address j*A + i, so what a block
+//    row writes directly are the output rows from some j on, and what is left
+//    in scratch of output row j is a suffix, copied back at the end;
+//  * forward (wide ones), the same backwards in time: block columns from the
+//    first to the last, every block written straight to its place.  Of each
+//    source row the suffix that will be overwritten before it is read is
+//    copied to scratch first, and read from there.
+// Either way a step (block row or block column) s may be written over once
+// all blocks of steps up to s - M are staged: M steps of slack, counted per
+// step, let the CTAs (which take blocks from a ticket) run without waiting
+// for one another.  The payload moves 2 x and half of it (plus M steps)
+// twice more.
+struct WaveArgs {
+  BJob job;
+  uint32_t nsteps, per;  // blocks of a step
+  uint32_t group, gper;  // steps and blocks of a count
+  uint32_t nblk, M, backward;
+  uint32_t stage_bytes;
+  uint32_t lines;        // step: rows or columns of its blocks
+  uint32_t *ticket;      // then the counts
+  uint32_t *status;
+  uint64_t timeout_ns;
+  FastDiv div_per, div_group, div_len;  // div_len: A (backward) or B (forward)
+};
+
+// Units whose places are not free (backward) or have been overwritten
+// (forward) at step s: output rows below it go to scratch, source rows below
+// it come from there.  L = step lines x (s' + M), s' the step's place in the
+// matrix: everything before line L may be unread or overwritten.
+__device__ __forceinline__ uint32_t wave_split(const WaveArgs &g, uint32_t at,
+                                               uint32_t M, uint32_t len,
+                                               uint32_t other) {
+  const uint64_t L = (uint64_t)(at + M) * g.lines;
+  if (L >= len) return other;
+  // ceil((L * other - at * lines) / len), all below 2^32
+  return fdiv((uint32_t)(L * other - (uint64_t)at * g.lines + len - 1),
+              g.div_len);
+}
+
+template <int MB, int RAG>
+__global__ void __launch_bounds__(kStageThreads, MB) k_wave(WaveArgs g) {
+  extern __shared__ __align__(128) unsigned char smem[];
+  __shared__ __align__(8) uint64_t bar[2];
+  __shared__ __align__(16) uint32_t rowoff[2][RAG & 1 ? kRowTable : kStageMaxS];
+  __shared__ __align__(16) BJob s_job;
+  __shared__ uint32_t s_n[2], s_split[2];
+  __shared__ int s_dead;
+  const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  uint32_t *done = g.ticket + 1;
+  uint32_t claimed = 0;   // thread 0: the block after the next
+  uint32_t frontier = 0;  // warp 1: groups of steps seen staged
+  auto block_of = [&](uint32_t n, uint32_t *s) {
+    *s = fdiv(n, g.div_per);
+    const uint32_t r = n - *s * g.per;
+    return g.backward ? (g.nsteps - 1 - *s) * g.per + r
+                      : r * g.job.nJ + *s;
+  };
+  auto fetch = [&](int slot) {
+    const uint32_t n = claimed;
+    claimed = atomicAdd(g.ticket, 1u);  // looked at a block later
+    s_n[slot] = n;
+    if (n >= g.nblk) return;
+    const uint32_t s = fdiv(n, g.div_per);
+    if (g.backward) {
+      // (blocks that stage rows of the next one keep that one's place, too)
+      const uint32_t k = g.nsteps - 1 - s;
+      uint32_t sp = wave_split(g, k, g.M + (RAG ? 1 : 0), g.job.a, g.job.B);
+      const uint32_t q = g.job.b == 1 && g.job.e < 4 ? 4 / g.job.e : 1;
+      s_split[slot] = (sp + q - 1) / q * q;  // whole staged words
+    } else {
+      s_split[slot] = wave_split(g, s, g.M, g.job.B, g.job.a);
+    }
+  };
+  auto issue = [&](int slot) {
+    uint32_t s;
+    const uint32_t q = block_of(s_n[slot], &s);
+    const RowCopy rc = gather_row_plan<kStageThreads, RAG>(
+        s_job, q, rowoff[slot], g.backward ? 0 : s_split[slot]);
+    gather_arrive(&bar[slot], rc.bytes);
+    __syncthreads();  // every warp's expected bytes before any copy
+    gather_row_issue(rc, smem + (size_t)slot * g.stage_bytes, &bar[slot]);
+  };
+  if (threadIdx.x == 0) {
+    mbar_init(&bar[0], kStageThreads / 32);
+    mbar_init(&bar[1], kStageThreads / 32);
+    fence_mbar_init();
+    s_dead = 0;
+    claimed = atomicAdd(g.ticket, 1u);
+    fetch(0);
+  }
+  if (warp == 0) copy_job(&s_job, &g.job);
+  __syncthreads();
+  if (s_n[0] >= g.nblk) return;
+  issue(0);
+  bool more = false;
+  uint32_t n = 0;
+  for (;; ++n) {
+    const int st = n & 1, nx = st ^ 1;
+    if (threadIdx.x == 0) fetch(nx);
+    __syncthreads();  // slot nx visible; stage nx free since the last pass
+    more = s_n[nx] < g.nblk;
+    if (more) issue(nx);
+    uint32_t s;
+    const uint32_t q = block_of(s_n[st], &s);
+    if (warp == 1 && s >= g.M) {
+      // every block of the steps up to s - M is staged (the counts are read
+      // while this block's copies land; a bounded wait where they are short)
+      const uint32_t need = fdiv(s - g.M, g.div_group) + 1;
+      const uint64_t t0 = global_timer_ns();
+      while (frontier < need) {
+        const uint32_t f = frontier + lane;
+        const bool full = f < need && ld_acquire_gpu(done + f) >= g.gper;
+        const unsigned mask = ~__ballot_sync(kFull, full);
+        frontier += mask ? __ffs(mask) - 1 : 32;
+        if (frontier < need && (s_dead || global_timer_ns() - t0 > g.timeout_ns)) {
+          s_dead = 1;
+          break;
+        }
+      }
+    }
+    const uint64_t t0 = global_timer_ns();
+    while (!mbar_try_wait(&bar[st], (n >> 1) & 1))
+      if (global_timer_ns() - t0 > g.timeout_ns) {
+        s_dead = 1;
+        break;
+      }
+    __syncthreads();  // staged for everyone, and its place is free
+    if (s_dead) break;
+    // (relaxed: the copies have completed, and a release would wait for this
+    // thread's stores of the last block)
+    if (threadIdx.x == 0) red_relaxed_gpu(done + fdiv(s, g.div_group), 1u);
+    const unsigned char *buf = smem + (size_t)st * g.stage_bytes;
+    const GBlock k = gather_decode<RAG>(s_job, q);
+    const uint32_t split = s_split[st];
+    for (int part = 0; part < 2; ++part) {
+      // backward: output rows below the split to scratch, the others in place
+      GBlock p = k;
+      const unsigned char *b = buf;
+      char *out = s_job.base;
+      if (g.backward) {
+        const uint32_t cut = split > k.j0 ? min(split - k.j0, k.sj) : 0u;
+        if (part == 0) {
+          p.sj = cut;
+          out = s_job.scratch;
+        } else {
+          p.j0 += cut;
+          p.sj -= cut;
+          b += cut * s_job.b * s_job.e;
+        }
+        if (p.sj == 0) continue;
+      } else if (part == 0) {
+        continue;
+      }
+      switch (s_job.e) {
+        case 1:
+          gather_store_at<1, kStageThreads, RAG>(s_job, p, out, b, rowoff[st]);
+          break;
+        case 2:
+          gather_store_at<2, kStageThreads, RAG>(s_job, p, out, b, rowoff[st]);
+          break;
+        case 4:
+          gather_store_at<4, kStageThreads, RAG>(s_job, p, out, b, rowoff[st]);
+          break;
+        default:
+          gather_store_at<8, kStageThreads, RAG>(s_job, p, out, b, rowoff[st]);
+      }
+    }
+    __syncthreads();  // stage st and slot st are free
+    if (!more) return;
+  }
+  // a wait that ran out: report it; nothing may still be landing in shared
+  // memory when the CTA exits
+  if (threadIdx.x == 0 && g.status) atomicExch(g.status, kStatusWaitTimeout);
+  for (uint32_t m = n; m < n + (more ? 2u : 1u); ++m) {
+    const uint64_t t1 = global_timer_ns();
+    while (!mbar_try_wait(&bar[m & 1], (m >> 1) & 1) &&
+           global_timer_ns() - t1 < g.timeout_ns) {
+    }
+  }
+}
+
+// The suffixes of the `rows` lines of `len` units of U bytes that k_wave
+// leaves in scratch (backward: output rows, dst = the buffer) or reads from
+// there (forward: source rows, dst = the scratch): line i from unit
+// first(i) on.  A warp copies a piece of 4 KB at a time, 16-byte vectors at
+// the equal alignments of the two, bytes at the ends.
+struct SuffixArgs {
+  char *dst;
+  const char *src;
+  uint64_t rows, len;
+  uint32_t U, lines, M;
+  uint32_t q;        // lines share the suffix of the multiple of q before them
+  uint32_t rag;      // e: bytes of elements of ragged blocks
+  uint32_t *clear;   // forward: the wave's ticket and counts, to be zero
+  uint32_t nclear;
+};
+
+__device__ __forceinline__ uint64_t suffix_first(const SuffixArgs &g,
+                                                 uint64_t i) {
+  // smallest step whose split (wave_split) lies beyond line i
+  const uint64_t P = i / g.q * g.q * g.len;
+  const uint64_t thr = (uint64_t)g.M * g.lines * g.rows;
+  if (P < thr) return 0;
+  uint64_t f = ((P - thr) / ((uint64_t)g.lines * (g.rows - 1)) + 1) * g.lines;
+  if (g.rag)  // a ragged block's share starts at a vector boundary
+    f += ((16 - ((uintptr_t)(g.dst + i * g.len * g.U) & 15)) & 15) / g.rag;
+  return f;
+}
+
+__global__ void __launch_bounds__(kStageThreads) k_suffix_copy(SuffixArgs g) {
+  constexpr uint64_t kPiece = 4096;
+  const uint32_t lane = threadIdx.x & 31;
+  for (uint32_t x = blockIdx.x * kStageThreads + threadIdx.x; x < g.nclear;
+       x += gridDim.x * kStageThreads)
+    g.clear[x] = 0u;
+  const uint64_t row = g.len * g.U, total = g.rows * row;
+  const uint64_t mis = (uintptr_t)g.dst & 15;
+  const uint64_t np = (total + mis + kPiece - 1) / kPiece;
+  const uint64_t warps = (uint64_t)gridDim.x * (kStageThreads / 32);
+  for (uint64_t p = (uint64_t)blockIdx.x * (kStageThreads / 32) +
+                    (threadIdx.x >> 5);
+       p < np; p += warps) {
+    uint64_t x = p ? p * kPiece - mis : 0;
+    const uint64_t end = min64(total, (p + 1) * kPiece - mis);
+    for (uint64_t i = x / row; x < end; ++i) {
+      const uint64_t y = min64(end, (i + 1) * row);
+      const uint64_t from = max(x, i * row + min64(suffix_first(g, i), g.len) * g.U);
+      x = y;
+      if (from >= y) continue;
+      const uint64_t v0 = min64(y, ((from + mis + 15) & ~(uint64_t)15) - mis);
+      const uint64_t nv = (y - v0) / 16;
+      const uint32_t nh = (uint32_t)(v0 - from), nt = (uint32_t)(y - v0 - nv * 16);
+      if (lane < nh) g.dst[from + lane] = g.src[from + lane];
+      if (lane < nt) g.dst[y - nt + lane] = g.src[y - nt + lane];
+      const uint4 *vs = reinterpret_cast<const uint4 *>(g.src + v0);
+      uint4 *vd = reinterpret_cast<uint4 *>(g.dst + v0);
+      uint4 v[8];
+#pragma unroll
+      for (int u = 0; u < 8; ++u)
+        if (lane + 32 * u < nv) v[u] = __ldcs(vs + lane + 32 * u);
+#pragma unroll
+      for (int u = 0; u < 8; ++u)
+        if (lane + 32 * u < nv) __stcs(vd + lane + 32 * u, v[u]);
+    }
+  }
+}
+
+// Geometry of the ordered form; false where it does not apply or its slack
+// would leave little of the half that it saves.
+static bool plan_wave(WaveArgs &g, size_t *scratch, void *buf, uint64_t a,
+                      uint64_t B, uint64_t b, int e) {
+  lm_job jb{};
+  jb.buf = buf;
+  jb.elem_bytes = e;
+  Normalized nz;
+  nz.ok = true;
+  nz.e = e;
+  nz.T = 1;
+  nz.a = a;
+  nz.B = B;
+  nz.b = b;
+  // (wave_split stays below 2^32)
+  if (a < 2 || B < 2 || a * B + a + B >= 0xffffffffull) return false;
+  uint64_t nblk = 0;
+  size_t stage = 0;
+  if (!staged_job(g.job, jb, nz, &nblk, &stage) || nblk >= 0x7fffffffull ||
+      2 * stage + 8192 > (size_t)device_info().max_smem_optin)
+    return false;
+  const uint32_t nJ = g.job.nJ, nI = g.job.nIJ / nJ;
+  // slack: twice what the CTAs write from, which is what they hold; counted
+  // over 128 blocks and more (a CTA reads 32 counts at a time)
+  const uint32_t blocks = (uint32_t)device_info().sms * 4;
+  auto slack = [&](uint32_t per) {
+    return (blocks + per - 1) / per + std::max<uint32_t>(1, 128 / per);
+  };
+  // forward unless its slack is more than an eighth of its steps and
+  // backward's is less (20003 x 5001 floats 212 us forward, 218 backward;
+  // 20003 x 15001 half-words 423 and 447; 125000 x 101 units of 32 bytes 268
+  // and 203)
+  const uint64_t mf = slack(nI), mb = slack(nJ);
+  g.backward = mf * 8 > nJ && mf * nI > mb * nJ;
+  g.nsteps = g.backward ? nI : nJ;
+  g.per = g.backward ? nJ : nI;
+  g.lines = g.backward ? g.job.S : g.job.Sj;
+  g.nblk = (uint32_t)nblk;
+  g.stage_bytes = (uint32_t)stage;
+  g.group = std::max<uint32_t>(1, 128 / g.per);
+  g.gper = g.group * g.per;
+  g.M = slack(g.per);
+  if ((uint64_t)g.M * 3 > g.nsteps) return false;
+  g.div_per = make_fastdiv(g.per);
+  g.div_group = make_fastdiv(g.group);
+  g.div_len = make_fastdiv((uint32_t)(g.backward ? a : B));
+  *scratch = (size_t)((g.job.bytes + 16 + 255) / 256 * 256) +
+             ((size_t)g.nsteps + 1) * 4;
+  return true;
+}
+
+size_t wave0100_scratch(void *buf, uint64_t a, uint64_t B, uint64_t b, int e) {
+  WaveArgs g{};
+  size_t scratch = 0;
+  return plan_wave(g, &scratch, buf, a, B, b, e) ? scratch : 0;
+}
+
+cudaError_t launch_wave0100(cudaStream_t s, void *buf, int e, uint64_t a,
+                            uint64_t B, uint64_t b, void *scratch,
+                            uint32_t *status, uint64_t timeout_ns) {
+  WaveArgs g{};
+  size_t need = 0;
+  if (!plan_wave(g, &need, buf, a, B, b, e)) return cudaErrorInvalidValue;
+  // the scratch copy sits at the buffer's address modulo 16
+  g.job.scratch = (char *)scratch + ((uintptr_t)buf & 15);
+  g.ticket = (uint32_t *)((char *)scratch + need - ((size_t)g.nsteps + 1) * 4);
+  g.status = status;
+  g.timeout_ns = timeout_ns;
+  cudaError_t err = cudaSuccess;
+  const uint32_t words = g.nsteps + 1;
+  if (g.backward &&
+      (err = cudaMemsetAsync(g.ticket, 0, (size_t)words * 4, s)) != cudaSuccess)
+    return err;
+  SuffixArgs c{};
+  if (!g.backward) c.clear = g.ticket, c.nclear = words;
+  c.dst = g.backward ? g.job.base : g.job.scratch;
+  c.src = g.backward ? g.job.scratch : g.job.base;
+  c.rows = g.backward ? B : a;
+  c.len = g.backward ? a : B;
+  c.U = (uint32_t)(b * e);
+  c.lines = g.lines;
+  const bool rag = g.job.ragged || g.job.contig;
+  c.M = g.M + (g.backward && rag ? 1 : 0);
+  c.q = g.backward && b == 1 && e < 4 ? 4 / e : 1;
+  c.rag = g.backward && g.job.ragged == 1 ? (uint32_t)e : 0;
+  const DeviceInfo &di = device_info();
+  auto copy = [&]() {
+    ProfScope ps(s, "suffix_copy");
+    k_suffix_copy<<<(unsigned)di.sms * 8, kStageThreads, 0, s>>>(c);
+    return cudaGetLastError();
+  };
+  if (!g.backward && (err = copy()) != cudaSuccess) return err;
+  {
+    auto kern = !rag ? k_wave<3, 0> : e <= 2 ? k_wave<2, 1> : k_wave<3, 2>;
+    static LaunchCache cache[3];
+    const size_t dyn = 2 * (size_t)g.stage_bytes;
+    const int occ = prepare_launch((const void *)kern, cache[!rag ? 0 : e <= 2 ? 1 : 2], dyn,
+                                   kStageThreads, &err);
+    if (err != cudaSuccess) return err;
+    const uint32_t grid = (uint32_t)std::min<uint64_t>(
+        (uint64_t)di.sms * std::max(occ, 1), g.nblk);
+    ProfScope ps(s, "wave");
+    kern<<<grid, kStageThreads, dyn, s>>>(g);
+    if ((err = cudaGetLastError()) != cudaSuccess) return err;
+  }
+  return g.backward ? copy() : cudaSuccess;
 }
 
 // ---- square 0100s ------------------------------------------------------------
@@ -2497,10 +2936,10 @@ __global__ void __launch_bounds__(kStageThreads, 3) k_square(SqArgs g) {
     square_pair(g, x, q);
     unsigned char *buf = smem + st * 2 * (size_t)g.stage_bytes;
     const RowCopy a =
-        gather_row_plan<kStageThreads, false>(s_job, q[0], rowoff[st][0]);
+        gather_row_plan<kStageThreads, 0>(s_job, q[0], rowoff[st][0]);
     RowCopy b{0, 0, 0};
     if (q[1] != q[0])
-      b = gather_row_plan<kStageThreads, false>(s_job, q[1], rowoff[st][1]);
+      b = gather_row_plan<kStageThreads, 0>(s_job, q[1], rowoff[st][1]);
     gather_arrive(&bar[st], a.bytes + b.bytes);
     __syncthreads();  // every warp's expected bytes before any copy
     gather_row_issue(a, buf, &bar[st]);
@@ -2529,10 +2968,10 @@ __global__ void __launch_bounds__(kStageThreads, 3) k_square(SqArgs g) {
       const unsigned char *b = buf + h * g.stage_bytes;
       const uint32_t *ro = rowoff[st][h];
       switch (s_job.e) {
-        case 1: gather_store<1, kStageThreads, false>(s_job, q[h], b, ro); break;
-        case 2: gather_store<2, kStageThreads, false>(s_job, q[h], b, ro); break;
-        case 4: gather_store<4, kStageThreads, false>(s_job, q[h], b, ro); break;
-        default: gather_store<8, kStageThreads, false>(s_job, q[h], b, ro);
+        case 1: gather_store<1, kStageThreads, 0>(s_job, q[h], b, ro); break;
+        case 2: gather_store<2, kStageThreads, 0>(s_job, q[h], b, ro); break;
+        case 4: gather_store<4, kStageThreads, 0>(s_job, q[h], b, ro); break;
+        default: gather_store<8, kStageThreads, 0>(s_job, q[h], b, ro);
       }
     }
     __syncthreads();  // stage st is free
@@ -2695,7 +3134,7 @@ __global__ void __launch_bounds__(kResThreads, 1) k_resident(ResArgs g) {
 #pragma unroll
   for (uint32_t k = 0; k < kResMaxBlocks; ++k)
     if (k < nmine) {
-      rc[k] = gather_row_plan<kResThreads, true>(s_job, blockIdx.x + k * gridDim.x,
+      rc[k] = gather_row_plan<kResThreads, 3>(s_job, blockIdx.x + k * gridDim.x,
                               rowoff + k * s_job.tab);
       bytes += rc[k].bytes;
     }
@@ -2737,10 +3176,10 @@ __global__ void __launch_bounds__(kResThreads, 1) k_resident(ResArgs g) {
       const unsigned char *buf = smem + (size_t)k * g.stage_bytes;
       const uint32_t *ro = rowoff + k * s_job.tab;
       switch (s_job.e) {
-        case 1: gather_store<1, kResThreads, true>(s_job, q, buf, ro); break;
-        case 2: gather_store<2, kResThreads, true>(s_job, q, buf, ro); break;
-        case 4: gather_store<4, kResThreads, true>(s_job, q, buf, ro); break;
-        default: gather_store<8, kResThreads, true>(s_job, q, buf, ro); break;
+        case 1: gather_store<1, kResThreads, 3>(s_job, q, buf, ro); break;
+        case 2: gather_store<2, kResThreads, 3>(s_job, q, buf, ro); break;
+        case 4: gather_store<4, kResThreads, 3>(s_job, q, buf, ro); break;
+        default: gather_store<8, kResThreads, 3>(s_job, q, buf, ro); break;
       }
     }
     return;
@@ -2809,7 +3248,7 @@ bool plan_resident(ResArgs &g, uint32_t *grid, size_t *dyn, void *buf,
                       12.5 * (double)(nper * stage) / 1024.0;
         // store_b1_ragged: the steps of a warp in a block, about 120 ns of the
         // CTA's time each
-        if (j.ragged == 1)
+        if (j.ragged == 1 && e <= 2)
           cost += 120.0 * (double)nper * ((j.S * e / 16 + 7) / 8) *
                   ((j.Sj * e + 15) / 16);
         if (!ok || cost < best_cost) {

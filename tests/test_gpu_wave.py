@@ -1,0 +1,88 @@
+"""Large single transpositions and SoA <-> ASTA conversions in the ordered form
+(k_wave), forward and backward, through the planner."""
+import pytest
+
+torch = pytest.importorskip("torch")
+
+from libmarshal_gb300 import lm
+
+pytestmark = pytest.mark.gpu
+
+
+def _check(a, B, b, e, offset=0, wave=True):
+    n = a * B * b * e
+    g = torch.Generator(device="cuda").manual_seed(a + offset)
+    raw = torch.randint(0, 256, (n + 64,), dtype=torch.uint8, device="cuda",
+                        generator=g)
+    before = raw.clone()
+    want = before[offset:offset + n].view(a, B, b * e).transpose(0, 1) \
+        .reshape(-1)
+    lm.prof_collect()
+    lm.prof_enable(True)
+    lm.transpose_100(raw.data_ptr() + offset, a, B, b, elem_bytes=e)
+    torch.cuda.synchronize()
+    lm.prof_enable(False)
+    ran = set(lm.prof_collect())
+    assert torch.equal(raw[offset:offset + n], want)
+    assert torch.equal(raw[:offset], before[:offset])
+    assert torch.equal(raw[offset + n:], before[offset + n:])
+    if wave:
+        assert ran == {"wave", "suffix_copy"}
+
+
+# output rows of whole vectors and not, both directions, last blocks of one
+# row or column, whole rows (one block column) and whole columns
+@pytest.mark.parametrize("a,B,b,e", [
+    (16000, 8192, 1, 1), (16001, 16385, 1, 1), (1001, 268167, 1, 1),
+    (268167, 1001, 1, 1), (149, 1500001, 1, 1), (12000001, 15, 1, 1),
+    (12000, 8000, 1, 2), (12001, 8003, 1, 2), (20003, 5001, 1, 2),
+    (3000001, 40, 1, 2), (18, 7000001, 1, 2),
+    (9001, 6000, 1, 4), (6000, 9001, 1, 4), (12289, 8193, 1, 4),
+    (1000001, 65, 1, 4), (106, 1178589, 1, 4), (5000001, 17, 1, 4),
+    (11871, 6065, 1, 8), (6065, 11872, 1, 8), (779268, 80, 1, 8),
+    (101, 125000, 8, 4), (125000, 101, 8, 4), (9001, 5003, 2, 8),
+    (40000, 501, 3, 4), (501, 40000, 5, 4), (70001, 120, 6, 8),
+])
+def test_wave(a, B, b, e):
+    _check(a, B, b, e)
+
+
+@pytest.mark.parametrize("e", [1, 2, 4, 8])
+def test_alignment(e):
+    for off in {e, 16 - e, 8}:
+        _check(8192 * 8 // e, 4100, 1, e, off)
+        _check(2000001 // e, 160, 1, e, off, wave=False)
+
+
+def test_under_capture():
+    x = torch.randint(0, 1 << 30, (9001 * 6001,), dtype=torch.int32,
+                      device="cuda")
+    want = x.view(9001, 6001).t().reshape(-1)
+    lm.transpose_100(x.clone(), 9001, 6001, 1)  # the first call allocates
+    gr = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(gr):
+        lm.transpose_100(x, 9001, 6001, 1)
+    gr.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(x, want)
+    gr.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(x, want.view(9001, 6001).t().reshape(-1))
+
+
+def test_concurrent_streams():
+    """Waves on several streams: every CTA's waits end whatever the others
+    hold of the GPU."""
+    streams = [torch.cuda.Stream() for _ in range(4)]
+    bufs = [torch.randint(0, 1 << 30, (8001 * 6003,), dtype=torch.int32,
+                          device="cuda") for _ in streams]
+    want = [b.view(8001, 6003).t().reshape(-1) for b in bufs]
+    torch.cuda.synchronize()
+    for s, b in zip(streams, bufs):
+        lm.transpose_100(b, 8001, 6003, 1, stream=s)
+        lm.transpose_100(b, 6003, 8001, 1, stream=s)
+        lm.transpose_100(b, 8001, 6003, 1, stream=s)
+    torch.cuda.synchronize()
+    for b, w in zip(bufs, want):
+        assert torch.equal(b, w)
+    assert lm.lib().lm_device_status(None) == 0
