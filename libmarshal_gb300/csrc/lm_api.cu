@@ -287,6 +287,10 @@ constexpr uint64_t kWalkMinBytes = 16ull << 20;
 // few steps)
 constexpr uint64_t kWaveMinBytes = 32ull << 20;
 
+// elements of one CTA's on-chip tile past which the form held in shared
+// memory is the faster one
+constexpr uint64_t kTileElems = 16 * 1024;
+
 enum class Method { Auto, BS, Pttwac, Stash, TwoPass, Cycles, Staged, Resident };
 
 TuneParams &tune_params() {
@@ -404,18 +408,24 @@ static bool do_0100(cudaStream_t s, void *buf, int e, uint64_t T, uint64_t a,
     const uint64_t sms = (uint64_t)device_info().sms;
     bool thin = m == Method::Auto && !t010 && bytes >= (1ull << 20) &&
                 ctas < sms;
-    // payloads the resident form takes (from 512 KB): the on-chip plan wins
-    // from half the SMs up (64 tiles of 64 x 4096 bytes in 2-CTA clusters:
-    // 0.0173 vs 0.0182 ms), the resident form below (one 1000 x 1000 byte
-    // tile over a 16-CTA cluster: 0.0336 vs 0.0144 ms)
-    if (m == Method::Auto && !t010 && p.feasible && bytes >= (512ull << 10) &&
-        !planner_beside_other_work() && !getenv("LM_NO_RESIDENT") &&
+    // Where the form held in shared memory can take it (about 10 us whatever
+    // the shape), the on-chip tile is the better one while a CTA has few
+    // elements to move one by one (about 5.3 us and 0.31 ns each): 41 x 1598
+    // bytes in one CTA 25.0 us, 12.2 held; 1704 x 38 half-words 24.8 and
+    // 10.4; 362 x 362 half-words in a cluster of four 18.8 and 11.9; but 66
+    // tiles of 363 x 17 doubles 8.3 and 10.4, 635 of 153 x 11 half-words 10.9
+    // and 14.4.  Clusters that leave SMs idle lose as well (15 tiles of 770 x
+    // 37 doubles 12.2 and 10.5).
+    const uint64_t elems = a * B * b * p.tiles_per_chunk / (uint64_t)p.cluster;
+    const bool held = elems > kTileElems || (p.cluster > 1 && ctas < sms);
+    if (m == Method::Auto && !t010 && p.feasible && !getenv("LM_NO_RESIDENT") &&
+        !planner_beside_other_work() && (thin || held) &&
         resident0100_applies(T, a, B, b, e)) {
       // (under stream capture the resident form does not run)
       cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
       if (cudaStreamIsCapturing(s, &cs) == cudaSuccess &&
           cs == cudaStreamCaptureStatusNone)
-        thin = ctas * 2 < sms;
+        thin = held;
     }
     if (p.feasible && !thin)
       return check_launch(launch_bs0100(s, buf, e, T, (uint32_t)a,

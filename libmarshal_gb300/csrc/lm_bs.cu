@@ -275,7 +275,9 @@ BsPlan plan_bs0100(uint64_t T, uint32_t a, uint32_t B, uint32_t b, int e,
   const uint64_t target = 40 * 1024;  // a few CTAs per SM overlap load/store
   if (tile_smem <= target) {
     uint64_t k = std::max<uint64_t>(1, target / tile_smem);
-    k = std::min<uint64_t>(k, T);
+    // few tiles spread over the SMs (143 tiles of 3 KB of bytes 16.5 us in
+    // chunks of 40 KB, 6.6 one by one)
+    k = std::min<uint64_t>(k, (T + 2 * di.sms - 1) / (2 * di.sms));
     while (k > 1 && k * tile_elems >= 0xffffffffull) k--;
     p.tiles_per_chunk = (uint32_t)k;
     p.cluster = 1;
