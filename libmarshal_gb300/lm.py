@@ -128,24 +128,56 @@ def buf_ptr(buf, elem_bytes=None):
     return buf.data_ptr(), int(elem_bytes or buf.element_size())
 
 
+_torch = None
+
+
+def _current_stream() -> int:
+    """torch's current stream of its current device.  (The raw getter: the
+    stream object that torch.cuda.current_stream() makes for it takes 3 us, as
+    long as a small conversion's launch.)"""
+    global _torch
+    if _torch is None:
+        import torch
+        _torch = torch
+    if not _torch.cuda.is_initialized():
+        return _torch.cuda.current_stream().cuda_stream
+    return _torch._C._cuda_getCurrentRawStream(_torch._C._cuda_getDevice())
+
+
 def stream_ptr(stream=None) -> int:
     if stream is None:
-        import torch
-        return torch.cuda.current_stream().cuda_stream
+        return _current_stream()
     if isinstance(stream, int):
         return stream
     return stream.cuda_stream
 
 
 class _Timer:
-    def __init__(self, timed):
-        self.v = ctypes.c_ulonglong(0) if timed else None
+    """The elapsed-time accumulator of one timed call."""
+
+    def __init__(self):
+        self.v = ctypes.c_ulonglong(0)
 
     def arg(self):
-        return ctypes.byref(self.v) if self.v is not None else None
+        return ctypes.byref(self.v)
 
     def ns(self):
-        return self.v.value if self.v is not None else None
+        return self.v.value
+
+
+class _Untimed:
+    def arg(self):
+        return None
+
+    def ns(self):
+        return None
+
+
+_UNTIMED = _Untimed()
+
+
+def _timer(timed):
+    return _Timer() if timed else _UNTIMED
 
 
 def aos_asta_bs(buf, height, width, tile_size, stream=None, elem_bytes=None):
@@ -187,7 +219,7 @@ def full_transpose(buf, M, N, variant010=0, stream=None, elem_bytes=None,
     p, e = buf_ptr(buf, elem_bytes)
     cap = buf.numel() * buf.element_size() // e if hasattr(buf, "numel") \
         else M * N
-    t = _Timer(timed)
+    t = _timer(timed)
     _check(lib().lm_full_transpose(stream_ptr(stream), p, e, M, N, cap,
                                    variant010, t.arg()), "lm_full_transpose")
     return t.ns()
@@ -196,7 +228,7 @@ def full_transpose(buf, M, N, variant010=0, stream=None, elem_bytes=None,
 def transpose(buf, A, a, B, b, R=1, stages=3, variant010=0, stream=None,
               elem_bytes=None, timed=False):
     p, e = buf_ptr(buf, elem_bytes)
-    t = _Timer(timed)
+    t = _timer(timed)
     if variant010:
         _check(lib().lm_transpose_ex(stream_ptr(stream), p, e, A, a, B, b, R,
                                      stages, variant010, t.arg()),
@@ -209,7 +241,7 @@ def transpose(buf, A, a, B, b, R=1, stages=3, variant010=0, stream=None,
 
 def transpose_010_bs(buf, A, a, B, stream=None, elem_bytes=None, timed=False):
     p, e = buf_ptr(buf, elem_bytes)
-    t = _Timer(timed)
+    t = _timer(timed)
     _check(lib().lm_transpose_010_bs(stream_ptr(stream), p, e, A, a, B,
                                      t.arg()), "lm_transpose_010_bs")
     return t.ns()
@@ -218,7 +250,7 @@ def transpose_010_bs(buf, A, a, B, stream=None, elem_bytes=None, timed=False):
 def transpose_010_pttwac(buf, A, a, B, R=1, P=1, stream=None,
                          elem_bytes=None, timed=False):
     p, e = buf_ptr(buf, elem_bytes)
-    t = _Timer(timed)
+    t = _timer(timed)
     _check(lib().lm_transpose_010_pttwac(stream_ptr(stream), p, e, A, a, B,
                                          t.arg(), R, P),
            "lm_transpose_010_pttwac")
@@ -227,7 +259,7 @@ def transpose_010_pttwac(buf, A, a, B, R=1, P=1, stream=None,
 
 def transpose_100(buf, A, B, b, stream=None, elem_bytes=None, timed=False):
     p, e = buf_ptr(buf, elem_bytes)
-    t = _Timer(timed)
+    t = _timer(timed)
     _check(lib().lm_transpose_100(stream_ptr(stream), p, e, A, B, b, t.arg()),
            "lm_transpose_100")
     return t.ns()
@@ -236,7 +268,7 @@ def transpose_100(buf, A, B, b, stream=None, elem_bytes=None, timed=False):
 def transpose_0100(buf, A, a, B, b, method=0, stream=None, elem_bytes=None,
                    timed=False):
     p, e = buf_ptr(buf, elem_bytes)
-    t = _Timer(timed)
+    t = _timer(timed)
     if method:
         _check(lib().lm_transpose_0100_method(stream_ptr(stream), p, e, A, a,
                                               B, b, method, t.arg()),
@@ -250,7 +282,7 @@ def transpose_0100(buf, A, a, B, b, method=0, stream=None, elem_bytes=None,
 def padding(buf, x_size, y_size, pad_size, stream=None, elem_bytes=None,
             timed=False):
     p, e = buf_ptr(buf, elem_bytes)
-    t = _Timer(timed)
+    t = _timer(timed)
     _check(lib().lm_padding(stream_ptr(stream), p, e, x_size, y_size, pad_size,
                             t.arg()), "lm_padding")
     return t.ns()
@@ -259,7 +291,7 @@ def padding(buf, x_size, y_size, pad_size, stream=None, elem_bytes=None,
 def unpadding(buf, x_size, y_size, pad_size, stream=None, elem_bytes=None,
               timed=False):
     p, e = buf_ptr(buf, elem_bytes)
-    t = _Timer(timed)
+    t = _timer(timed)
     _check(lib().lm_unpadding(stream_ptr(stream), p, e, x_size, y_size,
                               pad_size, t.arg()), "lm_unpadding")
     return t.ns()
