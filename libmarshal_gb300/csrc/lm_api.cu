@@ -408,16 +408,18 @@ static bool do_0100(cudaStream_t s, void *buf, int e, uint64_t T, uint64_t a,
     const uint64_t sms = (uint64_t)device_info().sms;
     bool thin = m == Method::Auto && !t010 && bytes >= (1ull << 20) &&
                 ctas < sms;
-    // Where the form held in shared memory can take it (about 10 us whatever
-    // the shape), the on-chip tile is the better one while a CTA has few
-    // elements to move one by one (about 5.3 us and 0.31 ns each): 41 x 1598
-    // bytes in one CTA 25.0 us, 12.2 held; 1704 x 38 half-words 24.8 and
-    // 10.4; 362 x 362 half-words in a cluster of four 18.8 and 11.9; but 66
-    // tiles of 363 x 17 doubles 8.3 and 10.4, 635 of 153 x 11 half-words 10.9
-    // and 14.4.  Clusters that leave SMs idle lose as well (15 tiles of 770 x
-    // 37 doubles 12.2 and 10.5).
+    // Where the form held in shared memory can take it (about 10 us and 0.25
+    // us per MB whatever the shape), the on-chip tile is the better one while
+    // a CTA has few elements to move one by one (about 5.3 us and 0.31 ns
+    // each): 41 x 1598 bytes in one CTA 25.0 us, 12.2 held; 1704 x 38
+    // half-words 24.8 and 10.4; 362 x 362 half-words in a cluster of four
+    // 18.8 and 11.9; but 66 tiles of 363 x 17 doubles 8.3 and 10.4, 100 of
+    // 129 x 129 12.2 and 13.9, 635 of 153 x 11 half-words 10.9 and 14.4.
+    // Clusters that leave SMs idle lose as well (15 tiles of 770 x 37 doubles
+    // 12.2 and 10.5).
     const uint64_t elems = a * B * b * p.tiles_per_chunk / (uint64_t)p.cluster;
-    const bool held = elems > kTileElems || (p.cluster > 1 && ctas < sms);
+    const bool held = elems > kTileElems + bytes / 1250 ||
+                      (p.cluster > 1 && ctas < sms);
     if (m == Method::Auto && !t010 && p.feasible && !getenv("LM_NO_RESIDENT") &&
         !planner_beside_other_work() && (thin || held) &&
         resident0100_applies(T, a, B, b, e)) {

@@ -1416,7 +1416,7 @@ __device__ void gather_store(const BJob &j, uint32_t q, const unsigned char *buf
 // 16384 x 16384 the other way: 0.126 vs 0.121 ms).
 // RAG: with the code of ragged blocks and of rows staged as one range (in a
 // kernel of its own: it takes 128 registers).
-template <int MB, int RAG>
+template <int MB, int RAG, int ES>
 __global__ void __launch_bounds__(kStageThreads, MB) k_batch_gather(BatchArgs g) {
   extern __shared__ __align__(128) unsigned char smem[];
   __shared__ __align__(8) uint64_t bar[2];
@@ -1499,11 +1499,15 @@ __global__ void __launch_bounds__(kStageThreads, MB) k_batch_gather(BatchArgs g)
       pending &= ~(1u << st);
       const BJob &j = s_jobs[st];
       const unsigned char *buf = smem + (size_t)st * g.stage_bytes;
-      switch (j.e) {
-        case 1: gather_store<1, kStageThreads, RAG>(j, cq, buf, rowoff[st]); break;
-        case 2: gather_store<2, kStageThreads, RAG>(j, cq, buf, rowoff[st]); break;
-        case 4: gather_store<4, kStageThreads, RAG>(j, cq, buf, rowoff[st]); break;
-        default: gather_store<8, kStageThreads, RAG>(j, cq, buf, rowoff[st]); break;
+      if constexpr (ES != 0) {
+        gather_store<ES, kStageThreads, RAG>(j, cq, buf, rowoff[st]);
+      } else {
+        switch (j.e) {
+          case 1: gather_store<1, kStageThreads, RAG>(j, cq, buf, rowoff[st]); break;
+          case 2: gather_store<2, kStageThreads, RAG>(j, cq, buf, rowoff[st]); break;
+          case 4: gather_store<4, kStageThreads, RAG>(j, cq, buf, rowoff[st]); break;
+          default: gather_store<8, kStageThreads, RAG>(j, cq, buf, rowoff[st]); break;
+        }
       }
     } else {
       s_dead = 1;
@@ -2409,7 +2413,7 @@ static bool launch_staged(cudaStream_t s, const BJob *d_jobs,
                           uint32_t *counter, size_t smem, bool copyback) {
   if (nitems == 0) return false;
   const DeviceInfo &di = device_info();
-  auto kern = copyback ? k_batch_copyback : k_batch_gather<3, 0>;
+  auto kern = copyback ? k_batch_copyback : k_batch_gather<3, 0, 0>;
   // the gather keeps two stages of `smem` bytes
   const size_t dyn = copyback ? 0 : 2 * smem;
   static LaunchCache copy_cache;
@@ -2474,17 +2478,22 @@ cudaError_t launch_staged0100(cudaStream_t s, void *buf, int e, uint64_t T,
   size_t stage = 0;
   if (!staged_job(g.single, jb, nz, &nblk, &stage)) return cudaErrorInvalidValue;
   g.single.scratch = reinterpret_cast<char *>(scratch);
-  const bool rag = g.single.ragged || g.single.contig, two = e == 2;
-  auto gather = rag   ? e <= 2 ? k_batch_gather<2, 1> : k_batch_gather<3, 2>
-                : two ? k_batch_gather<2, 0>
-                      : k_batch_gather<3, 0>;
+  // a kernel per element width: without the other widths' stores the
+  // registers of three CTAs per SM hold all of one width's
+  using Kern = void (*)(BatchArgs);
+  static const Kern kerns[2][4] = {
+      {k_batch_gather<3, 0, 1>, k_batch_gather<3, 0, 2>, k_batch_gather<3, 0, 4>,
+       k_batch_gather<3, 0, 8>},
+      {k_batch_gather<2, 1, 1>, k_batch_gather<2, 1, 2>, k_batch_gather<3, 2, 4>,
+       k_batch_gather<3, 2, 8>}};
+  static LaunchCache caches[2][4];
+  const int r = g.single.ragged || g.single.contig ? 1 : 0;
+  const int w = e == 1 ? 0 : e == 2 ? 1 : e == 4 ? 2 : 3;
+  const Kern gather = kerns[r][w];
   const size_t dyn = 2 * stage;
   cudaError_t err = cudaSuccess;
-  static LaunchCache rag_cache[2], two_cache;
-  const int occ = prepare_launch(
-      (const void *)gather,
-      rag ? rag_cache[e <= 2] : two ? two_cache : g_gather3_cache, dyn, kStageThreads,
-      &err);
+  const int occ = prepare_launch((const void *)gather, caches[r][w], dyn,
+                                 kStageThreads, &err);
   if (err != cudaSuccess) return err;
   const DeviceInfo &di = device_info();
   const uint32_t grid = (uint32_t)std::min<uint64_t>(
@@ -2561,7 +2570,7 @@ __device__ __forceinline__ uint32_t wave_split(const WaveArgs &g, uint32_t at,
               g.div_len);
 }
 
-template <int MB, int RAG>
+template <int MB, int RAG, int E>
 __global__ void __launch_bounds__(kStageThreads, MB) k_wave(WaveArgs g) {
   extern __shared__ __align__(128) unsigned char smem[];
   __shared__ __align__(8) uint64_t bar[2];
@@ -2675,19 +2684,7 @@ __global__ void __launch_bounds__(kStageThreads, MB) k_wave(WaveArgs g) {
       } else if (part == 0) {
         continue;
       }
-      switch (s_job.e) {
-        case 1:
-          gather_store_at<1, kStageThreads, RAG>(s_job, p, out, b, rowoff[st]);
-          break;
-        case 2:
-          gather_store_at<2, kStageThreads, RAG>(s_job, p, out, b, rowoff[st]);
-          break;
-        case 4:
-          gather_store_at<4, kStageThreads, RAG>(s_job, p, out, b, rowoff[st]);
-          break;
-        default:
-          gather_store_at<8, kStageThreads, RAG>(s_job, p, out, b, rowoff[st]);
-      }
+      gather_store_at<E, kStageThreads, RAG>(s_job, p, out, b, rowoff[st]);
     }
     __syncthreads();  // stage st and slot st are free
     if (!more) return;
@@ -2862,11 +2859,16 @@ cudaError_t launch_wave0100(cudaStream_t s, void *buf, int e, uint64_t a,
   };
   if (!g.backward && (err = copy()) != cudaSuccess) return err;
   {
-    auto kern = !rag ? k_wave<3, 0> : e <= 2 ? k_wave<2, 1> : k_wave<3, 2>;
-    static LaunchCache cache[3];
+    using Kern = void (*)(WaveArgs);
+    static const Kern kerns[2][4] = {
+        {k_wave<3, 0, 1>, k_wave<3, 0, 2>, k_wave<3, 0, 4>, k_wave<3, 0, 8>},
+        {k_wave<2, 1, 1>, k_wave<2, 1, 2>, k_wave<3, 2, 4>, k_wave<3, 2, 8>}};
+    static LaunchCache caches[2][4];
+    const int w = e == 1 ? 0 : e == 2 ? 1 : e == 4 ? 2 : 3;
+    const Kern kern = kerns[rag ? 1 : 0][w];
     const size_t dyn = 2 * (size_t)g.stage_bytes;
-    const int occ = prepare_launch((const void *)kern, cache[!rag ? 0 : e <= 2 ? 1 : 2], dyn,
-                                   kStageThreads, &err);
+    const int occ = prepare_launch((const void *)kern, caches[rag ? 1 : 0][w],
+                                   dyn, kStageThreads, &err);
     if (err != cudaSuccess) return err;
     const uint32_t grid = (uint32_t)std::min<uint64_t>(
         (uint64_t)di.sms * std::max(occ, 1), g.nblk);
@@ -3109,7 +3111,9 @@ struct ResArgs {
   uint64_t timeout_ns;
 };
 
+template <int E>
 __global__ void __launch_bounds__(kResThreads, 1) k_resident(ResArgs g) {
+  constexpr int RAG = E <= 2 ? 1 : 2;
   extern __shared__ __align__(128) unsigned char smem[];
   __shared__ __align__(8) uint64_t bar;
   __shared__ __align__(16) BJob s_job;
@@ -3134,7 +3138,7 @@ __global__ void __launch_bounds__(kResThreads, 1) k_resident(ResArgs g) {
 #pragma unroll
   for (uint32_t k = 0; k < kResMaxBlocks; ++k)
     if (k < nmine) {
-      rc[k] = gather_row_plan<kResThreads, 3>(s_job, blockIdx.x + k * gridDim.x,
+      rc[k] = gather_row_plan<kResThreads, RAG>(s_job, blockIdx.x + k * gridDim.x,
                               rowoff + k * s_job.tab);
       bytes += rc[k].bytes;
     }
@@ -3175,12 +3179,7 @@ __global__ void __launch_bounds__(kResThreads, 1) k_resident(ResArgs g) {
       const uint32_t q = blockIdx.x + k * gridDim.x;
       const unsigned char *buf = smem + (size_t)k * g.stage_bytes;
       const uint32_t *ro = rowoff + k * s_job.tab;
-      switch (s_job.e) {
-        case 1: gather_store<1, kResThreads, 3>(s_job, q, buf, ro); break;
-        case 2: gather_store<2, kResThreads, 3>(s_job, q, buf, ro); break;
-        case 4: gather_store<4, kResThreads, 3>(s_job, q, buf, ro); break;
-        default: gather_store<8, kResThreads, 3>(s_job, q, buf, ro); break;
-      }
+      gather_store<E, kResThreads, RAG>(s_job, q, buf, ro);
     }
     return;
   }
@@ -3316,6 +3315,10 @@ bool plan_resident_cached(ResArgs &g, uint32_t *grid, size_t *dyn, void *buf,
   return c.ok;
 }
 
+const void *const kResidentKernels[4] = {
+    (const void *)k_resident<1>, (const void *)k_resident<2>,
+    (const void *)k_resident<4>, (const void *)k_resident<8>};
+
 // The device's ResDevice, set up on first use (nullptr on failure).
 ResDevice *res_device() {
   const DeviceInfo &di = device_info();
@@ -3323,16 +3326,19 @@ ResDevice *res_device() {
   std::lock_guard<std::mutex> lock(g_res_mu);
   ResDevice *d = g_res_dev[di.device];
   if (d) return d;
-  cudaFuncAttributes fa{};
-  if (cudaFuncGetAttributes(&fa, k_resident) != cudaSuccess) return nullptr;
-  const size_t max_dyn =
-      (size_t)di.max_smem_optin > fa.sharedSizeBytes
-          ? ((size_t)di.max_smem_optin - fa.sharedSizeBytes) / 128 * 128
-          : 0;
-  if (cudaFuncSetAttribute(k_resident,
-                           cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           (int)max_dyn) != cudaSuccess)
-    return nullptr;
+  size_t max_dyn = (size_t)di.max_smem_optin;
+  for (const void *k : kResidentKernels) {
+    cudaFuncAttributes fa{};
+    if (cudaFuncGetAttributes(&fa, k) != cudaSuccess) return nullptr;
+    max_dyn = std::min(max_dyn, (size_t)di.max_smem_optin > fa.sharedSizeBytes
+                                    ? ((size_t)di.max_smem_optin -
+                                       fa.sharedSizeBytes) / 128 * 128
+                                    : 0);
+  }
+  for (const void *k : kResidentKernels)
+    if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)max_dyn) != cudaSuccess)
+      return nullptr;
   d = new ResDevice;
   d->max_dyn = max_dyn;
   g_res_dev[di.device] = d;
@@ -3379,8 +3385,9 @@ cudaError_t launch_resident0100(cudaStream_t s, void *buf, int e, uint64_t T,
   }
   void *args[] = {&g};
   ProfScope ps(s, "resident");
-  err = cudaLaunchCooperativeKernel((const void *)k_resident, dim3(grid),
-                                    dim3(kResThreads), args, dyn, s);
+  err = cudaLaunchCooperativeKernel(
+      kResidentKernels[e == 1 ? 0 : e == 2 ? 1 : e == 4 ? 2 : 3], dim3(grid),
+      dim3(kResThreads), args, dyn, s);
   if (err != cudaSuccess) {
     // no CTA arrives: the slot keeps the count it had
     std::lock_guard<std::mutex> lock(g_res_mu);
