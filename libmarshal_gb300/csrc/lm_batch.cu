@@ -1417,19 +1417,20 @@ __device__ void gather_store(const BJob &j, uint32_t q, const unsigned char *buf
 // RAG: with the code of ragged blocks and of rows staged as one range (in a
 // kernel of its own: it takes 128 registers).
 template <int MB, int RAG, int ES>
-__global__ void __launch_bounds__(kStageThreads, MB) k_batch_gather(BatchArgs g) {
+__global__ void __launch_bounds__(kStageThreads, MB) k_batch_gather(const __grid_constant__ BatchArgs g) {
   extern __shared__ __align__(128) unsigned char smem[];
   __shared__ __align__(8) uint64_t bar[2];
   __shared__ __align__(16) uint32_t rowoff[2][RAG & 1 ? kRowTable : kStageMaxS];
   __shared__ uint32_t s_job[2], s_q[2], s_valid[2];
   __shared__ int s_dead;
-  __shared__ __align__(16) BJob s_jobs[2];  // job of the block in each stage
+  // (ES: one job, read from the parameters; else the job of the block in each
+  // stage)
+  __shared__ __align__(16) BJob s_jobs[ES ? 1 : 2];
   const uint32_t warp = threadIdx.x >> 5;
-  const BJob *jobs = g.items ? g.jobs : &g.single;
   uint32_t c_job = 0, c_q = 0, c_end = 0;  // thread 0's cursor
   bool c_first = true;
   auto fetch = [&](int slot) {
-    if (!g.items) {
+    if (ES) {
       c_q = c_first ? blockIdx.x : c_q + gridDim.x;
       c_first = false;
       s_valid[slot] = c_q < g.nitems;
@@ -1463,8 +1464,9 @@ __global__ void __launch_bounds__(kStageThreads, MB) k_batch_gather(BatchArgs g)
   if (!s_valid[0]) return;
   uint32_t cq = s_q[0];
   {
-    if (warp == 0) copy_job(&s_jobs[0], &jobs[s_job[0]]);
-    const RowCopy rc = gather_row_plan<kStageThreads, RAG>(jobs[s_job[0]], cq, rowoff[0]);
+    if (!ES && warp == 0) copy_job(&s_jobs[0], &g.jobs[s_job[0]]);
+    const RowCopy rc = gather_row_plan<kStageThreads, RAG>(
+        ES ? g.single : g.jobs[s_job[0]], cq, rowoff[0]);
     gather_arrive(&bar[0], rc.bytes);
     __syncthreads();  // every warp's expected bytes before any copy
     gather_row_issue(rc, smem, &bar[0]);
@@ -1479,8 +1481,9 @@ __global__ void __launch_bounds__(kStageThreads, MB) k_batch_gather(BatchArgs g)
     const bool more = s_valid[nx] != 0 && !s_dead;
     const uint32_t nj = s_job[nx], nq = s_q[nx];
     if (more) {
-      if (warp == 0) copy_job(&s_jobs[nx], &jobs[nj]);
-      const RowCopy rc = gather_row_plan<kStageThreads, RAG>(jobs[nj], nq, rowoff[nx]);
+      if (!ES && warp == 0) copy_job(&s_jobs[nx], &g.jobs[nj]);
+      const RowCopy rc = gather_row_plan<kStageThreads, RAG>(
+          ES ? g.single : g.jobs[nj], nq, rowoff[nx]);
       gather_arrive(&bar[nx], rc.bytes);
       __syncthreads();  // every warp's expected bytes before any copy
       gather_row_issue(rc, smem + (size_t)nx * g.stage_bytes, &bar[nx]);
@@ -1497,7 +1500,7 @@ __global__ void __launch_bounds__(kStageThreads, MB) k_batch_gather(BatchArgs g)
     if (landed) {
       parity ^= 1u << st;
       pending &= ~(1u << st);
-      const BJob &j = s_jobs[st];
+      const BJob &j = ES ? g.single : s_jobs[ES ? 0 : st];
       const unsigned char *buf = smem + (size_t)st * g.stage_bytes;
       if constexpr (ES != 0) {
         gather_store<ES, kStageThreads, RAG>(j, cq, buf, rowoff[st]);
@@ -2480,7 +2483,7 @@ cudaError_t launch_staged0100(cudaStream_t s, void *buf, int e, uint64_t T,
   g.single.scratch = reinterpret_cast<char *>(scratch);
   // a kernel per element width: without the other widths' stores the
   // registers of three CTAs per SM hold all of one width's
-  using Kern = void (*)(BatchArgs);
+  using Kern = void (*)(const BatchArgs);
   static const Kern kerns[2][4] = {
       {k_batch_gather<3, 0, 1>, k_batch_gather<3, 0, 2>, k_batch_gather<3, 0, 4>,
        k_batch_gather<3, 0, 8>},
@@ -2571,11 +2574,10 @@ __device__ __forceinline__ uint32_t wave_split(const WaveArgs &g, uint32_t at,
 }
 
 template <int MB, int RAG, int E>
-__global__ void __launch_bounds__(kStageThreads, MB) k_wave(WaveArgs g) {
+__global__ void __launch_bounds__(kStageThreads, MB) k_wave(const __grid_constant__ WaveArgs g) {
   extern __shared__ __align__(128) unsigned char smem[];
   __shared__ __align__(8) uint64_t bar[2];
   __shared__ __align__(16) uint32_t rowoff[2][RAG & 1 ? kRowTable : kStageMaxS];
-  __shared__ __align__(16) BJob s_job;
   __shared__ uint32_t s_n[2], s_split[2];
   __shared__ int s_dead;
   const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -2608,7 +2610,7 @@ __global__ void __launch_bounds__(kStageThreads, MB) k_wave(WaveArgs g) {
     uint32_t s;
     const uint32_t q = block_of(s_n[slot], &s);
     const RowCopy rc = gather_row_plan<kStageThreads, RAG>(
-        s_job, q, rowoff[slot], g.backward ? 0 : s_split[slot]);
+        g.job, q, rowoff[slot], g.backward ? 0 : s_split[slot]);
     gather_arrive(&bar[slot], rc.bytes);
     __syncthreads();  // every warp's expected bytes before any copy
     gather_row_issue(rc, smem + (size_t)slot * g.stage_bytes, &bar[slot]);
@@ -2621,7 +2623,6 @@ __global__ void __launch_bounds__(kStageThreads, MB) k_wave(WaveArgs g) {
     claimed = atomicAdd(g.ticket, 1u);
     fetch(0);
   }
-  if (warp == 0) copy_job(&s_job, &g.job);
   __syncthreads();
   if (s_n[0] >= g.nblk) return;
   issue(0);
@@ -2663,28 +2664,28 @@ __global__ void __launch_bounds__(kStageThreads, MB) k_wave(WaveArgs g) {
     // thread's stores of the last block)
     if (threadIdx.x == 0) red_relaxed_gpu(done + fdiv(s, g.div_group), 1u);
     const unsigned char *buf = smem + (size_t)st * g.stage_bytes;
-    const GBlock k = gather_decode<RAG>(s_job, q);
+    const GBlock k = gather_decode<RAG>(g.job, q);
     const uint32_t split = s_split[st];
     for (int part = 0; part < 2; ++part) {
       // backward: output rows below the split to scratch, the others in place
       GBlock p = k;
       const unsigned char *b = buf;
-      char *out = s_job.base;
+      char *out = g.job.base;
       if (g.backward) {
         const uint32_t cut = split > k.j0 ? min(split - k.j0, k.sj) : 0u;
         if (part == 0) {
           p.sj = cut;
-          out = s_job.scratch;
+          out = g.job.scratch;
         } else {
           p.j0 += cut;
           p.sj -= cut;
-          b += cut * s_job.b * s_job.e;
+          b += cut * g.job.b * g.job.e;
         }
         if (p.sj == 0) continue;
       } else if (part == 0) {
         continue;
       }
-      gather_store_at<E, kStageThreads, RAG>(s_job, p, out, b, rowoff[st]);
+      gather_store_at<E, kStageThreads, RAG>(g.job, p, out, b, rowoff[st]);
     }
     __syncthreads();  // stage st and slot st are free
     if (!more) return;
@@ -2859,7 +2860,7 @@ cudaError_t launch_wave0100(cudaStream_t s, void *buf, int e, uint64_t a,
   };
   if (!g.backward && (err = copy()) != cudaSuccess) return err;
   {
-    using Kern = void (*)(WaveArgs);
+    using Kern = void (*)(const WaveArgs);
     static const Kern kerns[2][4] = {
         {k_wave<3, 0, 1>, k_wave<3, 0, 2>, k_wave<3, 0, 4>, k_wave<3, 0, 8>},
         {k_wave<2, 1, 1>, k_wave<2, 1, 2>, k_wave<3, 2, 4>, k_wave<3, 2, 8>}};
@@ -2917,11 +2918,10 @@ __device__ __forceinline__ void square_pair(const SqArgs &g, uint32_t x,
   q[1] = t * g.job.nIJ + J * g.nb + I;
 }
 
-__global__ void __launch_bounds__(kStageThreads, 3) k_square(SqArgs g) {
+__global__ void __launch_bounds__(kStageThreads, 3) k_square(const __grid_constant__ SqArgs g) {
   extern __shared__ __align__(128) unsigned char smem[];
   __shared__ __align__(8) uint64_t bar[2];
   __shared__ __align__(16) uint32_t rowoff[2][2][kSquareMaxS];
-  __shared__ __align__(16) BJob s_job;
   __shared__ int s_dead;
   const uint32_t warp = threadIdx.x >> 5;
   if (threadIdx.x == 0) {
@@ -2930,7 +2930,6 @@ __global__ void __launch_bounds__(kStageThreads, 3) k_square(SqArgs g) {
     fence_mbar_init();
     s_dead = 0;
   }
-  if (warp == 0) copy_job(&s_job, &g.job);
   __syncthreads();
   // the copies of pair x into stage st
   auto issue = [&](uint32_t x, uint32_t st) {
@@ -2938,10 +2937,10 @@ __global__ void __launch_bounds__(kStageThreads, 3) k_square(SqArgs g) {
     square_pair(g, x, q);
     unsigned char *buf = smem + st * 2 * (size_t)g.stage_bytes;
     const RowCopy a =
-        gather_row_plan<kStageThreads, 0>(s_job, q[0], rowoff[st][0]);
+        gather_row_plan<kStageThreads, 0>(g.job, q[0], rowoff[st][0]);
     RowCopy b{0, 0, 0};
     if (q[1] != q[0])
-      b = gather_row_plan<kStageThreads, 0>(s_job, q[1], rowoff[st][1]);
+      b = gather_row_plan<kStageThreads, 0>(g.job, q[1], rowoff[st][1]);
     gather_arrive(&bar[st], a.bytes + b.bytes);
     __syncthreads();  // every warp's expected bytes before any copy
     gather_row_issue(a, buf, &bar[st]);
@@ -2969,11 +2968,11 @@ __global__ void __launch_bounds__(kStageThreads, 3) k_square(SqArgs g) {
     for (uint32_t h = 0; h < (q[0] == q[1] ? 1u : 2u); ++h) {
       const unsigned char *b = buf + h * g.stage_bytes;
       const uint32_t *ro = rowoff[st][h];
-      switch (s_job.e) {
-        case 1: gather_store<1, kStageThreads, 0>(s_job, q[h], b, ro); break;
-        case 2: gather_store<2, kStageThreads, 0>(s_job, q[h], b, ro); break;
-        case 4: gather_store<4, kStageThreads, 0>(s_job, q[h], b, ro); break;
-        default: gather_store<8, kStageThreads, 0>(s_job, q[h], b, ro);
+      switch (g.job.e) {
+        case 1: gather_store<1, kStageThreads, 0>(g.job, q[h], b, ro); break;
+        case 2: gather_store<2, kStageThreads, 0>(g.job, q[h], b, ro); break;
+        case 4: gather_store<4, kStageThreads, 0>(g.job, q[h], b, ro); break;
+        default: gather_store<8, kStageThreads, 0>(g.job, q[h], b, ro);
       }
     }
     __syncthreads();  // stage st is free
@@ -3008,12 +3007,16 @@ static bool plan_square(SqArgs &g, void *buf, uint64_t T, uint64_t a,
   nz.T = T;
   nz.a = nz.B = a;
   nz.b = b;
-  // blocks of 16 to 32 KB with rows of 128 bytes and more (16384^2 half-words
-  // 209 us with 128 rows, 267 with 64; 8192^2 floats 98 with 64, 215 with
-  // 32; 8192^2 doubles 202 with 64, 240 with 32), of even size, and smaller
-  // where they are fewer than SMs (333^2 floats 10.6 us with 64 rows, 10.0
-  // with 32)
-  uint64_t S = unit <= 2 ? 128 : unit <= 8 ? 64 : 32;
+  // blocks of 16 to 32 KB with rows of 128 bytes and more: 16384^2 half-words
+  // 209 us with 128 rows, 267 with 64; 8192^2 floats 99 with 64, 215 with 32,
+  // and from about 256 MB 80 are better (two CTAs per SM: 16384^2 floats 373
+  // and 362); doubles in whole vectors 48 (5000^2 82 us with 64, 71 with 48),
+  // else 64 (8191^2 185 and 202).  Of even size, and smaller where they are
+  // fewer than SMs (333^2 floats 10.6 us with 64 rows, 10.0 with 32)
+  uint64_t S = 32;
+  if (unit <= 2) S = 128;
+  else if (unit <= 4) S = T * a * a * unit >= (256ull << 20) ? 80 : 64;
+  else if (unit <= 8) S = (a * unit) % 16 || ((uintptr_t)buf & 15) ? 64 : 48;
   auto pairs = [&](uint64_t s) {
     const uint64_t n = (a + s - 1) / s;
     return T * (n * (n + 1) / 2);
@@ -3112,11 +3115,10 @@ struct ResArgs {
 };
 
 template <int E>
-__global__ void __launch_bounds__(kResThreads, 1) k_resident(ResArgs g) {
+__global__ void __launch_bounds__(kResThreads, 1) k_resident(const __grid_constant__ ResArgs g) {
   constexpr int RAG = E <= 2 ? 1 : 2;
   extern __shared__ __align__(128) unsigned char smem[];
   __shared__ __align__(8) uint64_t bar;
-  __shared__ __align__(16) BJob s_job;
   __shared__ int s_ok;
   const uint32_t warp = threadIdx.x >> 5, nw = kResThreads / 32;
   const uint32_t nmine =
@@ -3129,7 +3131,6 @@ __global__ void __launch_bounds__(kResThreads, 1) k_resident(ResArgs g) {
     fence_mbar_init();
     s_ok = 1;
   }
-  if (warp == 0) copy_job(&s_job, &g.job);
   __syncthreads();
   // every row of every block by its own bulk copy, spread over all warps;
   // one barrier for all of them
@@ -3138,8 +3139,8 @@ __global__ void __launch_bounds__(kResThreads, 1) k_resident(ResArgs g) {
 #pragma unroll
   for (uint32_t k = 0; k < kResMaxBlocks; ++k)
     if (k < nmine) {
-      rc[k] = gather_row_plan<kResThreads, RAG>(s_job, blockIdx.x + k * gridDim.x,
-                              rowoff + k * s_job.tab);
+      rc[k] = gather_row_plan<kResThreads, RAG>(g.job, blockIdx.x + k * gridDim.x,
+                              rowoff + k * g.job.tab);
       bytes += rc[k].bytes;
     }
   gather_arrive(&bar, bytes);
@@ -3178,8 +3179,8 @@ __global__ void __launch_bounds__(kResThreads, 1) k_resident(ResArgs g) {
     for (uint32_t k = 0; k < nmine; ++k) {
       const uint32_t q = blockIdx.x + k * gridDim.x;
       const unsigned char *buf = smem + (size_t)k * g.stage_bytes;
-      const uint32_t *ro = rowoff + k * s_job.tab;
-      gather_store<E, kResThreads, RAG>(s_job, q, buf, ro);
+      const uint32_t *ro = rowoff + k * g.job.tab;
+      gather_store<E, kResThreads, RAG>(g.job, q, buf, ro);
     }
     return;
   }
