@@ -220,6 +220,70 @@ struct HostWord {
   }
 };
 
+// The task flags of one padding call.  Blocks of kWords words are kept per
+// device (kKept at most, until lm_marshal_finalize) and never cleared: a call
+// hands its kernel an epoch that no word holds yet and the ticket word's
+// value.  A block is given back when the call has waited for its kernel; one
+// whose kernel failed is not.  Larger calls allocate theirs.
+struct PadBlock {
+  static constexpr uint64_t kWords = 16 * 1024;
+  static constexpr size_t kKept = 16;
+  struct Kept {
+    uint32_t *p;
+    uint32_t ticket, epoch;
+  };
+  static std::mutex &mu() {
+    static std::mutex m;
+    return m;
+  }
+  static std::vector<Kept> &pool(int dev) {
+    static std::vector<Kept> v[64];
+    return v[dev & 63];
+  }
+  PadFlags f;
+  Scratch own;        // not from the pool
+  int dev = 0;
+  bool kept = false;  // from the pool
+  bool done = false;  // the kernel has finished without a failure
+  uint64_t tasks = 0;
+  // false: no memory
+  bool take(uint64_t n, cudaStream_t s) {
+    tasks = n;
+    cudaGetDevice(&dev);
+    kept = n + 2 <= kWords;
+    if (kept) {
+      std::lock_guard<std::mutex> lock(mu());
+      if (!pool(dev).empty()) {
+        const Kept k = pool(dev).back();
+        pool(dev).pop_back();
+        f.p = k.p;
+        f.words = kWords;
+        f.ticket = k.ticket;
+        f.epoch = k.epoch + 1;
+        return true;
+      }
+    }
+    f.words = kept ? kWords : n + 2;
+    if (get_zeroed(own, f.words * 4, s)) return false;
+    f.p = (uint32_t *)own.p;
+    if (kept) own.p = nullptr;
+    return true;
+  }
+  ~PadBlock() {
+    if (!kept || !f.p) return;
+    std::lock_guard<std::mutex> lock(mu());
+    if (done && pool(dev).size() < kKept && f.epoch != 0xffffffffu)
+      pool(dev).push_back({f.p, f.ticket + (uint32_t)tasks, f.epoch});
+    else
+      cudaFreeAsync(f.p, own.s);  // (the call has waited for its stream)
+  }
+  static void clear(int dev) {
+    std::lock_guard<std::mutex> lock(mu());
+    for (const Kept &k : pool(dev)) cudaFree(k.p);
+    pool(dev).clear();
+  }
+};
+
 // Reads and clears the status word after the stream's work has finished.
 static bool check_status(cudaStream_t s, const char *what) {
   uint32_t *w = device_status_word();
@@ -746,18 +810,16 @@ static bool do_pad(cudaStream_t s, void *buf, int e, int64_t x, int64_t y,
   if ((y == 0 || pad == x) && stall_block < 0) return false;
   if (buf == nullptr) return fail("null buffer");
   if (misaligned(buf, e)) return fail("buffer must be aligned to the element size");
-  Scratch sc;
-  const size_t flags = stall_block >= 0
-                           ? std::max<size_t>(pad_scratch_bytes(buf, e, y, pad), 16)
-                           : pad_scratch_bytes(buf, e, y, pad);
-  if (flags && get_zeroed(sc, flags, s)) return true;
+  PadBlock block;
+  const uint64_t tasks = pad_tasks(buf, e, y, pad);
+  if ((tasks > 1 || stall_block >= 0) && !block.take(tasks, s)) return true;
   // (a word of host memory, so that no copy follows the kernel)
   HostWord st;
   if (!st.p) return fail("padding: no status word");
   cudaError_t err =
-      padding ? launch_padding(s, buf, e, x, y, pad, (uint32_t *)sc.p, st.p,
+      padding ? launch_padding(s, buf, e, x, y, pad, block.f, st.p,
                                timeout_ns, stall_block)
-              : launch_unpadding(s, buf, e, x, y, pad, (uint32_t *)sc.p, st.p,
+              : launch_unpadding(s, buf, e, x, y, pad, block.f, st.p,
                                  timeout_ns, stall_block);
   if (err != cudaSuccess) return cuda_fail(err, padding ? "padding" : "unpadding");
   err = cudaStreamSynchronize(s);
@@ -769,6 +831,7 @@ static bool do_pad(cudaStream_t s, void *buf, int e, int64_t x, int64_t y,
   if (status != kStatusOk)
     return fail("%s: an inter-CTA wait timed out (status %u)",
                 padding ? "padding" : "unpadding", status);
+  block.done = true;
   return false;
 }
 
@@ -883,6 +946,7 @@ void lm_marshal_finalize(void) {
   if (cudaGetDevice(&dev) != cudaSuccess) return;
   cycle_cache_clear();
   stash_cache_clear();
+  PadBlock::clear(dev);
   cudaMemPool_t pool;
   if (cudaDeviceGetDefaultMemPool(&pool, dev) == cudaSuccess)
     cudaMemPoolTrimTo(pool, 0);

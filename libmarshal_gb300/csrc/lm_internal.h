@@ -281,18 +281,24 @@ uint32_t *device_status_word();
 // ---- row padding / unpadding with bounded inter-CTA waits ----------------
 // padding:   [y][x] -> [y][pad] (new columns zero)
 // unpadding: [y][pad] -> [y][x], tail y*x..y*pad-1 zero.
-// `scratch` must hold pad_scratch_bytes(...) zeroed bytes (0 and nullptr: one
-// task, which waits for nothing); `status` one zeroed word of pinned host
-// memory that the kernel sets to kStatusWaitTimeout when a wait runs out.
-// stall_block >= 0 makes that task wait on a flag nothing sets
-// (failure-detection test hook; it needs the scratch of two tasks).
-size_t pad_scratch_bytes(const void *buf, int e, uint64_t y, uint64_t pad);
+// `flags`: a ticket word, a word per task (pad_tasks) that none of which
+// equals `epoch`, and a last one that never does; p == nullptr: one task,
+// which waits for nothing.  `status`: one zeroed word of pinned host memory
+// that the kernel sets to kStatusWaitTimeout when a wait runs out.
+// stall_block >= 0 makes that task wait on the last word (failure-detection
+// test hook; it needs flags).
+struct PadFlags {
+  uint32_t *p = nullptr;
+  uint64_t words = 0;
+  uint32_t ticket = 0, epoch = 1;  // the ticket word's value before the launch
+};
+uint64_t pad_tasks(const void *buf, int e, uint64_t y, uint64_t pad);
 cudaError_t launch_padding(cudaStream_t s, void *buf, int e, uint64_t x,
-                           uint64_t y, uint64_t pad, uint32_t *scratch,
+                           uint64_t y, uint64_t pad, const PadFlags &flags,
                            uint32_t *status, uint64_t timeout_ns,
                            int64_t stall_block);
 cudaError_t launch_unpadding(cudaStream_t s, void *buf, int e, uint64_t x,
-                             uint64_t y, uint64_t pad, uint32_t *scratch,
+                             uint64_t y, uint64_t pad, const PadFlags &flags,
                              uint32_t *status, uint64_t timeout_ns,
                              int64_t stall_block);
 

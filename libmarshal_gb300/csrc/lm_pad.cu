@@ -45,19 +45,20 @@ struct PadArgs {
   uint32_t P;        // buf modulo 16; task k: padded bytes k*task - P and on
   uint32_t task;     // bytes of a task, a multiple of 16
   uint32_t rows;     // unpadding: 1 = copy the rows of a task one by one
-  uint32_t *ticket;  // scratch[0]
-  uint32_t *loaded;  // scratch[1 .. ntasks]
-  uint32_t *never;   // scratch[ntasks + 1], never set
+  uint32_t *ticket;  // scratch[0]; counts up from ticket0
+  uint32_t *loaded;  // scratch[1 .. ntasks]: `epoch` once loaded
+  uint32_t *never;   // the last word, never set
+  uint32_t ticket0, epoch;
   uint32_t *status;  // host memory, read when the stream has finished
   uint64_t timeout_ns;
   int64_t stall_block;
   FastDiv div_x, div_pad;  // where rows are no longer than a task
 };
 
-__device__ __forceinline__ bool wait_flag(const uint32_t *f, uint64_t t0,
-                                          uint64_t timeout_ns) {
+__device__ __forceinline__ bool wait_flag(const uint32_t *f, uint32_t epoch,
+                                          uint64_t t0, uint64_t timeout_ns) {
   unsigned ns = 32;
-  while (ld_acquire_gpu(f) == 0) {
+  while (ld_acquire_gpu(f) != epoch) {
     if (global_timer_ns() - t0 > timeout_ns) return false;
     __nanosleep(ns);
     if (ns < 4096) ns <<= 1;
@@ -99,7 +100,7 @@ struct PadTask {
 template <bool PAD>
 __device__ __forceinline__ void pad_claim(const PadArgs &g, PadTask &t) {
   // (a single task has no one to wait for and no flags)
-  const uint64_t n = g.ticket ? atomicAdd(g.ticket, 1u) : 0;
+  const uint64_t n = g.ticket ? atomicAdd(g.ticket, 1u) - g.ticket0 : 0;
   const uint64_t k = t.k = PAD ? g.ntasks - 1 - n : n;
   t.lo = k * g.task > g.P ? k * g.task - g.P : 0;
   t.hi = min64(g.O, (k + 1) * g.task - g.P);
@@ -183,7 +184,7 @@ __global__ void __launch_bounds__(kPadThreads) k_pad(PadArgs g) {
       break;
     }
   __syncthreads();
-  if (tid == 0 && s_ok && g.ticket) st_release_gpu(g.loaded + k, 1u);
+  if (tid == 0 && s_ok && g.ticket) st_release_gpu(g.loaded + k, g.epoch);
 
   // ---- wait for the tasks whose sources lie where this one writes
   if (tid < 32) {
@@ -203,9 +204,9 @@ __global__ void __launch_bounds__(kPadThreads) k_pad(PadArgs g) {
     }
     const uint64_t t1 = global_timer_ns();
     bool good = true;
-    if ((int64_t)k == g.stall_block) good = wait_flag(g.never, t1, g.timeout_ns);
+    if ((int64_t)k == g.stall_block) good = wait_flag(g.never, g.epoch, t1, g.timeout_ns);
     for (int64_t w = k0 + tid; good && w <= k1; w += 32)
-      if (w != (int64_t)k) good = wait_flag(g.loaded + w, t1, g.timeout_ns);
+      if (w != (int64_t)k) good = wait_flag(g.loaded + w, g.epoch, t1, g.timeout_ns);
     if (!good) s_ok = 0;
   }
   __syncthreads();
@@ -293,15 +294,14 @@ static uint32_t pad_task_bytes(uint64_t bytes) {
   return (uint32_t)(std::max(kPadMinTask, std::min(kPadTask, per)) / 128 * 128);
 }
 
-size_t pad_scratch_bytes(const void *buf, int e, uint64_t y, uint64_t pad) {
+uint64_t pad_tasks(const void *buf, int e, uint64_t y, uint64_t pad) {
   const uint64_t O = y * pad * e, task = pad_task_bytes(O);
-  const uint64_t n = (O + ((uintptr_t)buf & 15) + task - 1) / task;
-  return n > 1 ? (size_t)(n + 2) * 4 : 0;
+  return (O + ((uintptr_t)buf & 15) + task - 1) / task;
 }
 
 template <bool PAD>
 static cudaError_t run_pad(cudaStream_t s, void *buf, int e, uint64_t x,
-                           uint64_t y, uint64_t pad, uint32_t *scratch,
+                           uint64_t y, uint64_t pad, const PadFlags &flags,
                            uint32_t *status, uint64_t timeout_ns,
                            int64_t stall_block) {
   if (pad < x) return cudaErrorInvalidValue;
@@ -318,10 +318,13 @@ static cudaError_t run_pad(cudaStream_t s, void *buf, int e, uint64_t x,
   if (g.ntasks >= 0x7fffffffull) return cudaErrorInvalidValue;
   // rows of 1 KB and more with an eighth or more of padding
   g.rows = g.x >= 1024 && (g.pad - g.x) * 8 >= g.pad ? 1u : 0u;
-  if (g.ntasks > 1 && !scratch) return cudaErrorInvalidValue;
-  g.ticket = scratch;
-  g.loaded = scratch + 1;
-  g.never = scratch + 1 + g.ntasks;
+  if (flags.p ? flags.words < g.ntasks + 2 : g.ntasks > 1)
+    return cudaErrorInvalidValue;
+  g.ticket = flags.p;
+  g.loaded = flags.p + 1;
+  g.never = flags.p + flags.words - 1;
+  g.ticket0 = flags.ticket;
+  g.epoch = flags.epoch;
   g.status = status;
   g.timeout_ns = timeout_ns;
   g.stall_block = stall_block;
@@ -343,18 +346,18 @@ static cudaError_t run_pad(cudaStream_t s, void *buf, int e, uint64_t x,
 }
 
 cudaError_t launch_padding(cudaStream_t s, void *buf, int e, uint64_t x,
-                           uint64_t y, uint64_t pad, uint32_t *scratch,
+                           uint64_t y, uint64_t pad, const PadFlags &flags,
                            uint32_t *status, uint64_t timeout_ns,
                            int64_t stall_block) {
-  return run_pad<true>(s, buf, e, x, y, pad, scratch, status, timeout_ns,
+  return run_pad<true>(s, buf, e, x, y, pad, flags, status, timeout_ns,
                        stall_block);
 }
 
 cudaError_t launch_unpadding(cudaStream_t s, void *buf, int e, uint64_t x,
-                             uint64_t y, uint64_t pad, uint32_t *scratch,
+                             uint64_t y, uint64_t pad, const PadFlags &flags,
                              uint32_t *status, uint64_t timeout_ns,
                              int64_t stall_block) {
-  return run_pad<false>(s, buf, e, x, y, pad, scratch, status, timeout_ns,
+  return run_pad<false>(s, buf, e, x, y, pad, flags, status, timeout_ns,
                         stall_block);
 }
 
