@@ -8,7 +8,7 @@
 // unbounded spin, until its predecessor has stored (cl_aos_asta.cl:855-858,
 // 914-917), so the stores of the whole buffer are serialised.
 //
-// GB300 design: a task is a range of the padded layout (24 KB, less where the
+// GB300 design: a task is a range of the padded layout (16 KB, less where the
 // buffer is small), cut at 16-byte addresses, and the compact bytes that
 // belong to it, one range too.  A CTA takes a task from a ticket counter
 // (padding from the back, unpadding from the front), brings its source into
@@ -22,10 +22,13 @@
 //
 // Output is written in the 16-byte vectors of its address: inside a row,
 // which is a shift by a constant, four words from five shared ones; across a
-// row's end, element by element into the vector.  Bound by DRAM for rows of
-// some hundred bytes: 8192 x 12289 floats to 12320 columns (806 MB moved)
-// 173 us = 4.7 TB/s (313 us with tasks of single elements in registers),
-// 7382 x 30496 bytes back to 30484 columns 103 us (596).
+// row's end, two of those, masked (a row end handled element by element kept
+// one warp lane busy for sixteen bytes while the rest waited: 5,195,000 rows
+// of 28 bytes to 32 took 192 us, now 86; 519,500 of 280 to 288 178, now 82).
+// Bound by DRAM and the rate at which tasks start: 8192 x 12289 floats to
+// 12320 columns (806 MB moved) 173 us = 4.7 TB/s (313 us with tasks of single
+// elements in registers), 7382 x 30496 bytes back to 30484 columns 103 us
+// (596).
 #include <algorithm>
 
 #include "lm_core.cuh"
@@ -155,13 +158,24 @@ __device__ __forceinline__ void pad_load(const PadArgs &g, const PadTask &t,
   }
 }
 
+// Mask of the first n of 16 bytes (n <= 16).
+__device__ __forceinline__ uint4 pad_low(uint32_t n) {
+  auto word = [n](uint32_t w) {
+    const uint32_t t = n <= 4 * w ? 0u : min(n - 4 * w, 4u);
+    return (uint32_t)((1ull << (8 * t)) - 1);
+  };
+  return make_uint4(word(0), word(1), word(2), word(3));
+}
+
 // One task per CTA.  (Persistent CTAs that load their next task's source
 // meanwhile publish it only after the current task, so the waits of all
 // others grow into a convoy: 420 us where this form takes 175.)
 template <int E, bool PAD>
 __global__ void __launch_bounds__(kPadThreads) k_pad(PadArgs g) {
   using T = typename Elem<E>::T;
-  extern __shared__ __align__(128) unsigned char smem[];
+  // (reads of masked vectors reach 16 bytes to either side of the source)
+  extern __shared__ __align__(128) unsigned char stage[];
+  unsigned char *smem = stage + 16;
   __shared__ __align__(8) uint64_t bar;
   __shared__ PadTask tk;
   __shared__ int s_ok;
@@ -248,7 +262,30 @@ __global__ void __launch_bounds__(kPadThreads) k_pad(PadArgs g) {
       *reinterpret_cast<uint4 *>(g.buf + o) = make_uint4(0, 0, 0, 0);
       continue;
     }
-    // across a row's end, or at an end of the task: element by element
+    if (whole && row >= 16) {
+      // across a row's end: the rest of row r, and the start of the next
+      uint4 a = make_uint4(0, 0, 0, 0);
+      const uint64_t next = row - c;  // bytes up to the next row's place
+      if (c < g.x) {
+        const uint4 m = pad_low((uint32_t)min64(16, g.x - c));
+        a = pad_read16(smem, (uint32_t)(at0 + (int64_t)(r * from + c)));
+        a = make_uint4(a.x & m.x, a.y & m.y, a.z & m.z, a.w & m.w);
+      }
+      if (next < 16) {
+        const uint32_t n = (uint32_t)next;
+        const uint4 lo4 = pad_low(n),
+                    hi4 = pad_low((uint32_t)min64(16, next + g.x));
+        const uint4 b = pad_read16(
+            stage, (uint32_t)(at0 + 16 + (int64_t)((r + 1) * from) - n));
+        a.x |= b.x & hi4.x & ~lo4.x;
+        a.y |= b.y & hi4.y & ~lo4.y;
+        a.z |= b.z & hi4.z & ~lo4.z;
+        a.w |= b.w & hi4.w & ~lo4.w;
+      }
+      *reinterpret_cast<uint4 *>(g.buf + o) = a;
+      continue;
+    }
+    // rows of a few bytes, or an end of the task: element by element
     T e[16 / E];
     const uint64_t oe = min64((uint64_t)(o + 16), d1);
     uint32_t n = (uint32_t)((oe - ob) / E);
@@ -330,9 +367,9 @@ static cudaError_t run_pad(cudaStream_t s, void *buf, int e, uint64_t x,
   g.stall_block = stall_block;
   g.div_x = make_fastdiv((uint32_t)std::min<uint64_t>(g.x ? g.x : 1, 1u << 30));
   g.div_pad = make_fastdiv((uint32_t)std::min<uint64_t>(g.pad, 1u << 30));
-  // the task's bytes, the rest of its first and last 16, and the word that
-  // the last unaligned read runs over
-  const size_t smem = g.task + 64;
+  // the task's bytes, the rest of its first and last 16, and what masked
+  // vectors read around them
+  const size_t smem = g.task + 128;
   const unsigned grid = (unsigned)g.ntasks;
   ProfScope ps(s, PAD ? "padding" : "unpadding");
   switch (e) {

@@ -55,3 +55,13 @@ def test_alignments(e):
                                        (2, 663, 50001, 672), (8, 25, 200000, 28)])
 def test_large(e, x, y, pad):
     _check(e, x, y, pad)
+
+
+@pytest.mark.parametrize("e", [1, 2, 4, 8])
+@pytest.mark.parametrize("row", [15, 16, 17, 31, 32, 33])
+def test_rows_about_a_vector(e, row):
+    """Rows of one to two output vectors: a vector holds the end of one row
+    and the whole or the start of the next."""
+    for x in sorted({1, 7, row // 2, row - 1}):
+        _check(e, x, 700, row)
+        _check(e, x, 700, row, offset=16 - e)
