@@ -1173,7 +1173,10 @@ constexpr uint64_t kCopyVecsPerItem = 16384;     // 256 KB
 // line from L2 once read, so dirty scratch lines are not written back to
 // DRAM (staged 100s of 64-200 MB: 2-7 % faster than cudaMemcpyAsync;
 // smaller jobs, whose scratch and buffer both fit L2, copy back 3-8 %
-// faster with cudaMemcpyAsync, and from 256 MB the scratch has left L2)
+// faster with cudaMemcpyAsync, and from 256 MB the scratch has left L2).
+// Beside a batch's other work smaller jobs do so too: its copies shared the
+// rest's bandwidth and wrote the scratch to DRAM as well (512 mixed jobs, 9 of
+// them of 17 to 68 MB: 728 us, 708 so; another 512 655 and 640).
 constexpr uint64_t kL2StageMinBytes = 48ull << 20;   // exclusive
 constexpr uint64_t kL2StageMaxBytes = 208ull << 20;
 
@@ -1734,6 +1737,7 @@ struct lm_batch_st {
   // staged waves: gather items, copy-back items, shared memory of the gather
   std::vector<lm::BItem> wgather[lm::kMaxWaves], wcopy[lm::kMaxWaves];
   size_t wsmem[lm::kMaxWaves] = {};
+  bool wragged[lm::kMaxWaves] = {};  // has ragged blocks
   int nwaves = 0;
   char *d_arena = nullptr;  // scratch of the staged jobs of one wave
   uint64_t cap_arena = 0, need_arena = 0;
@@ -2122,6 +2126,7 @@ static bool plan_batch(lm_batch_t bt, const lm_job *jobs, int n,
     bt->wgather[w].clear();
     bt->wcopy[w].clear();
     bt->wsmem[w] = 0;
+    bt->wragged[w] = false;
   }
   bt->nwaves = 0;
   bt->need_arena = 0;
@@ -2283,9 +2288,10 @@ static bool plan_batch(lm_batch_t bt, const lm_job *jobs, int n,
           BJob j;
           uint64_t nblk = 0;
           size_t stage = 0;
-          // (the waves' kernel holds no code for ragged blocks: its mixed
-          // items ran 3 % slower with the registers that these take)
-          tune_params().staged_plain = 1;
+          // (ragged blocks of 1- and 2-byte elements only: 28 MB of bytes in
+          // 12 jobs 52 us without, 29 with; those of 4- and 8-byte elements
+          // gain nothing beside other items, 245 MB 111 us either way)
+          tune_params().staged_plain = nz.e >= 4;
           const bool fits = staged_job(j, jb, nz, &nblk, &stage);
           tune_params().staged_plain = 0;
           if (!fits) goto planner;
@@ -2310,6 +2316,7 @@ static bool plan_batch(lm_batch_t bt, const lm_job *jobs, int n,
             bt->wcopy[w].push_back(it);
           }
           bt->wsmem[w] = std::max<size_t>(bt->wsmem[w], stage);
+          if (j.ragged || j.contig) bt->wragged[w] = true;
           wave_used += foot;
           bt->need_arena = std::max(bt->need_arena, wave_used);
           bt->stats.staged_jobs += 1;
@@ -2413,16 +2420,23 @@ static LaunchCache g_gather3_cache;
 
 static bool launch_staged(cudaStream_t s, const BJob *d_jobs,
                           const BItem *d_items, uint32_t nitems,
-                          uint32_t *counter, size_t smem, bool copyback) {
+                          uint32_t *counter, size_t smem, bool copyback,
+                          bool ragged) {
   if (nitems == 0) return false;
   const DeviceInfo &di = device_info();
-  auto kern = copyback ? k_batch_copyback : k_batch_gather<3, 0, 0>;
+  // (the code of ragged blocks takes registers that mixed items would miss)
+  auto kern = copyback ? k_batch_copyback
+              : ragged ? k_batch_gather<2, 1, 0>
+                       : k_batch_gather<3, 0, 0>;
   // the gather keeps two stages of `smem` bytes
   const size_t dyn = copyback ? 0 : 2 * smem;
-  static LaunchCache copy_cache;
+  static LaunchCache copy_cache, ragged_cache;
   cudaError_t err = cudaSuccess;
   const int occ = prepare_launch((const void *)kern,
-                                 copyback ? copy_cache : g_gather3_cache, dyn,
+                                 copyback ? copy_cache
+                                 : ragged ? ragged_cache
+                                          : g_gather3_cache,
+                                 dyn,
                                  kStageThreads, &err);
   if (err != cudaSuccess || occ < 1) return set_error("batch: occupancy");
   const uint32_t grid =
@@ -2512,7 +2526,8 @@ cudaError_t launch_staged0100(cudaStream_t s, void *buf, int e, uint64_t T,
     gather<<<grid, kStageThreads, dyn, s>>>(g);
     if ((err = cudaGetLastError()) != cudaSuccess) return err;
   }
-  if (g.single.bytes <= kL2StageMinBytes || g.single.bytes > kL2StageMaxBytes ||
+  if ((g.single.bytes <= kL2StageMinBytes && !planner_beside_other_work()) ||
+      g.single.bytes > kL2StageMaxBytes ||
       (((uintptr_t)buf ^ (uintptr_t)scratch) & 15) || getenv("LM_NO_L2STAGE"))
     return cudaMemcpyAsync(buf, scratch, g.single.bytes,
                            cudaMemcpyDeviceToDevice, s);
@@ -3681,12 +3696,12 @@ static bool enqueue_batch(lm_batch_t bt, cudaStream_t s, const lm_job *jobs,
       uint32_t *c = bt->d_counters + (2 + kBandGroups + 2 * w) * kCounterStride;
       if (launch_staged(ws0, bt->d_jobs, bt->d_items + off,
                         (uint32_t)bt->wgather[w].size(), c, bt->wsmem[w],
-                        false))
+                        false, bt->wragged[w]))
         return true;
       off += bt->wgather[w].size();
       if (launch_staged(ws0, bt->d_jobs, bt->d_items + off,
                         (uint32_t)bt->wcopy[w].size(), c + kCounterStride, 0,
-                        true))
+                        true, false))
         return true;
       off += bt->wcopy[w].size();
     }
