@@ -730,11 +730,19 @@ __device__ __forceinline__ void store_b1_vecc(const unsigned char *buf,
 // from the first vector boundary at or after its first row to the first one
 // at or after its last; only the first and the last rows of the matrix leave
 // partial vectors, element by element.  A lane reads the 32-bit words of its
-// 4/E columns in the 2 RW rows from a group's first one on (two shared words
-// and a funnel shift each, as rows start on any byte), transposes them in
-// registers, and takes each column's vector out of its 32 bytes.  Eight
-// lanes take consecutive groups of rows (128 bytes of an output row), four
-// lanes consecutive words.
+// 4/E columns in the RW rows of a group (two shared words and a funnel shift
+// each, as rows start on any byte), transposes them in registers, and turns
+// each column's 16 bytes to start at that column's boundary; what lies past
+// the group comes from the next lane, turned alike.  Eight lanes take
+// consecutive groups of rows and write seven (112 bytes of an output row),
+// four lanes consecutive words.  CONTIG: a lane reads both groups' rows
+// itself and all eight write (their blocks have a multiple of eight groups;
+// 10727152 x 46 bytes 358 us so, 366 by the exchange).
+// Bound by instructions, a third of them the rows' bulk copies, with few
+// warps to issue them: reading 2 RW rows took 118 registers, so two CTAs per
+// SM.  The exchange and three CTAs: 50034 x 4286 bytes 184 -> 165 us, 70825 x
+// 12506 667 -> 590, 10710 x 10711 half-words 167 -> 154, 5004 x 20003 bytes
+// 90 -> 84 (three CTAs alone: 172, 615, 158, 92).
 // tab holds each row's offset in the stage, rounded down to words, RW rows and
 // 4 words of padding per group (the eight lanes' reads fall in distinct
 // banks), 0 for rows that are not there; its first word of padding holds the
@@ -751,12 +759,14 @@ __device__ __forceinline__ void store_b1_ragged(
   static_assert(E == 1 || E == 2, "narrow elements only");
   using T = typename Elem<E>::T;
   constexpr uint32_t RW = 16 / E, TW = RW + 4, CW = 4 / E;
+  constexpr uint32_t QN = CONTIG ? 8 : 4;
   const uint32_t lane = threadIdx.x & 31;
   const uint32_t ng = S / RW;
   const uint32_t nwc = (ncols + CW - 1) / CW;
   // eight lanes on consecutive groups (four where there are no more)
-  const uint32_t lg = ng > 4 ? 3 : 2;
-  const uint32_t ngc = (ng + (1 << lg) - 1) >> lg;
+  const uint32_t lg = ng > (CONTIG ? 4 : 3) ? 3 : 2, last = (1u << lg) - 1;
+  const uint32_t per = CONTIG ? last + 1 : last;  // groups that they write
+  const uint32_t ngc = (ng + per - 1) / per;
   const uint32_t nwd = (nwc + (32 >> lg) - 1) >> (5 - lg);
   // bits of a row's first element past a word: the same every fourth row
   const uint32_t m0 = CONTIG ? tab[0] : tab[RW];
@@ -764,66 +774,91 @@ __device__ __forceinline__ void store_b1_ragged(
                  sh3 = (m0 + 3 * rb) * 8;
   for (uint32_t u = warp; u < ngc * nwd; u += nwarps) {
     const uint32_t d = u / ngc, gc = u - d * ngc;
-    const uint32_t g = (gc << lg) + (lane & ((1 << lg) - 1));
+    const uint32_t g = gc * per + (lane & last);
     const uint32_t wc = (d << (5 - lg)) + (lane >> lg);
-    if (g >= ng || wc >= nwc || g * RW >= nrows) continue;
-    uint32_t w[CW][8];  // 2 RW rows of each column
-    const uint32_t *tg = tab + g * TW;
-    const unsigned char *bw = buf + wc * 4;
-    auto word = [&](uint32_t off, uint32_t sh) {
-      const uint32_t *q = reinterpret_cast<const uint32_t *>(bw + off);
-      return __funnelshift_r(q[0], q[1], sh);
-    };
-    // rows without a table: the words of rows 0..3 of the group, a multiple
-    // of 4 bytes further on for each four rows
-    const uint32_t o0 = m0 + g * (RW * pitch + gp);
-    const uint32_t c0 = o0 & ~3u, c1 = (o0 + pitch) & ~3u,
-                   c2 = (o0 + 2 * pitch) & ~3u, c3 = (o0 + 3 * pitch) & ~3u;
+    if (CONTIG && (wc >= nwc || g >= ng || g * RW >= nrows)) continue;
+    uint32_t w[CW][QN];  // the group's rows of each column (CONTIG: 2 RW)
+    if constexpr (!CONTIG)
+      for (uint32_t c = 0; c < CW; ++c)
+        for (uint32_t q = 0; q < QN; ++q) w[c][q] = 0;
+    if (CONTIG ||
+        (wc < nwc && g <= ng && (g == 0 || (g - 1) * RW < nrows))) {
+      const uint32_t *tg = tab + g * TW;
+      const unsigned char *bw = buf + wc * 4;
+      auto word = [&](uint32_t off, uint32_t sh) {
+        const uint32_t *q = reinterpret_cast<const uint32_t *>(bw + off);
+        return __funnelshift_r(q[0], q[1], sh);
+      };
+      // rows without a table: the words of rows 0..3 of the group, a multiple
+      // of 4 bytes further on for each four rows
+      const uint32_t o0 = m0 + g * (RW * pitch + gp);
+      const uint32_t c0 = o0 & ~3u, c1 = (o0 + pitch) & ~3u,
+                     c2 = (o0 + 2 * pitch) & ~3u, c3 = (o0 + 3 * pitch) & ~3u;
 #pragma unroll
-    for (uint32_t q = 0; q < 8; ++q) {
-      if constexpr (E == 1) {
-        uint4 t;
-        if constexpr (CONTIG) {
-          const uint32_t st = q * 4 * pitch + (q / 4) * gp;
-          t = make_uint4(c0 + st, c1 + st, c2 + st, c3 + st);
+      for (uint32_t q = 0; q < QN; ++q) {
+        if constexpr (E == 1) {
+          uint4 t;
+          if constexpr (CONTIG) {
+            const uint32_t st = q * 4 * pitch + (q / 4) * gp;
+            t = make_uint4(c0 + st, c1 + st, c2 + st, c3 + st);
+          } else {
+            t = *reinterpret_cast<const uint4 *>(tg + q * 4);
+          }
+          const uint32_t a0 = word(t.x, sh0), a1 = word(t.y, sh1),
+                         a2 = word(t.z, sh2), a3 = word(t.w, sh3);
+          const uint32_t lo01 = __byte_perm(a0, a1, 0x5140);
+          const uint32_t hi01 = __byte_perm(a0, a1, 0x7362);
+          const uint32_t lo23 = __byte_perm(a2, a3, 0x5140);
+          const uint32_t hi23 = __byte_perm(a2, a3, 0x7362);
+          w[0][q] = __byte_perm(lo01, lo23, 0x5410);
+          w[1][q] = __byte_perm(lo01, lo23, 0x7632);
+          w[2][q] = __byte_perm(hi01, hi23, 0x5410);
+          w[3][q] = __byte_perm(hi01, hi23, 0x7632);
         } else {
-          t = *reinterpret_cast<const uint4 *>(tg + (q / 4) * TW + (q % 4) * 4);
+          uint2 t;
+          if constexpr (CONTIG) {
+            const uint32_t st = (q / 2) * 4 * pitch + (q / 4) * gp;
+            t = q % 2 ? make_uint2(c2 + st, c3 + st)
+                      : make_uint2(c0 + st, c1 + st);
+          } else {
+            t = *reinterpret_cast<const uint2 *>(tg + q * 2);
+          }
+          const uint32_t a0 = word(t.x, q % 2 ? sh2 : sh0),
+                         a1 = word(t.y, q % 2 ? sh3 : sh1);
+          w[0][q] = __byte_perm(a0, a1, 0x5410);
+          w[1][q] = __byte_perm(a0, a1, 0x7632);
         }
-        const uint32_t a0 = word(t.x, sh0), a1 = word(t.y, sh1),
-                       a2 = word(t.z, sh2), a3 = word(t.w, sh3);
-        const uint32_t lo01 = __byte_perm(a0, a1, 0x5140);
-        const uint32_t hi01 = __byte_perm(a0, a1, 0x7362);
-        const uint32_t lo23 = __byte_perm(a2, a3, 0x5140);
-        const uint32_t hi23 = __byte_perm(a2, a3, 0x7362);
-        w[0][q] = __byte_perm(lo01, lo23, 0x5410);
-        w[1][q] = __byte_perm(lo01, lo23, 0x7632);
-        w[2][q] = __byte_perm(hi01, hi23, 0x5410);
-        w[3][q] = __byte_perm(hi01, hi23, 0x7632);
-      } else {
-        uint2 t;
-        if constexpr (CONTIG) {
-          const uint32_t st = (q / 2) * 4 * pitch + (q / 4) * gp;
-          t = q % 2 ? make_uint2(c2 + st, c3 + st) : make_uint2(c0 + st, c1 + st);
-        } else {
-          t = *reinterpret_cast<const uint2 *>(tg + (q / 4) * TW + (q % 4) * 2);
-        }
-        const uint32_t a0 = word(t.x, q % 2 ? sh2 : sh0),
-                       a1 = word(t.y, q % 2 ? sh3 : sh1);
-        w[0][q] = __byte_perm(a0, a1, 0x5410);
-        w[1][q] = __byte_perm(a0, a1, 0x7632);
       }
     }
+    const bool out = (CONTIG || (lane & last) < last) && g < ng;
     unsigned char *run =
         reinterpret_cast<unsigned char *>(dst + (uint64_t)(wc * CW) * ostride);
 #pragma unroll
     for (uint32_t c = 0; c < CW; ++c, run += (uint64_t)ostride * E) {
       const uint32_t h = (16 - ((uintptr_t)run & 15)) & 15;  // bytes
-      uint32_t x[6], y[5];
+      // the words from the one of byte h on
+      uint32_t y[5];
+      if constexpr (CONTIG) {
+        uint32_t x[6];
 #pragma unroll
-      for (int i = 0; i < 6; ++i) x[i] = h & 8 ? w[c][i + 2] : w[c][i];
+        for (int i = 0; i < 6; ++i) x[i] = h & 8 ? w[c][i + 2] : w[c][i];
 #pragma unroll
-      for (int i = 0; i < 5; ++i) y[i] = h & 4 ? x[i + 1] : x[i];
-      if (wc * CW + c < ncols && g * 16 + h + 16 <= nrows * E)
+        for (int i = 0; i < 5; ++i) y[i] = h & 4 ? x[i + 1] : x[i];
+      } else {
+        uint32_t x[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) x[i] = h & 8 ? w[c][i ^ 2] : w[c][i];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) y[i] = h & 4 ? x[(i + 1) & 3] : x[i];
+        // (h is a column's, so the next lane has turned its words alike)
+        y[4] = __shfl_down_sync(kFull, y[0], 1);
+#pragma unroll
+        for (int i = 1; i < 4; ++i) {
+          const uint32_t next = __shfl_down_sync(kFull, y[i], 1);
+          if (i * 4 + h >= 16) y[i] = next;
+        }
+      }
+      if (out && wc * CW + c < ncols && g * 16 + h + 16 <= nrows * E)
         __stcg(reinterpret_cast<uint4 *>(run + g * 16 + h),
                make_uint4(__funnelshift_r(y[0], y[1], h * 8),
                           __funnelshift_r(y[1], y[2], h * 8),
@@ -1418,7 +1453,8 @@ __device__ void gather_store(const BJob &j, uint32_t q, const unsigned char *buf
 // gather 0.0933 vs 0.0963 ms; 500 x 268435: 0.161 vs 0.167 ms; 1-byte
 // 16384 x 16384 the other way: 0.126 vs 0.121 ms).
 // RAG: with the code of ragged blocks and of rows staged as one range (in a
-// kernel of its own: it takes 128 registers).
+// kernel of its own: alone it has the registers of three CTAs, but not beside
+// the other items of a batch: 697 us with two, 715 with three).
 template <int MB, int RAG, int ES>
 __global__ void __launch_bounds__(kStageThreads, MB) k_batch_gather(const __grid_constant__ BatchArgs g) {
   extern __shared__ __align__(128) unsigned char smem[];
@@ -2007,6 +2043,8 @@ static bool staged_job(BJob &j, const lm_job &jb, const Normalized &nz,
       Si = kStageTileBytes / (Sj * nz.e);
     }
     Si = std::max<uint64_t>(std::min<uint64_t>(Si, kStageMaxS) / RW, 2) * RW - RW;
+    // (store_b1_ragged writes seven groups of RW rows at a time)
+    if (Si >= 7 * RW) Si = Si / (7 * RW) * (7 * RW);
   }
   if (j.contig || (off && Si < nz.a)) {
     // blocks that take RW - 1 rows beyond theirs (store_b1_ragged): as many
@@ -2501,7 +2539,7 @@ cudaError_t launch_staged0100(cudaStream_t s, void *buf, int e, uint64_t T,
   static const Kern kerns[2][4] = {
       {k_batch_gather<3, 0, 1>, k_batch_gather<3, 0, 2>, k_batch_gather<3, 0, 4>,
        k_batch_gather<3, 0, 8>},
-      {k_batch_gather<2, 1, 1>, k_batch_gather<2, 1, 2>, k_batch_gather<3, 2, 4>,
+      {k_batch_gather<3, 1, 1>, k_batch_gather<3, 1, 2>, k_batch_gather<3, 2, 4>,
        k_batch_gather<3, 2, 8>}};
   static LaunchCache caches[2][4];
   const int r = g.single.ragged || g.single.contig ? 1 : 0;
@@ -2878,7 +2916,7 @@ cudaError_t launch_wave0100(cudaStream_t s, void *buf, int e, uint64_t a,
     using Kern = void (*)(const WaveArgs);
     static const Kern kerns[2][4] = {
         {k_wave<3, 0, 1>, k_wave<3, 0, 2>, k_wave<3, 0, 4>, k_wave<3, 0, 8>},
-        {k_wave<2, 1, 1>, k_wave<2, 1, 2>, k_wave<3, 2, 4>, k_wave<3, 2, 8>}};
+        {k_wave<3, 1, 1>, k_wave<3, 1, 2>, k_wave<3, 2, 4>, k_wave<3, 2, 8>}};
     static LaunchCache caches[2][4];
     const int w = e == 1 ? 0 : e == 2 ? 1 : e == 4 ? 2 : 3;
     const Kern kern = kerns[rag ? 1 : 0][w];

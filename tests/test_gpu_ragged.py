@@ -73,3 +73,14 @@ def test_near_the_limit():
     """Payloads that shared memory holds only without the extra rows."""
     for a, B in ((1001, 26816), (5007, 6001), (3001, 10007)):
         _check(1, a, B, 1, RESIDENT)
+
+
+@pytest.mark.parametrize("e", [1, 2])
+@pytest.mark.parametrize("groups", [1, 2, 3, 4, 6, 7, 8, 13, 14, 15, 28])
+def test_groups_of_rows(groups, e):
+    """Columns of so many 16-byte groups and a row less or more: groups are
+    written seven (three) at a time with the rows of the one after."""
+    for a in (groups * 16 // e - 1, groups * 16 // e + 1):
+        for B in (7, 131, 517):
+            _check(2, a, B, e, STAGED)
+            _check(2, a, B, e, RESIDENT)
