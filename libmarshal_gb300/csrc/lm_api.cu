@@ -347,9 +347,33 @@ static uint64_t wait_timeout_ns() {
 // ---- planner ----------------------------------------------------------------
 
 constexpr uint64_t kWalkMinBytes = 16ull << 20;
-// (what is smaller is held in shared memory, or, under capture, leaves too
-// few steps)
-constexpr uint64_t kWaveMinBytes = 32ull << 20;
+
+// Whether the ordered form (3 x payload, k_wave) is faster than the staged one
+// (4 x, but no waits, and a copy back out of L2 up to 208 MB): its slack is
+// 20 MB of blocks in flight.  Microseconds, staged and ordered: floats of 401
+// columns, 90 MB 58 and 62, 120 MB 79 and 80, 150 MB 97 and 93; doubles of
+// 2001, 90 MB 57 and 55, 150 MB 97 and 86; half-words of 1001, 120 MB 88 and
+// 92, 150 MB 110 and 110; bytes of 5001, 120 MB 95 and 100, 150 MB 121 and
+// 119.  Output rows of whole vectors: floats 88 MB 57 and 56, 109 MB 73 and
+// 66; bytes 104 MB 70 and 72, 131 MB 91 and 87; units of 32 bytes, 81 MB 50
+// and 50, 101 MB 65 and 60.  Short rows make more blocks per byte: rows of
+// 46 bytes, 190 MB 138 and 151, 300 MB 223 and 226; 17 floats, 150 MB 99 and
+// 107, 300 MB 201 and 190; 11 floats, 600 MB 404 and 423; 3 doubles 513 and
+// 663.  Several instances run in the ordered form one after another, in the
+// staged one at once: 3 of 100 MB of floats 199 and 197, 3 of 168 MB 330 and
+// 300, 2 of 268 MB 351 and 282; 3 of 117 MB of bytes 279 and 291.
+static bool wave_preferred(const void *buf, uint64_t T, uint64_t a, uint64_t B,
+                           uint64_t U) {
+  const uint64_t bytes = a * B * U, row = B * U;
+  const bool vectors = ((uintptr_t)buf & 15) == 0 && a * U % 16 == 0;
+  uint64_t least = (U < 4 ? (vectors ? 104ull : 144ull)
+                          : (vectors ? 88ull : 112ull)) << 20;
+  if (U < 4 && row <= 304) least = 208ull << 20;
+  if (U >= 4 && row < 96) least = 192ull << 20;
+  if (U >= 4 && row < 64) return false;
+  if (T > 1) least = std::max<uint64_t>(least, 128ull << 20);
+  return bytes >= least;
+}
 
 // elements of one CTA's on-chip tile past which the form held in shared
 // memory is the faster one
@@ -559,15 +583,26 @@ static bool do_0100(cudaStream_t s, void *buf, int e, uint64_t T, uint64_t a,
   }
   // a large matrix at 3 x payload: half of its blocks in place, the others
   // through scratch (lm_batch.cu, k_wave)
-  if (m == Method::Auto && T == 1 && U < kStagedMaxUnit &&
-      a * B * U >= kWaveMinBytes && !getenv("LM_NO_WAVE")) {
-    const size_t need = wave0100_scratch(buf, a, B, b, e);
-    uint32_t *status = need ? device_status_word() : nullptr;
+  if (m == Method::Auto && U < kStagedMaxUnit &&
+      wave_preferred(buf, T, a, B, U) && !getenv("LM_NO_WAVE")) {
+    // (the same plan for every instance, but for its place in 16 bytes)
+    const uint64_t step = a * B * U;
+    size_t need = 0;
+    bool fits = true;
+    for (uint64_t t = 0; t < T && t < 16 && fits; ++t) {
+      const size_t n = wave0100_scratch((char *)buf + t * step, a, B, b, e);
+      fits = n != 0;
+      need = std::max(need, n);
+    }
+    uint32_t *status = fits ? device_status_word() : nullptr;
     Scratch sc;
-    if (need && status && try_scratch(sc, need, s))
-      return check_launch(launch_wave0100(s, buf, e, a, B, b, sc.p, status,
-                                          wait_timeout_ns()),
-                          "wave launch");
+    if (fits && status && try_scratch(sc, need, s)) {
+      cudaError_t err = cudaSuccess;
+      for (uint64_t t = 0; t < T && err == cudaSuccess; ++t)
+        err = launch_wave0100(s, (char *)buf + t * step, e, a, B, b, sc.p,
+                              status, wait_timeout_ns());
+      return check_launch(err, "wave launch");
+    }
   }
   // any shape through scratch: block transposes out of place, then a copy
   // back (4 x payload, but every access in whole sectors); falls through

@@ -33,8 +33,8 @@ def _check(a, B, b, e, offset=0, wave=True):
 # output rows of whole vectors and not, both directions, last blocks of one
 # row or column, whole rows (one block column) and whole columns
 @pytest.mark.parametrize("a,B,b,e", [
-    (16000, 8192, 1, 1), (16001, 16385, 1, 1), (1001, 268167, 1, 1),
-    (268167, 1001, 1, 1), (149, 1500001, 1, 1), (12000001, 15, 1, 1),
+    (20000, 8192, 1, 1), (16001, 16385, 1, 1), (1001, 268167, 1, 1),
+    (268167, 1001, 1, 1), (149, 1500001, 1, 1), (16000001, 15, 1, 1),
     (12000, 8000, 1, 2), (12001, 8003, 1, 2), (20003, 5001, 1, 2),
     (3000001, 40, 1, 2), (18, 7000001, 1, 2),
     (9001, 6000, 1, 4), (6000, 9001, 1, 4), (12289, 8193, 1, 4),
@@ -86,3 +86,26 @@ def test_concurrent_streams():
     for b, w in zip(bufs, want):
         assert torch.equal(b, w)
     assert lm.lib().lm_device_status(None) == 0
+
+
+@pytest.mark.parametrize("T,a,B,e", [(3, 6001, 6003, 4), (2, 15159, 10641, 1),
+                                     (17, 4001, 4201, 8), (2, 9001, 9003, 2)])
+def test_instances(T, a, B, e):
+    """Large instances one after another, each at its own place in 16 bytes."""
+    n = a * B * e
+    raw = torch.randint(0, 256, (T * n,), dtype=torch.uint8, device="cuda")
+    want = raw.view(T, a, B, e).transpose(1, 2).reshape(-1)
+    lm.prof_collect()
+    lm.prof_enable(True)
+    lm.transpose_0100(raw, T, a, B, 1, elem_bytes=e)
+    torch.cuda.synchronize()
+    lm.prof_enable(False)
+    assert set(lm.prof_collect()) == {"wave", "suffix_copy"}
+    assert torch.equal(raw, want)
+
+
+@pytest.mark.parametrize("a,B,e", [(9000001, 5, 4), (40001, 701, 4),
+                                   (24001, 5001, 1), (3000001, 33, 2)])
+def test_staged_is_left(a, B, e):
+    """Below the sizes of the ordered form, and rows too short for it."""
+    _check(a, B, 1, e, wave=False)
