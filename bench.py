@@ -42,10 +42,10 @@ CONFIG = {
     "steps_alternate": "(16384,12289) then (12289,16384)",
 }
 # DRAM traffic of the dominant kernel per launch (dram__bytes_read.sum +
-# dram__bytes_write.sum), from one ncu capture of k_stash_wave on the
-# forward 100(16384, 12289) fp32 call (profiles/stash_wave_save_100_16384x
-# 12289_f32.txt): 809.8 MB read + 753.3 MB written.
-NCU_TRAFFIC = {"stash_wave": 1563118848}
+# dram__bytes_write.sum), from one ncu capture of k_wave on the forward
+# 100(16384, 12289) fp32 call (profiles/wave_100_16384x12289_f32.txt): 809.6 MB
+# read + 751.3 MB written.
+NCU_TRAFFIC = {"wave": 1560905984}
 
 
 def peak_hbm():
