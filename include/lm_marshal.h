@@ -25,17 +25,21 @@
  *     the caller's stream (calls on different streams never share it):
  *       cycle following (PTTWAC): one done bit per unit (a 16384 x 12289
  *         fp32 transpose: 786 KB);
- *       the stash plan (100 on units under 128 bytes, e.g. the plain
- *         transpose of a large matrix): the stash, about half the payload
- *         (421 MB for 16384 x 12289 fp32), plus 8 bytes per row;
- *       the staged form (blocks transposed out of place, then copied back):
- *         the payload's size plus 16 bytes;
- *       padding: 8 bytes per 4096-element task;
+ *       the ordered form (large 100s on units under 1 KB, e.g. the plain
+ *         transpose of a large matrix) and the staged form (blocks
+ *         transposed out of place, then copied back): the payload's size
+ *         and a little more (the ordered form of several instances: one
+ *         instance's size);
+ *       walks (100s on units of 128 bytes and more): an eighth of the
+ *         payload and a list of the cycles' segments;
+ *       padding: 4 bytes per task of up to 16 KB, up to 16 blocks of 64 KB
+ *         kept per device until lm_marshal_finalize;
  *     payloads that fit the shared memory of all SMs (about 30 MB on GB300)
- *     move through shared memory instead and take no scratch.
- *     When the pool cannot supply the stash or the staged form's scratch
- *     the planner falls through to a method that needs less (ultimately
- *     cycle following); lm_transpose_100_noalloc allocates nothing.
+ *     and square matrices move through shared memory instead and take none.
+ *     When the pool cannot supply a method's scratch the planner falls
+ *     through to one that needs less: the stash plan (about half the
+ *     payload, 421 MB for 16384 x 12289 fp32, plus 8 bytes per row),
+ *     ultimately cycle following; lm_transpose_100_noalloc allocates nothing.
  *
  * Notation: 010  [A][a][B]     -> [A][B][a]
  *           100  [A][B][b]     -> [B][A][b]

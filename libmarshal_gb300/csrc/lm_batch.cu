@@ -39,8 +39,8 @@ constexpr size_t kCounterBytes =
     (size_t)(5 + kBandGroups + 2 * kMaxWaves) * kCounterStride * 4;
 constexpr int kT010Counter = 2 + kBandGroups + 2 * kMaxWaves;
 constexpr uint64_t kDefaultArenaBytes = 1ull << 30;
-// jobs at least this large that the stash plan applies to skip the staged
-// form (the stash moves 3 x payload, the staged form 4 x)
+// jobs at least this large and with enough rows skip the waves: the planner
+// takes the ordered form (3 x payload, the staged form 4 x) where that pays
 constexpr uint64_t kStashPreferBytes = 64ull << 20;
 constexpr int kSideStreams = 6;      // streams of the large jobs
 constexpr int kGroupStreams = 8;     // streams of the item groups
@@ -2301,8 +2301,8 @@ static bool plan_batch(lm_batch_t bt, const lm_job *jobs, int n,
         bt->stats.big_bytes += bytes;
         continue;
       }
-      // a large 100 that the stash plan serves (3 x payload instead of the
-      // staged form's 4) goes to the planner
+      // a large 100 of many rows goes to the planner (whose ordered form moves
+      // 3 x payload instead of the staged form's 4)
       if (nz.T == 1 && unit < 128 && bytes >= kStashPreferBytes &&
           nz.a >= kStashRowsPerSm * (uint64_t)di.sms &&
           nz.a * nz.B >= (1ull << 20) &&
