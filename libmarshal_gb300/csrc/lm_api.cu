@@ -375,6 +375,21 @@ static bool wave_preferred(const void *buf, uint64_t T, uint64_t a, uint64_t B,
   return bytes >= least;
 }
 
+// Half-words in tall matrices whose output rows are no whole vectors long: the
+// ordered form stages 7 rows more than it writes of each block, and from some
+// 23000 rows on the stash plan's strips are the shorter ones.  Microseconds,
+// stash and ordered: 22001 x 10005 276 and 277, 24001 x 14003 393 and 412,
+// 28775 x 13530 443 and 476, 30001 x 20003 677 and 731, 36001 x 9005 363 and
+// 399; but rows of 2 bytes past whole vectors, 28775 x 7001 274 and 257, 33001 x
+// 15001 631 and 594.  (Bytes, 28775 x 27060: 657 and 514.)
+static bool stash_preferred(const void *buf, uint64_t T, uint64_t a, uint64_t B,
+                            uint64_t b, int e) {
+  if (T != 1 || e != 2 || b != 1 || a < 23000 || B * 2 % 16 == 2) return false;
+  if (a * 2 % 16 == 0) return false;
+  return wave_preferred(buf, T, a, B, 2) && !getenv("LM_NO_STASH") &&
+         plan_stash(a, B, 1, 2).feasible;
+}
+
 // elements of one CTA's on-chip tile past which the form held in shared
 // memory is the faster one
 constexpr uint64_t kTileElems = 16 * 1024;
@@ -581,9 +596,11 @@ static bool do_0100(cudaStream_t s, void *buf, int e, uint64_t T, uint64_t a,
                          cs == cudaStreamCaptureStatusNone),
           "walk launch");
   }
+  const bool stash_first =
+      m == Method::Auto && stash_preferred(buf, T, a, B, b, e);
   // a large matrix at 3 x payload: half of its blocks in place, the others
   // through scratch (lm_batch.cu, k_wave)
-  if (m == Method::Auto && U < kStagedMaxUnit &&
+  if (m == Method::Auto && U < kStagedMaxUnit && !stash_first &&
       wave_preferred(buf, T, a, B, U) && !getenv("LM_NO_WAVE")) {
     // (the same plan for every instance, but for its place in 16 bytes)
     const uint64_t step = a * B * U;
@@ -613,7 +630,7 @@ static bool do_0100(cudaStream_t s, void *buf, int e, uint64_t T, uint64_t a,
   // on 18 tiles of 72 x 100 1600-byte units ran 2.3 TB/s, the staged form
   // 2.9 TB/s)
   if (m == Method::Staged ||
-      (m == Method::Auto &&
+      (m == Method::Auto && !stash_first &&
        (U < kStagedMaxUnit || (T > 1 && a * B < 65536)) &&
        T * a * B * b * e >= (1ull << 20) &&
        !getenv("LM_NO_STAGED"))) {

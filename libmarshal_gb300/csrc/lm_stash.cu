@@ -9,7 +9,8 @@
 // form (k_wave, lm_batch.cu) moves as much with blocks by ticket and is as fast
 // or faster (16384 x 12289 floats 389 us here, 390 there; 32768 x 16000 doubles
 // 2555 and 1896), so the planner comes here where that form's scratch, the
-// payload's size, cannot be had: the stash is half of it.
+// payload's size, cannot be had (the stash is half of it), and for tall
+// matrices of unaligned half-words (28775 x 13530: 443 and 476 us).
 //
 //   [A][B] units -> [B][A].  Destination rows are produced in groups of g
 //   (one group = g source columns, a column strip of the source) in order

@@ -109,3 +109,24 @@ def test_instances(T, a, B, e):
 def test_staged_is_left(a, B, e):
     """Below the sizes of the ordered form, and rows too short for it."""
     _check(a, B, 1, e, wave=False)
+
+
+@pytest.mark.parametrize("a,B,ran", [
+    (28775, 4005, {"stash_save", "stash_wave"}),
+    (28776, 4005, {"wave", "suffix_copy"}),  # whole vectors
+    (28775, 4001, {"wave", "suffix_copy"}),  # rows 2 bytes past some
+    (22999, 5005, {"wave", "suffix_copy"}),
+    (40001, 3005, {"wave", "suffix_copy"}),  # more rows than the stash takes
+])
+def test_tall_half_words(a, B, ran):
+    """Which of the two forms at 3 x payload takes tall matrices."""
+    x = torch.randint(-30000, 30000, (a, B), dtype=torch.int16, device="cuda")
+    want = x.t().reshape(-1)
+    lm.transpose_100(x.clone(), a, B, 1)  # (plans are kept per shape)
+    lm.prof_collect()
+    lm.prof_enable(True)
+    lm.transpose_100(x, a, B, 1)
+    torch.cuda.synchronize()
+    lm.prof_enable(False)
+    assert set(lm.prof_collect()) == ran
+    assert torch.equal(x.view(-1), want)
