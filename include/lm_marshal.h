@@ -217,6 +217,14 @@ bool lm_debug_resident_stall(lm_stream_t stream, void *buf, int elem_bytes,
                              int A, int a, int B, int b,
                              unsigned long long timeout_ns);
 
+/* Failure-detection hook (no reference counterpart): the ordered form of
+ * 100(a, B, b) with each block waiting for one block more of an earlier step
+ * than there are.  Every wait gives up after timeout_ns; the call must return
+ * true and leave the CUDA context usable (the buffer holds part of the
+ * transposition). */
+bool lm_debug_wave_stall(lm_stream_t stream, void *buf, int elem_bytes, int a,
+                         int B, int b, unsigned long long timeout_ns);
+
 /* ---- batched conversion (no reference counterpart) -------------------------
  * A batch is a list of independent in-place jobs, each on its own device
  * buffer (buffers must not overlap), of any op and element width.

@@ -1219,6 +1219,32 @@ bool lm_debug_resident_stall(lm_stream_t stream, void *buf, int elem_bytes,
   return check_status(s, "resident");
 }
 
+// Failure-detection hook: the ordered form of 100(a, B, b) whose blocks wait
+// for one block more of each step than there are, bounded by timeout_ns.  Must
+// return true (error) with a timeout message and leave the context usable.
+bool lm_debug_wave_stall(lm_stream_t stream, void *buf, int elem_bytes, int a,
+                         int B, int b, unsigned long long timeout_ns) {
+  cudaStream_t s = (cudaStream_t)stream;
+  if (!valid_e(elem_bytes))
+    return fail("element size must be 1, 2, 4 or 8 (got %d)", elem_bytes);
+  if (a <= 1 || B <= 1 || b <= 0) return fail("dimensions must be positive");
+  if (buf == nullptr) return fail("null buffer");
+  if (misaligned(buf, elem_bytes))
+    return fail("buffer must be aligned to the element size");
+  const size_t need = wave0100_scratch(buf, (uint64_t)a, (uint64_t)B,
+                                       (uint64_t)b, elem_bytes);
+  if (need == 0) return fail("wave: the ordered form does not take this shape");
+  uint32_t *status = device_status_word();
+  if (!status) return fail("wave: no status word");
+  Scratch sc;
+  if (get_scratch(sc, need, s)) return true;
+  if (check_launch(launch_wave0100(s, buf, elem_bytes, (uint64_t)a, (uint64_t)B,
+                                   (uint64_t)b, sc.p, status, timeout_ns, 1),
+                   "wave launch"))
+    return true;
+  return check_status(s, "wave");
+}
+
 // Waits for `stream` and returns (then clears) the accumulated status of
 // waiting kernels on the current device: 0 = ok.
 unsigned lm_device_status(lm_stream_t stream) {

@@ -2602,7 +2602,7 @@ cudaError_t launch_staged0100(cudaStream_t s, void *buf, int e, uint64_t T,
 struct WaveArgs {
   BJob job;
   uint32_t nsteps, per;  // blocks of a step
-  uint32_t group, gper;  // steps and blocks of a count
+  uint32_t group, gper;  // steps of a count, and what it is waited to reach
   uint32_t nblk, M, backward;
   uint32_t stage_bytes;
   uint32_t lines;        // step: rows or columns of its blocks
@@ -2699,8 +2699,12 @@ __global__ void __launch_bounds__(kStageThreads, MB) k_wave(const __grid_constan
         const bool full = f < need && ld_acquire_gpu(done + f) >= g.gper;
         const unsigned mask = ~__ballot_sync(kFull, full);
         frontier += mask ? __ffs(mask) - 1 : 32;
-        if (frontier < need && (s_dead || global_timer_ns() - t0 > g.timeout_ns)) {
-          s_dead = 1;
+        // (decided by the warp as one: a lane that gave up by itself would
+        // leave the others in the next ballot)
+        const bool late = *(volatile int *)&s_dead ||
+                          global_timer_ns() - t0 > g.timeout_ns;
+        if (frontier < need && __any_sync(kFull, late)) {
+          if (lane == 0) s_dead = 1;
           break;
         }
       }
@@ -2879,10 +2883,12 @@ size_t wave0100_scratch(void *buf, uint64_t a, uint64_t B, uint64_t b, int e) {
 
 cudaError_t launch_wave0100(cudaStream_t s, void *buf, int e, uint64_t a,
                             uint64_t B, uint64_t b, void *scratch,
-                            uint32_t *status, uint64_t timeout_ns) {
+                            uint32_t *status, uint64_t timeout_ns,
+                            uint32_t missing) {
   WaveArgs g{};
   size_t need = 0;
   if (!plan_wave(g, &need, buf, a, B, b, e)) return cudaErrorInvalidValue;
+  g.gper += missing;
   // the scratch copy sits at the buffer's address modulo 16
   g.job.scratch = (char *)scratch + ((uintptr_t)buf & 15);
   g.ticket = (uint32_t *)((char *)scratch + need - ((size_t)g.nsteps + 1) * 4);

@@ -216,10 +216,13 @@ cudaError_t launch_staged0100(cudaStream_t s, void *buf, int e, uint64_t T,
 // ---- one large 0100 at 3 x payload (lm_batch.cu) ------------------------------
 // The staged form's blocks in an order that lets half of them be written in
 // place.  wave0100_scratch: bytes of `scratch`, 0 where it does not apply.
+// `missing` blocks more than there are are waited for (failure-detection test
+// hook).
 size_t wave0100_scratch(void *buf, uint64_t a, uint64_t B, uint64_t b, int e);
 cudaError_t launch_wave0100(cudaStream_t s, void *buf, int e, uint64_t a,
                             uint64_t B, uint64_t b, void *scratch,
-                            uint32_t *status, uint64_t timeout_ns);
+                            uint32_t *status, uint64_t timeout_ns,
+                            uint32_t missing = 0);
 
 // ---- square 0100s (lm_batch.cu) ----------------------------------------------
 // T squares of a x a units, block pairs exchanged through shared memory: 2 x

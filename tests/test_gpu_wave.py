@@ -130,3 +130,25 @@ def test_tall_half_words(a, B, ran):
     lm.prof_enable(False)
     assert set(lm.prof_collect()) == ran
     assert torch.equal(x.view(-1), want)
+
+
+# forward and backward, blocks of whole vectors and ragged ones
+@pytest.mark.parametrize("a,B,b,e", [(8192, 8191, 1, 4), (8191, 4097, 1, 4),
+                                     (125000, 101, 8, 4), (40001, 3001, 1, 1),
+                                     (300001, 301, 1, 2)])
+def test_wait_that_runs_out_is_reported(a, B, b, e):
+    """Blocks that wait for one block more of an earlier step than there are
+    give up after 20 ms, as whole warps; the call reports it, and the next ones
+    work."""
+    x = torch.randint(0, 256, (a * B * b * e,), dtype=torch.uint8, device="cuda")
+    want = x.view(a, B, b * e).transpose(0, 1).reshape(-1)
+    for _ in range(2):
+        y = x.clone()
+        assert lm.lib().lm_debug_wave_stall(None, y.data_ptr(), e, a, B, b,
+                                            20_000_000) is True
+        assert "timed out" in lm.last_error()
+    assert lm.lib().lm_device_status(None) == 0
+    lm.transpose_100(x, a, B, b, elem_bytes=e)
+    torch.cuda.synchronize()
+    assert torch.equal(x, want)
+    assert lm.lib().lm_device_status(None) == 0
