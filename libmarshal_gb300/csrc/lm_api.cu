@@ -245,10 +245,9 @@ struct PadBlock {
   int dev = 0;
   bool kept = false;  // from the pool
   bool done = false;  // the kernel has finished without a failure
-  uint64_t tasks = 0;
+  uint64_t started = 0;  // tasks of the kernel, which take a ticket each
   // false: no memory
   bool take(uint64_t n, cudaStream_t s) {
-    tasks = n;
     cudaGetDevice(&dev);
     kept = n + 2 <= kWords;
     if (kept) {
@@ -273,7 +272,7 @@ struct PadBlock {
     if (!kept || !f.p) return;
     std::lock_guard<std::mutex> lock(mu());
     if (done && pool(dev).size() < kKept && f.epoch != 0xffffffffu)
-      pool(dev).push_back({f.p, f.ticket + (uint32_t)tasks, f.epoch});
+      pool(dev).push_back({f.p, f.ticket + (uint32_t)started, f.epoch});
     else
       cudaFreeAsync(f.p, own.s);  // (the call has waited for its stream)
   }
@@ -862,17 +861,18 @@ static bool do_pad(cudaStream_t s, void *buf, int e, int64_t x, int64_t y,
   if ((y == 0 || pad == x) && stall_block < 0) return false;
   if (buf == nullptr) return fail("null buffer");
   if (misaligned(buf, e)) return fail("buffer must be aligned to the element size");
-  PadBlock block;
   const uint64_t tasks = pad_tasks(buf, e, y, pad);
+  if (tasks == 0) return false;  // an empty layout, with a stall asked for
+  PadBlock block;
   if ((tasks > 1 || stall_block >= 0) && !block.take(tasks, s)) return true;
   // (a word of host memory, so that no copy follows the kernel)
   HostWord st;
   if (!st.p) return fail("padding: no status word");
   cudaError_t err =
       padding ? launch_padding(s, buf, e, x, y, pad, block.f, st.p,
-                               timeout_ns, stall_block)
+                               timeout_ns, stall_block, &block.started)
               : launch_unpadding(s, buf, e, x, y, pad, block.f, st.p,
-                                 timeout_ns, stall_block);
+                                 timeout_ns, stall_block, &block.started);
   if (err != cudaSuccess) return cuda_fail(err, padding ? "padding" : "unpadding");
   err = cudaStreamSynchronize(s);
   if (err != cudaSuccess) {

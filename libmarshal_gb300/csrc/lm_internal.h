@@ -289,7 +289,8 @@ uint32_t *device_status_word();
 // which waits for nothing.  `status`: one zeroed word of pinned host memory
 // that the kernel sets to kStatusWaitTimeout when a wait runs out.
 // stall_block >= 0 makes that task wait on the last word (failure-detection
-// test hook; it needs flags).
+// test hook; it needs flags).  *started: the tasks that the launch started,
+// by which the ticket word counts up; as it was where none ran.
 struct PadFlags {
   uint32_t *p = nullptr;
   uint64_t words = 0;
@@ -299,10 +300,10 @@ uint64_t pad_tasks(const void *buf, int e, uint64_t y, uint64_t pad);
 cudaError_t launch_padding(cudaStream_t s, void *buf, int e, uint64_t x,
                            uint64_t y, uint64_t pad, const PadFlags &flags,
                            uint32_t *status, uint64_t timeout_ns,
-                           int64_t stall_block);
+                           int64_t stall_block, uint64_t *started);
 cudaError_t launch_unpadding(cudaStream_t s, void *buf, int e, uint64_t x,
                              uint64_t y, uint64_t pad, const PadFlags &flags,
                              uint32_t *status, uint64_t timeout_ns,
-                             int64_t stall_block);
+                             int64_t stall_block, uint64_t *started);
 
 }  // namespace lm

@@ -333,6 +333,7 @@ static uint32_t pad_task_bytes(uint64_t bytes) {
 
 uint64_t pad_tasks(const void *buf, int e, uint64_t y, uint64_t pad) {
   const uint64_t O = y * pad * e, task = pad_task_bytes(O);
+  if (O == 0) return 0;
   return (O + ((uintptr_t)buf & 15) + task - 1) / task;
 }
 
@@ -340,7 +341,7 @@ template <bool PAD>
 static cudaError_t run_pad(cudaStream_t s, void *buf, int e, uint64_t x,
                            uint64_t y, uint64_t pad, const PadFlags &flags,
                            uint32_t *status, uint64_t timeout_ns,
-                           int64_t stall_block) {
+                           int64_t stall_block, uint64_t *started) {
   if (pad < x) return cudaErrorInvalidValue;
   PadArgs g;
   g.buf = reinterpret_cast<char *>(buf);
@@ -379,23 +380,25 @@ static cudaError_t run_pad(cudaStream_t s, void *buf, int e, uint64_t x,
     case 8: k_pad<8, PAD><<<grid, kPadThreads, smem, s>>>(g); break;
     default: return cudaErrorInvalidValue;
   }
-  return cudaGetLastError();
+  const cudaError_t err = cudaGetLastError();
+  if (err == cudaSuccess) *started = g.ntasks;
+  return err;
 }
 
 cudaError_t launch_padding(cudaStream_t s, void *buf, int e, uint64_t x,
                            uint64_t y, uint64_t pad, const PadFlags &flags,
                            uint32_t *status, uint64_t timeout_ns,
-                           int64_t stall_block) {
+                           int64_t stall_block, uint64_t *started) {
   return run_pad<true>(s, buf, e, x, y, pad, flags, status, timeout_ns,
-                       stall_block);
+                       stall_block, started);
 }
 
 cudaError_t launch_unpadding(cudaStream_t s, void *buf, int e, uint64_t x,
                              uint64_t y, uint64_t pad, const PadFlags &flags,
                              uint32_t *status, uint64_t timeout_ns,
-                             int64_t stall_block) {
+                             int64_t stall_block, uint64_t *started) {
   return run_pad<false>(s, buf, e, x, y, pad, flags, status, timeout_ns,
-                        stall_block);
+                        stall_block, started);
 }
 
 }  // namespace lm

@@ -65,3 +65,17 @@ def test_rows_about_a_vector(e, row):
     for x in sorted({1, 7, row // 2, row - 1}):
         _check(e, x, 700, row)
         _check(e, x, 700, row, offset=16 - e)
+
+
+@pytest.mark.parametrize("off", [0, 4, 12])
+def test_calls_after_an_empty_one(off):
+    """A call that starts no kernel books no tickets on the flags that are kept
+    between calls."""
+    raw = torch.zeros(4096, dtype=torch.uint8, device="cuda")
+    for unpad in (0, 1):
+        _check(4, 1000, 600, 1010, off)
+        for x, y, pad in ((3, 0, 5), (0, 7, 0)):
+            assert lm.lib().lm_debug_pad_stall(None, raw.data_ptr() + off, 4, x,
+                                               y, pad, unpad, 0,
+                                               1_000_000) is False
+        _check(4, 1000, 600, 1010, off)

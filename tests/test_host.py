@@ -146,3 +146,26 @@ int main(void) {
     out = subprocess.run([str(exe)], capture_output=True, text=True)
     assert out.returncode == 0, out.stdout + out.stderr
     assert "aligned" in out.stdout
+
+
+@pytest.mark.parametrize("unpad", [0, 1])
+@pytest.mark.parametrize("x,y,pad", [(3, 0, 5), (5, 0, 5), (0, 7, 0)])
+def test_empty_padding_takes_no_flags(built, unpad, x, y, pad):
+    """An empty layout starts no kernel, whatever stall is asked for, so it
+    needs no flag block and does not come to one: without a device (and on a
+    buffer at any place in 16 bytes) it succeeds.  Run in a process that sees
+    none, as elsewhere the flags could be had."""
+    import subprocess
+    import sys
+    code = ("from libmarshal_gb300 import lm\n"
+            "L = lm.lib()\n"
+            "for p in (0x1000, 0x1004, 0x100c):\n"
+            "    assert L.lm_debug_pad_stall(None, p, 4, %d, %d, %d, %d, 0,\n"
+            "                                1000) is False, lm.last_error()\n"
+            "assert L.lm_debug_pad_stall(None, None, 4, %d, %d, %d, %d, 0,\n"
+            "                            1000) is True\n"
+            % ((x, y, pad, unpad) * 2))
+    env = dict(os.environ, CUDA_VISIBLE_DEVICES="")
+    r = subprocess.run([sys.executable, "-c", code], cwd=ROOT, env=env,
+                       capture_output=True, text=True)
+    assert r.returncode == 0, r.stderr
