@@ -2411,8 +2411,7 @@ static bool launch_band(cudaStream_t s, const BJob *d_jobs,
                         uint32_t *counter, size_t smem, int C) {
   if (nitems == 0) return false;
   const size_t dyn = 2 * smem;  // two stages
-  cudaError_t err = cudaFuncSetAttribute(
-      k_batch_band, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn);
+  cudaError_t err = grow_smem_limit((const void *)k_batch_band, dyn);
   if (err == cudaSuccess && C > 8)
     err = cudaFuncSetAttribute(k_batch_band,
                                cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
@@ -2453,9 +2452,6 @@ static bool launch_band(cudaStream_t s, const BJob *d_jobs,
   return false;
 }
 
-// (one for both launchers: a kernel's shared-memory limit only grows)
-static LaunchCache g_gather3_cache;
-
 static bool launch_staged(cudaStream_t s, const BJob *d_jobs,
                           const BItem *d_items, uint32_t nitems,
                           uint32_t *counter, size_t smem, bool copyback,
@@ -2468,12 +2464,12 @@ static bool launch_staged(cudaStream_t s, const BJob *d_jobs,
                        : k_batch_gather<3, 0, 0>;
   // the gather keeps two stages of `smem` bytes
   const size_t dyn = copyback ? 0 : 2 * smem;
-  static LaunchCache copy_cache, ragged_cache;
+  static LaunchCache copy_cache, plain_cache, ragged_cache;
   cudaError_t err = cudaSuccess;
   const int occ = prepare_launch((const void *)kern,
                                  copyback ? copy_cache
                                  : ragged ? ragged_cache
-                                          : g_gather3_cache,
+                                          : plain_cache,
                                  dyn,
                                  kStageThreads, &err);
   if (err != cudaSuccess || occ < 1) return set_error("batch: occupancy");
@@ -3466,8 +3462,7 @@ static bool launch_small(cudaStream_t s, const BJob *d_jobs,
   constexpr size_t kFlat = (kSmallItem + 32 + 127) / 128 * 128;
   const size_t smem = kFlat + kSmallItem + 256;
   const DeviceInfo &di = device_info();
-  cudaError_t err = cudaFuncSetAttribute(
-      k_batch_small, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  cudaError_t err = grow_smem_limit((const void *)k_batch_small, smem);
   if (err != cudaSuccess) return set_error("batch: smem attribute");
   int occ = 0;
   err = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_batch_small,
@@ -3520,8 +3515,7 @@ static bool launch_items(cudaStream_t s, const BJob *d_jobs,
                          uint32_t *counter, size_t smem) {
   if (nitems == 0) return false;
   const DeviceInfo &di = device_info();
-  cudaError_t err = cudaFuncSetAttribute(
-      k_batch_bs, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  cudaError_t err = grow_smem_limit((const void *)k_batch_bs, smem);
   if (err != cudaSuccess) return set_error("batch: smem attribute");
   int occ = 0;
   err = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_batch_bs,

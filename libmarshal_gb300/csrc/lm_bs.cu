@@ -340,8 +340,7 @@ static cudaError_t run_bs(cudaStream_t s, const BsArgs &g, const BsPlan &p) {
     kern<<<(unsigned)blocks, kBsThreads, p.smem_bytes, s>>>(g);
     return cudaGetLastError();
   }
-  err = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)p.smem_bytes);
+  err = grow_smem_limit((const void *)kern, p.smem_bytes);
   if (err != cudaSuccess) return err;
   if (p.cluster > 8) {
     err = cudaFuncSetAttribute(kern,

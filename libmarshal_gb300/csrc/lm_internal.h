@@ -65,10 +65,14 @@ cudaError_t launch_bs0100(cudaStream_t s, void *buf, int e, uint64_t T,
 // for the last size asked: small conversions are bound by host time per
 // call, and these driver queries cost about as much as the launch itself.
 struct LaunchCache {
-  std::atomic<int> smem_set[8];       // per device: largest limit set (+1)
+  std::atomic<int> smem_set[8];       // per device: largest size seen to (+1)
   std::atomic<uint64_t> occ_key[8];   // per device: (smem << 16) | occupancy
 };
-// Sets the attribute if needed and returns the CTAs per SM for `threads`
+// Raises the limit of `kern` on the current device to `smem` bytes if it is
+// lower.  Every kernel launched with different sizes has its limit set here
+// alone, so that no thread lowers it under another's launch.
+cudaError_t grow_smem_limit(const void *kern, size_t smem);
+// Raises the limit if needed and returns the CTAs per SM for `threads`
 // threads and `smem` dynamic bytes (0 on error, with *err set).
 int prepare_launch(const void *kern, LaunchCache &c, size_t smem, int threads,
                    cudaError_t *err);

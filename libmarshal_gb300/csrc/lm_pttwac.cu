@@ -408,11 +408,8 @@ cudaError_t launch_pttwac010_smem(cudaStream_t s, void *buf, int e,
   const DeviceInfo &di = device_info();
   cudaError_t err = cudaSuccess;
   auto go = [&](auto kern) {
-    if (smem > 48 * 1024) {
-      err = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)smem);
-      if (err != cudaSuccess) return;
-    }
+    err = grow_smem_limit((const void *)kern, smem);
+    if (err != cudaSuccess) return;
     int occ = 0;
     err = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, 1024, smem);
     if (err != cudaSuccess) return;

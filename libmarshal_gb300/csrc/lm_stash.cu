@@ -565,9 +565,7 @@ static uint32_t stash_pitch(uint64_t row_bytes, int e) {
 template <int E>
 static int wave_occupancy(size_t smem) {
   auto kern = k_stash_wave<E>;
-  if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           (int)smem) != cudaSuccess)
-    return 0;
+  if (grow_smem_limit((const void *)kern, smem) != cudaSuccess) return 0;
   int occ = 0;
   if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, kWaveThreads,
                                                     smem) != cudaSuccess)
@@ -839,8 +837,7 @@ static cudaError_t run_stash(cudaStream_t s, StashArgs g, const StashPlan &p) {
     if ((err = cudaGetLastError()) != cudaSuccess) return err;
   }
   auto kern = k_stash_wave<E>;
-  err = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)p.smem_bytes);
+  err = grow_smem_limit((const void *)kern, p.smem_bytes);
   if (err != cudaSuccess) return err;
   int occ = 0;
   err = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, kWaveThreads,
