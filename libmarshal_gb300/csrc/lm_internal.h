@@ -65,8 +65,8 @@ cudaError_t launch_bs0100(cudaStream_t s, void *buf, int e, uint64_t T,
 // for the last size asked: small conversions are bound by host time per
 // call, and these driver queries cost about as much as the launch itself.
 struct LaunchCache {
-  std::atomic<int> smem_set[8];       // per device: largest size seen to (+1)
-  std::atomic<uint64_t> occ_key[8];   // per device: (smem << 16) | occupancy
+  std::atomic<int> smem_set[64];      // per device: largest size seen to (+1)
+  std::atomic<uint64_t> occ_key[64];  // per device: (smem << 16) | occupancy
 };
 // Raises the limit of `kern` on the current device to `smem` bytes if it is
 // lower.  Every kernel launched with different sizes has its limit set here

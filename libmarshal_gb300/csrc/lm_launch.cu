@@ -32,7 +32,7 @@ int prepare_launch(const void *kern, LaunchCache &c, size_t smem, int threads,
   *err = cudaSuccess;
   int dev = 0;
   cudaGetDevice(&dev);
-  const int d = dev & 7;
+  const int d = dev & 63;
   const int need = (int)smem + 1;
   if (c.smem_set[d].load(std::memory_order_acquire) < need) {
     if ((*err = grow_smem_limit(kern, smem)) != cudaSuccess) return 0;

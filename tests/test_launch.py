@@ -109,3 +109,14 @@ def test_limit_only_grows(tmp_path):
   static char k;
   for (int kb : {1, 60, 100, 50, 100, 227, 60}) launch(&k, c, kb << 10);
   if (g_sets != 3) return printf("%d calls of the driver\n", (int)g_sets), 1;""")
+
+
+def test_devices_have_their_own(tmp_path):
+    """Devices past the eighth do not pass for one of the first eight."""
+    _run(tmp_path, r"""
+  static lm::LaunchCache c;
+  static char k;
+  for (int dev : {0, 8, 15, 7, 63}) {
+    t_dev = dev;
+    launch(&k, c, 100 << 10);
+  }""")
