@@ -141,9 +141,13 @@ def _current_stream() -> int:
     if _torch is None:
         import torch
         _torch = torch
-    if not _torch.cuda.is_initialized():
-        return _torch.cuda.current_stream().cuda_stream
-    return _torch._C._cuda_getCurrentRawStream(_torch._C._cuda_getDevice())
+    if _torch.cuda.is_initialized():
+        try:
+            return _torch._C._cuda_getCurrentRawStream(
+                _torch._C._cuda_getDevice())
+        except AttributeError:  # a torch without these private names
+            pass
+    return _torch.cuda.current_stream().cuda_stream
 
 
 def stream_ptr(stream=None) -> int:

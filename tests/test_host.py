@@ -169,3 +169,22 @@ def test_empty_padding_takes_no_flags(built, unpad, x, y, pad):
     r = subprocess.run([sys.executable, "-c", code], cwd=ROOT, env=env,
                        capture_output=True, text=True)
     assert r.returncode == 0, r.stderr
+
+
+@pytest.mark.parametrize("missing", ["_cuda_getCurrentRawStream",
+                                     "_cuda_getDevice", "neither"])
+def test_current_stream_without_the_raw_getter(monkeypatch, missing):
+    """The stream of the calls comes from torch's raw getters where torch has
+    them, and else from its stream object."""
+    import types
+    from libmarshal_gb300 import lm
+    c = types.SimpleNamespace(_cuda_getCurrentRawStream=lambda d: 100 + d,
+                              _cuda_getDevice=lambda: 3)
+    if missing != "neither":
+        delattr(c, missing)
+    cuda = types.SimpleNamespace(
+        is_initialized=lambda: True,
+        current_stream=lambda: types.SimpleNamespace(cuda_stream=7))
+    monkeypatch.setattr(lm, "_torch", types.SimpleNamespace(_C=c, cuda=cuda))
+    assert lm.stream_ptr() == (103 if missing == "neither" else 7)
+    assert lm.stream_ptr(5) == 5
