@@ -181,11 +181,16 @@ cudaError_t launch_move(cudaStream_t s, char *base, uint64_t T,
 
 // Cycle leaders depend only on (a, B) and which cycles they stand for (kind:
 // 0 for all of them, k > 0 for those that hold no start of lm_walk.cu's
-// blocks of 2^k positions): lists computed outside stream capture are kept per device (the first kCacheEntries shapes, kCacheBytes in all,
-// until lm_marshal_finalize) and reused; a later call on another stream
-// waits for the producing kernel.
-constexpr int kCacheEntries = 16;
-constexpr size_t kCacheBytes = 512ull << 20;
+// blocks of 2^k positions): lists computed outside stream capture are kept
+// per device until lm_marshal_finalize and reused; a later call on another
+// stream waits for the producing kernel.  The lists of all cycles and those
+// of the walks have room of their own each (the first shapes, and so many
+// bytes), so that neither takes the other's.
+struct CycRoom {
+  int entries;
+  size_t bytes;
+};
+constexpr CycRoom kCycRoom[2] = {{16, 512ull << 20}, {64, 256ull << 20}};
 struct CycEntry {
   void *mem = nullptr;  // count word + list
   size_t bytes = 0;
@@ -258,10 +263,15 @@ cudaError_t cycle_list_for(
   const size_t bytes = cycle_scratch_bytes(a, B);
   // a full cache admits nothing more (no eviction: freeing device memory
   // would synchronise the device); other shapes use per-call memory
+  const CycRoom &room = kCycRoom[kind ? 1 : 0];
   size_t total = bytes;
-  for (auto &kv : g_cyc) total += kv.second.bytes;
-  if ((int)g_cyc.size() >= kCacheEntries || total > kCacheBytes)
-    return into_scratch();
+  int kept = 0;
+  for (auto &kv : g_cyc)
+    if (std::get<0>(kv.first) == dev && !std::get<3>(kv.first) == !kind) {
+      total += kv.second.bytes;
+      ++kept;
+    }
+  if (kept >= room.entries || total > room.bytes) return into_scratch();
   CycEntry en;
   en.bytes = bytes;
   // stream-ordered: a plain cudaMalloc may synchronise the device

@@ -96,3 +96,26 @@ def test_walk_concurrent_streams():
     torch.cuda.synchronize()
     for b, w in zip(bufs, want):
         assert torch.equal(b, w)
+
+
+def test_walks_leave_room_for_the_lists_of_cycles(monkeypatch):
+    """Shapes that are walked in segments do not take the room of the lists of
+    whole cycles: after many of them a new shape's list is still kept."""
+    monkeypatch.setenv("LM_NO_RESIDENT", "1")
+    lm.lib().lm_marshal_finalize()
+    for B in range(5501, 5521):  # 17 MB of 128-byte units each
+        x = torch.zeros(24 * B * 32, dtype=torch.int32, device="cuda")
+        lm.transpose_100(x, 24, B, 32)
+    x = torch.arange(12 * 12 * 65536, dtype=torch.int32, device="cuda")
+    want = x.view(12, 12, 65536).transpose(0, 1).reshape(-1)
+    ran = []
+    for _ in range(3):
+        lm.prof_collect()
+        lm.prof_enable(True)
+        lm.transpose_100(x, 12, 12, 65536)
+        torch.cuda.synchronize()
+        lm.prof_enable(False)
+        ran.append(set(lm.prof_collect()))
+    assert ran == [{"cycle_leaders", "cycle_move"}, {"cycle_move"},
+                   {"cycle_move"}]
+    assert torch.equal(x, want)
