@@ -115,6 +115,14 @@ static bool try_scratch(Scratch &sc, size_t bytes, cudaStream_t s) {
   return true;
 }
 
+// Memory for a list of cycles that is not kept, asked for where there is
+// such a list alone.
+static auto list_scratch(Scratch &sc, cudaStream_t s) {
+  return [&sc, s](size_t bytes) -> void * {
+    return try_scratch(sc, bytes, s) ? sc.p : nullptr;
+  };
+}
+
 static bool get_scratch(Scratch &sc, size_t bytes, cudaStream_t s) {
   pool_keep_memory();
   sc.s = s;
@@ -522,11 +530,10 @@ static bool do_0100(cudaStream_t s, void *buf, int e, uint64_t T, uint64_t a,
       // (where the list is computed into per-call scratch)
       cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
       cudaStreamIsCapturing(s, &cs);
-      Scratch sc;
-      if (get_scratch(sc, cycle_scratch_bytes(a, B), s)) return true;
+      Scratch list;
       return check_launch(
           launch_cycles100(s, buf, e, T, (uint32_t)a, (uint32_t)B,
-                           (uint32_t)b, L, sc.p,
+                           (uint32_t)b, L, list_scratch(list, s),
                            cs == cudaStreamCaptureStatusNone),
           "cycles launch");
     }
@@ -560,12 +567,12 @@ static bool do_0100(cudaStream_t s, void *buf, int e, uint64_t T, uint64_t a,
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
     cudaStreamIsCapturing(s, &cs);
     Scratch sc, list;
-    if (try_scratch(sc, walk_scratch_bytes(buf, T, a, B, U), s) &&
-        try_scratch(list, cycle_scratch_bytes(a, B), s))
-      return check_launch(
-          launch_walk100(s, buf, T, a, B, U, sc.p, list.p,
-                         cs == cudaStreamCaptureStatusNone),
-          "walk launch");
+    if (try_scratch(sc, walk_scratch_bytes(buf, T, a, B, U), s)) {
+      const cudaError_t err =
+          launch_walk100(s, buf, T, a, B, U, sc.p, list_scratch(list, s),
+                         cs == cudaStreamCaptureStatusNone);
+      if (err != cudaErrorMemoryAllocation) return check_launch(err, "walk launch");
+    }
   }
   const bool stash_first =
       m == Method::Auto && stash_preferred(buf, T, a, B, b, e);

@@ -237,8 +237,8 @@ static cudaError_t run_leaders(cudaStream_t s, uint32_t a, const ModM &m,
 
 // See lm_internal.h.
 cudaError_t cycle_list_for(
-    cudaStream_t s, uint64_t a, uint64_t B, uint32_t kind, void *scratch,
-    bool may_cache, void **mem,
+    cudaStream_t s, uint64_t a, uint64_t B, uint32_t kind,
+    const std::function<void *(size_t)> &scratch, bool may_cache, void **mem,
     const std::function<cudaError_t(uint32_t *, uint32_t *)> &find) {
   auto find_into = [&](void *p) {
     uint32_t *count = reinterpret_cast<uint32_t *>(p);
@@ -247,8 +247,8 @@ cudaError_t cycle_list_for(
     return find(reinterpret_cast<uint32_t *>((char *)p + 256), count);
   };
   auto into_scratch = [&]() {
-    *mem = scratch;
-    return find_into(scratch);
+    *mem = scratch(cycle_scratch_bytes(a, B));
+    return *mem ? find_into(*mem) : cudaErrorMemoryAllocation;
   };
   if (!may_cache) return into_scratch();
   int dev = 0;
@@ -315,7 +315,8 @@ void cycle_cache_clear() {
 
 cudaError_t launch_cycles100(cudaStream_t s, void *buf, int e, uint64_t T,
                              uint32_t a, uint32_t B, uint32_t b, uint32_t L,
-                             void *scratch, bool may_cache) {
+                             const std::function<void *(size_t)> &scratch,
+                             bool may_cache) {
   const uint64_t M = (uint64_t)a * B - 1;
   if (L == 0 || L > kCycleMaxLen || M >= (1ull << 32))
     return cudaErrorInvalidValue;

@@ -181,32 +181,33 @@ void cycle_cache_clear();
 // byte 256 on.  It comes from the per-device cache (with may_cache, never
 // while the stream is being captured), or `find` enqueues the kernels that
 // fill it (the count is zero before them), into a new cache entry or, when
-// there is no room, into `scratch` (cycle_scratch_bytes(a, B) bytes).
+// there is no room, into what `scratch` gives for its bytes (nullptr: the
+// call returns cudaErrorMemoryAllocation and has enqueued nothing).
 cudaError_t cycle_list_for(
-    cudaStream_t s, uint64_t a, uint64_t B, uint32_t kind, void *scratch,
-    bool may_cache, void **mem,
+    cudaStream_t s, uint64_t a, uint64_t B, uint32_t kind,
+    const std::function<void *(size_t)> &scratch, bool may_cache, void **mem,
     const std::function<cudaError_t(uint32_t *, uint32_t *)> &find);
 // T instances of 100(a, B, b) whose cycles have at most L <= kCycleMaxLen
-// units.  `scratch` holds cycle_scratch_bytes(a, B) bytes; with may_cache
-// (never while the stream is being captured) the cycle leaders come from a
-// per-device cache of shapes, else they are computed into the scratch.
+// units; `scratch` and `may_cache` as above.
 cudaError_t launch_cycles100(cudaStream_t s, void *buf, int e, uint64_t T,
                              uint32_t a, uint32_t B, uint32_t b, uint32_t L,
-                             void *scratch, bool may_cache);
+                             const std::function<void *(size_t)> &scratch,
+                             bool may_cache);
 
 // ---- segments of cycles (lm_walk.cu) -----------------------------------------
 // T instances of 100(a, B) on units of U bytes (whole 16-byte vectors in a
 // 16-byte aligned buffer, 128 bytes or 192 and more) at 2 x payload:
-// walk_scratch_bytes bytes of `scratch` (about payload / 8), and
-// cycle_scratch_bytes(a, B) of `list_scratch` for a shape whose list of
-// cycles is not cached.
+// walk_scratch_bytes bytes of `scratch` (about payload / 8), and memory from
+// `list_scratch` for a shape whose list of cycles is not kept
+// (cudaErrorMemoryAllocation, the buffer as it was, where there is none).
 bool walk_applies(const void *buf, uint64_t T, uint64_t a, uint64_t B,
                   uint64_t U);
 size_t walk_scratch_bytes(const void *buf, uint64_t T, uint64_t a, uint64_t B,
                           uint64_t U);
 cudaError_t launch_walk100(cudaStream_t s, void *buf, uint64_t T, uint64_t a,
                            uint64_t B, uint64_t U, void *scratch,
-                           void *list_scratch, bool may_cache);
+                           const std::function<void *(size_t)> &list_scratch,
+                           bool may_cache);
 
 // ---- 0100 through scratch (lm_batch.cu) -------------------------------------
 // The blocks of every tile transposed through shared memory into `scratch`

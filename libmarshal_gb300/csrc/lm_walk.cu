@@ -320,7 +320,8 @@ size_t walk_scratch_bytes(const void *buf, uint64_t T, uint64_t a, uint64_t B,
 
 cudaError_t launch_walk100(cudaStream_t s, void *buf, uint64_t T, uint64_t a,
                            uint64_t B, uint64_t U, void *scratch,
-                           void *list_scratch, bool may_cache) {
+                           const std::function<void *(size_t)> &list_scratch,
+                           bool may_cache) {
   WalkArgs g;
   if (!walk_args(buf, T, a, B, U, &g)) return cudaErrorInvalidValue;
   g.base = reinterpret_cast<char *>(buf);

@@ -119,3 +119,30 @@ def test_walks_leave_room_for_the_lists_of_cycles(monkeypatch):
     assert ran == [{"cycle_leaders", "cycle_move"}, {"cycle_move"},
                    {"cycle_move"}]
     assert torch.equal(x, want)
+
+
+def test_a_kept_list_takes_no_scratch():
+    """A call on a shape whose list of cycles is kept allocates its walk's
+    scratch, an eighth of the payload, and no memory for the list."""
+    import ctypes
+    cu = ctypes.CDLL("libcuda.so.1")
+    pool, v = ctypes.c_void_p(), ctypes.c_uint64()
+    torch.zeros(1, device="cuda")
+    assert cu.cuDeviceGetDefaultMemPool(ctypes.byref(pool), 0) == 0
+
+    def used(attr):  # 7: used now, 8: most since the last reset
+        assert cu.cuMemPoolGetAttribute(pool, attr, ctypes.byref(v)) == 0
+        return v.value
+
+    a, B, words = 25, 30011, 32  # 96 MB of 128-byte units
+    x = torch.zeros(a * B * words, dtype=torch.int32, device="cuda")
+    for _ in range(2):
+        lm.transpose_100(x, a, B, words)
+    torch.cuda.synchronize()
+    before = used(7)
+    zero = ctypes.c_uint64(0)
+    assert cu.cuMemPoolSetAttribute(pool, 8, ctypes.byref(zero)) == 0
+    lm.transpose_100(x, a, B, words)
+    torch.cuda.synchronize()
+    walk = x.numel() * 4 // 8 + 2048
+    assert used(8) - before < walk + (1 << 19)  # (the list: 1.5 MB)
