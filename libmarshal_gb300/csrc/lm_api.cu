@@ -326,6 +326,7 @@ static uint64_t wait_timeout_ns() {
 // ---- planner ----------------------------------------------------------------
 
 constexpr uint64_t kWalkMinBytes = 16ull << 20;
+constexpr uint64_t kWalkUnkeptBytes = 80ull << 20;
 
 // Whether the ordered form (3 x payload, k_wave) is faster than the staged one
 // (4 x, but no waits, and a copy back out of L2 up to 208 MB): its slack is
@@ -352,6 +353,38 @@ static bool wave_preferred(const void *buf, uint64_t T, uint64_t a, uint64_t B,
   if (U >= 4 && row < 64) return false;
   if (T > 1) least = std::max<uint64_t>(least, 128ull << 20);
   return bytes >= least;
+}
+
+// Whether a walk is the faster form for units that it takes: against the
+// ordered form by the lines that it reads, beyond L2 (walk_by_lines; 128 MB: 66
+// and 79 us at 140 MB for 128-byte units on lines, 57 and 57 at 100 and 87 and
+// 78 at 140 off them); against the staged form always where the list of its
+// cycles is kept (60 MB of 128-byte units 27 and 33, of 320-byte ones 33 and
+// 35), and from 80 MB on where it is found on every call, as under stream
+// capture (34 MB 29 and 23, 60 MB 35 to 48 and 35, 84 MB 44 to 49 and 52).
+// Units of 1 KB and more have neither (34 MB 19 and 33 by done bits).
+static bool walk_preferred(const void *buf, uint64_t T, uint64_t a, uint64_t B,
+                           uint64_t U, bool may_keep, bool wave) {
+  const uint64_t bytes = T * a * B * U;
+  if (U >= kStagedMaxUnit) return true;
+  if (bytes < kWalkUnkeptBytes && !(may_keep && walk_list_kept(a, B)))
+    return false;
+  return bytes < (128ull << 20) || !wave || walk_by_lines(buf, U);
+}
+
+// Scratch of the ordered form for T instances one after another (the same plan
+// for every instance, but for its place in 16 bytes); 0 where it does not
+// take them.
+static size_t wave_scratch(void *buf, uint64_t T, uint64_t a, uint64_t B,
+                           uint64_t b, int e) {
+  const uint64_t step = a * B * b * e;
+  size_t need = 0;
+  for (uint64_t t = 0; t < T && t < 16; ++t) {
+    const size_t n = wave0100_scratch((char *)buf + t * step, a, B, b, e);
+    if (n == 0) return 0;
+    need = std::max(need, n);
+  }
+  return need;
 }
 
 // Half-words in tall matrices whose output rows are no whole vectors long: the
@@ -561,40 +594,37 @@ static bool do_0100(cudaStream_t s, void *buf, int e, uint64_t T, uint64_t a,
                   (unsigned long long)T, (unsigned long long)a,
                   (unsigned long long)B, (unsigned long long)b);
   }
-  // longer cycles of units of 64 bytes and more, cut into segments
+  const bool stash_first =
+      m == Method::Auto && stash_preferred(buf, T, a, B, b, e);
+  const size_t wave_need =
+      m == Method::Auto && U < kStagedMaxUnit && !stash_first &&
+              wave_preferred(buf, T, a, B, U) && !getenv("LM_NO_WAVE")
+          ? wave_scratch(buf, T, a, B, b, e)
+          : 0;
+  // longer cycles of units of 128 bytes and of 192 and more, cut into segments
   if (m == Method::Auto && T * a * B * U >= kWalkMinBytes &&
       !getenv("LM_NO_WALK") && walk_applies(buf, T, a, B, U)) {
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
     cudaStreamIsCapturing(s, &cs);
     Scratch sc, list;
-    if (try_scratch(sc, walk_scratch_bytes(buf, T, a, B, U), s)) {
+    if (walk_preferred(buf, T, a, B, U, cs == cudaStreamCaptureStatusNone,
+                       wave_need != 0) &&
+        try_scratch(sc, walk_scratch_bytes(buf, T, a, B, U), s)) {
       const cudaError_t err =
           launch_walk100(s, buf, T, a, B, U, sc.p, list_scratch(list, s),
                          cs == cudaStreamCaptureStatusNone);
       if (err != cudaErrorMemoryAllocation) return check_launch(err, "walk launch");
     }
   }
-  const bool stash_first =
-      m == Method::Auto && stash_preferred(buf, T, a, B, b, e);
   // a large matrix at 3 x payload: half of its blocks in place, the others
   // through scratch (lm_batch.cu, k_wave)
-  if (m == Method::Auto && U < kStagedMaxUnit && !stash_first &&
-      wave_preferred(buf, T, a, B, U) && !getenv("LM_NO_WAVE")) {
-    // (the same plan for every instance, but for its place in 16 bytes)
-    const uint64_t step = a * B * U;
-    size_t need = 0;
-    bool fits = true;
-    for (uint64_t t = 0; t < T && t < 16 && fits; ++t) {
-      const size_t n = wave0100_scratch((char *)buf + t * step, a, B, b, e);
-      fits = n != 0;
-      need = std::max(need, n);
-    }
-    uint32_t *status = fits ? device_status_word() : nullptr;
+  if (wave_need) {
+    uint32_t *status = device_status_word();
     Scratch sc;
-    if (fits && status && try_scratch(sc, need, s)) {
+    if (status && try_scratch(sc, wave_need, s)) {
       cudaError_t err = cudaSuccess;
       for (uint64_t t = 0; t < T && err == cudaSuccess; ++t)
-        err = launch_wave0100(s, (char *)buf + t * step, e, a, B, b, sc.p,
+        err = launch_wave0100(s, (char *)buf + t * a * B * U, e, a, B, b, sc.p,
                               status, wait_timeout_ns());
       return check_launch(err, "wave launch");
     }

@@ -235,6 +235,27 @@ static cudaError_t run_leaders(cudaStream_t s, uint32_t a, const ModM &m,
   return cudaGetLastError();
 }
 
+// Whether a new list of this kind has room (with the lock held).
+static bool cycle_room(int dev, uint64_t a, uint64_t B, uint32_t kind) {
+  const CycRoom &room = kCycRoom[kind ? 1 : 0];
+  size_t total = cycle_scratch_bytes(a, B);
+  int kept = 0;
+  for (auto &kv : g_cyc)
+    if (std::get<0>(kv.first) == dev && !std::get<3>(kv.first) == !kind) {
+      total += kv.second.bytes;
+      ++kept;
+    }
+  return kept < room.entries && total <= room.bytes;
+}
+
+bool cycle_list_kept(uint64_t a, uint64_t B, uint32_t kind) {
+  int dev = 0;
+  cudaGetDevice(&dev);
+  std::lock_guard<std::mutex> lock(g_cyc_mu);
+  return g_cyc.count(std::make_tuple(dev, a, B, kind)) != 0 ||
+         cycle_room(dev, a, B, kind);
+}
+
 // See lm_internal.h.
 cudaError_t cycle_list_for(
     cudaStream_t s, uint64_t a, uint64_t B, uint32_t kind,
@@ -263,15 +284,7 @@ cudaError_t cycle_list_for(
   const size_t bytes = cycle_scratch_bytes(a, B);
   // a full cache admits nothing more (no eviction: freeing device memory
   // would synchronise the device); other shapes use per-call memory
-  const CycRoom &room = kCycRoom[kind ? 1 : 0];
-  size_t total = bytes;
-  int kept = 0;
-  for (auto &kv : g_cyc)
-    if (std::get<0>(kv.first) == dev && !std::get<3>(kv.first) == !kind) {
-      total += kv.second.bytes;
-      ++kept;
-    }
-  if (kept >= room.entries || total > room.bytes) return into_scratch();
+  if (!cycle_room(dev, a, B, kind)) return into_scratch();
   CycEntry en;
   en.bytes = bytes;
   // stream-ordered: a plain cudaMalloc may synchronise the device

@@ -174,6 +174,9 @@ constexpr uint32_t kCycleMaxLen = 32;
 // 100(a, B) divides), or 0 when it exceeds `limit` or a*B - 1 >= 2^32.
 uint32_t cycle_order(uint64_t a, uint64_t B, uint32_t limit);
 size_t cycle_scratch_bytes(uint64_t a, uint64_t B);
+// Whether the list of 100(a, B) is kept, or would be by a call outside stream
+// capture.
+bool cycle_list_kept(uint64_t a, uint64_t B, uint32_t kind);
 // Frees the cached cycle-leader lists of the current device (waits for
 // their readers).
 void cycle_cache_clear();
@@ -204,6 +207,11 @@ bool walk_applies(const void *buf, uint64_t T, uint64_t a, uint64_t B,
                   uint64_t U);
 size_t walk_scratch_bytes(const void *buf, uint64_t T, uint64_t a, uint64_t B,
                           uint64_t U);
+// Whether the walk's lanes read whole lines enough to be faster than the
+// ordered form on a payload that is larger than L2.
+bool walk_by_lines(const void *buf, uint64_t U);
+// Whether the shape's list of cycles is kept, or would be (cycle_list_kept).
+bool walk_list_kept(uint64_t a, uint64_t B);
 cudaError_t launch_walk100(cudaStream_t s, void *buf, uint64_t T, uint64_t a,
                            uint64_t B, uint64_t U, void *scratch,
                            const std::function<void *(size_t)> &list_scratch,

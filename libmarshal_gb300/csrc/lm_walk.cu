@@ -318,6 +318,31 @@ size_t walk_scratch_bytes(const void *buf, uint64_t T, uint64_t a, uint64_t B,
   return (size_t)g.inst * g.m.nS * g.lanes * 16;
 }
 
+// A group of lanes reads its slice of a unit at a random place, so what it
+// costs is the lines that the slice touches and the sectors that it touches in
+// part, and what it hides is the bytes that a warp has in flight.  At 300 MB
+// (walk and ordered form, us): slices of 128 bytes on lines 125 and 155, 64 past
+// them 199 and 155; of 192, 146 and 160 on halves of lines, 169 and 161 on
+// sectors; of 256 off lines 155 and 154; of 320 (and 640, which are two of
+// them) 150 and 159 on sectors, 162 and 161 off them; of 352 off them 157 and
+// 160; 17 lanes (272 bytes, 528) 172 and 159.  Up to about 100 MB, in L2, the
+// walk is the faster one anyhow.
+bool walk_by_lines(const void *buf, uint64_t U) {
+  WalkArgs g;
+  if (!walk_args(buf, 1, 2, 2, U, &g)) return false;
+  const uint64_t slice = (uint64_t)g.lanes * 16;
+  const uint64_t at = (uint64_t)(uintptr_t)buf | U | (g.slices > 1 ? slice : 0);
+  const uint64_t least = at % 128 == 0  ? 128
+                         : at % 64 == 0 ? 192
+                         : at % 32 == 0 ? 320
+                                        : 352;
+  return slice >= least;
+}
+
+bool walk_list_kept(uint64_t a, uint64_t B) {
+  return cycle_list_kept(a, B, kWalkLogBlock);
+}
+
 cudaError_t launch_walk100(cudaStream_t s, void *buf, uint64_t T, uint64_t a,
                            uint64_t B, uint64_t U, void *scratch,
                            const std::function<void *(size_t)> &list_scratch,

@@ -146,3 +146,70 @@ def test_a_kept_list_takes_no_scratch():
     torch.cuda.synchronize()
     walk = x.numel() * 4 // 8 + 2048
     assert used(8) - before < walk + (1 << 19)  # (the list: 1.5 MB)
+
+
+def _ran(ptr, T, a, B, unit):
+    lm.prof_collect()
+    lm.prof_enable(True)
+    lm.transpose_0100(ptr, T, a, B, unit // 8, elem_bytes=8)
+    torch.cuda.synchronize()
+    lm.prof_enable(False)
+    return set(lm.prof_collect())
+
+
+WALK, WAVE = {"walk_save", "walk"}, {"suffix_copy", "wave"}
+
+
+# units on lines, halves of lines, sectors and off them; lanes that fill little
+# of a warp (17 of 32), slices of a unit; below the size of L2 and with many
+# tiles nothing but the alignment to 16 bytes counts
+@pytest.mark.parametrize("T,a,mb,unit,off,ran", [
+    (1, 24, 140, 128, 0, WALK), (1, 24, 140, 128, 64, WAVE),
+    (1, 24, 140, 128, 16, WAVE), (1, 24, 110, 128, 64, WALK),
+    (1, 24, 140, 192, 64, WALK), (1, 24, 140, 192, 32, WAVE),
+    (1, 24, 140, 208, 0, WAVE), (1, 24, 110, 208, 0, WALK),
+    (1, 24, 140, 272, 0, WAVE), (1, 24, 140, 320, 32, WALK),
+    (1, 24, 140, 320, 16, WAVE), (1, 24, 140, 352, 16, WALK),
+    (1, 24, 140, 528, 0, WAVE), (1, 24, 140, 640, 0, WALK),
+    (2, 100, 280, 128, 32, WAVE), (12, 24, 280, 128, 32, WALK),
+    (1, 24, 140, 1040, 48, WALK),
+])
+def test_walk_by_alignment(T, a, mb, unit, off, ran):
+    B = (mb << 20) // (T * a * unit)
+    n = T * a * B * unit
+    raw = torch.randint(0, 256, (n + 256,), dtype=torch.uint8, device="cuda")
+    before = raw.clone()
+    first = _ran(raw.data_ptr() + off, T, a, B, unit)
+    assert first - {"walk_leaders"} == ran
+    want = before[off:off + n].view(T, a, B, unit).transpose(1, 2).reshape(-1)
+    assert torch.equal(raw[off:off + n], want)
+    assert torch.equal(raw[:off], before[:off])
+    assert torch.equal(raw[off + n:], before[off + n:])
+
+
+def test_walk_whose_list_is_not_kept(monkeypatch):
+    """Under capture, and where no more lists are kept, each call finds its
+    cycles: worth it from 80 MB on alone."""
+    monkeypatch.setenv("LM_NO_RESIDENT", "1")
+    lm.lib().lm_marshal_finalize()
+    buf = torch.zeros(100 << 20, dtype=torch.uint8, device="cuda")
+    shapes = [B for B in range(5501, 5601) if _order(24, 24 * B - 1) > 32][:64]
+    for B in shapes:  # 17 MB each
+        assert _ran(buf.data_ptr(), 1, 24, B, 128) == WALK | {"walk_leaders"}
+    assert _ran(buf.data_ptr(), 1, 24, shapes[0], 128) == WALK
+    staged = _ran(buf.data_ptr(), 1, 24, 20011, 128)  # 61 MB
+    assert "staged_gather" in staged
+    assert _ran(buf.data_ptr(), 1, 24, 30011, 128) == WALK | {"walk_leaders"}
+    lm.lib().lm_marshal_finalize()
+    assert _ran(buf.data_ptr(), 1, 24, 20011, 128) == WALK | {"walk_leaders"}
+    lm.transpose_100(torch.zeros(1000 * 777, dtype=torch.int32, device="cuda"),
+                     1000, 777, 1)
+    for B in (20011, 30011):
+        x = torch.arange(24 * B * 32, dtype=torch.int32, device="cuda")
+        want = x.view(24, B, 32).transpose(0, 1).reshape(-1)
+        gr = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(gr):
+            lm.transpose_100(x, 24, B, 32)
+        gr.replay()
+        torch.cuda.synchronize()
+        assert torch.equal(x, want)
