@@ -387,19 +387,37 @@ static size_t wave_scratch(void *buf, uint64_t T, uint64_t a, uint64_t B,
   return need;
 }
 
-// Half-words in tall matrices whose output rows are no whole vectors long: the
-// ordered form stages 7 rows more than it writes of each block, and from some
-// 23000 rows on the stash plan's strips are the shorter ones.  Microseconds,
-// stash and ordered: 22001 x 10005 276 and 277, 24001 x 14003 393 and 412,
-// 28775 x 13530 443 and 476, 30001 x 20003 677 and 731, 36001 x 9005 363 and
-// 399; but rows of 2 bytes past whole vectors, 28775 x 7001 274 and 257, 33001 x
-// 15001 631 and 594.  (Bytes, 28775 x 27060: 657 and 514.)
+// The stash plan before the forms through scratch, where its wavefront has the
+// rows (kStashRowsPerSm).  Its writers go down a column of rows, the blocks of
+// the others write units of several elements one element at a time:
+//  * units of several bytes or half-words, at every size (us, stash and the
+//    better of staged and ordered, 60 / 130 / 400 MB): 15001 rows of 7-byte
+//    units 95 / 178 / 473 and 143 / 284 / 792; of 66-byte units 64 / 110 / 269
+//    and 85 / 176 / 493; 7400 rows of 9-byte units 120 / 237 / 672 and 141 / 284
+//    / 821;
+//  * units of several words from 128 MB on, where a step's strip holds 384 bytes
+//    of a row: 15001 rows of 12-byte units 60 / 102 / 235 and 57 / 115 / 309 (of
+//    8-byte elements never: 24-byte units 55 / 97 / 229 and 43 / 89 / 225);
+//  * half-words in tall matrices whose output rows are no whole vectors long:
+//    at 13529 columns level with the ordered form at 24000 rows, and faster above
+//    (28775 465 and 475, 31006 486 and 506, 38902 583 and 629).  With fewer
+//    columns it is the slower one, at 31001 rows by 4 % at 7003, 12 at 4005
+//    and 31 at 2005: none below 4000.  Rows 2 bytes past whole vectors take it
+//    13-20 % longer at every height, for no cause that could be shown; those of
+//    the seven other places do not differ.  (Bytes, 28775 x 27060: 657 and 514.)
 static bool stash_preferred(const void *buf, uint64_t T, uint64_t a, uint64_t B,
                             uint64_t b, int e) {
-  if (T != 1 || e != 2 || b != 1 || a < 23000 || B * 2 % 16 == 2) return false;
-  if (a * 2 % 16 == 0) return false;
-  return wave_preferred(buf, T, a, B, 2) && !getenv("LM_NO_STASH") &&
-         plan_stash(a, B, 1, 2).feasible;
+  const uint64_t bytes = a * B * b * e;
+  if (T != 1 || b * e >= 128 || a * B < (1ull << 20) ||
+      a < kStashRowsPerSm * (uint64_t)device_info().sms)
+    return false;
+  if (b == 1 ? e != 2 || a < 23000 || B < 4000 || B * 2 % 16 == 2 ||
+                   a * 2 % 16 == 0 || !wave_preferred(buf, T, a, B, 2)
+             : e > 4 || (e == 4 && bytes < (128ull << 20)))
+    return false;
+  if (getenv("LM_NO_STASH")) return false;
+  const StashPlan p = plan_stash(a, B, (uint32_t)b, e);
+  return p.feasible && (e != 4 || p.g * b * e >= 384);
 }
 
 // elements of one CTA's on-chip tile past which the form held in shared
