@@ -342,15 +342,27 @@ constexpr uint64_t kWalkUnkeptBytes = 80ull << 20;
 // 663.  Several instances run in the ordered form one after another, in the
 // staged one at once: 3 of 100 MB of floats 199 and 197, 3 of 168 MB 330 and
 // 300, 2 of 268 MB 351 and 282; 3 of 117 MB of bytes 279 and 291.
+// Units of several elements that are no whole vectors are written one element
+// at a time: blocks that take longer and of which fewer are in flight, so the
+// form pays later (20000 rows and 40, wave and staged: 12-byte units 130 MB 124
+// and 113, 110 and 114, 200 MB 167 and 175, 160 and 172; 66-byte ones 200 MB 273
+// and 270, 251 and 264, 300 MB 398 and 409, 370 and 402; 9-byte ones 130 MB 285
+// and 290, 278 and 292; 24-byte ones of doubles 110 MB 80 and 76, 72 and 73, 160
+// MB 107 and 109, 99 and 108).
 static bool wave_preferred(const void *buf, uint64_t T, uint64_t a, uint64_t B,
-                           uint64_t U) {
-  const uint64_t bytes = a * B * U, row = B * U;
+                           uint64_t b, int e) {
+  const uint64_t U = b * e, bytes = a * B * U, row = B * U;
   const bool vectors = ((uintptr_t)buf & 15) == 0 && a * U % 16 == 0;
   uint64_t least = (U < 4 ? (vectors ? 104ull : 144ull)
                           : (vectors ? 88ull : 112ull)) << 20;
   if (U < 4 && row <= 304) least = 208ull << 20;
   if (U >= 4 && row < 96) least = 192ull << 20;
   if (U >= 4 && row < 64) return false;
+  if (b > 1 && (U % 16 || ((uintptr_t)buf & 15)))
+    least = std::max<uint64_t>(least, (e == 1   ? 160ull
+                                       : e == 2 ? 256ull
+                                       : e == 4 ? 208ull
+                                                : 144ull) << 20);
   if (T > 1) least = std::max<uint64_t>(least, 128ull << 20);
   return bytes >= least;
 }
@@ -412,7 +424,7 @@ static bool stash_preferred(const void *buf, uint64_t T, uint64_t a, uint64_t B,
       a < kStashRowsPerSm * (uint64_t)device_info().sms)
     return false;
   if (b == 1 ? e != 2 || a < 23000 || B < 4000 || B * 2 % 16 == 2 ||
-                   a * 2 % 16 == 0 || !wave_preferred(buf, T, a, B, 2)
+                   a * 2 % 16 == 0 || !wave_preferred(buf, T, a, B, 1, 2)
              : e > 4 || (e == 4 && bytes < (128ull << 20)))
     return false;
   if (getenv("LM_NO_STASH")) return false;
@@ -616,7 +628,7 @@ static bool do_0100(cudaStream_t s, void *buf, int e, uint64_t T, uint64_t a,
       m == Method::Auto && stash_preferred(buf, T, a, B, b, e);
   const size_t wave_need =
       m == Method::Auto && U < kStagedMaxUnit && !stash_first &&
-              wave_preferred(buf, T, a, B, U) && !getenv("LM_NO_WAVE")
+              wave_preferred(buf, T, a, B, b, e) && !getenv("LM_NO_WAVE")
           ? wave_scratch(buf, T, a, B, b, e)
           : 0;
   // longer cycles of units of 128 bytes and of 192 and more, cut into segments

@@ -41,3 +41,16 @@ def _route(T, a, B, b, e, off=0):
 ])
 def test_stash(a, B, b, e, off, stash):
     assert (_route(1, a, B, b, e, off) - {"stash_offsets"} == STASH) == stash
+
+
+@pytest.mark.parametrize("a,mb,b,e,off,wave", [
+    (1000, 180, 3, 4, 0, False), (1000, 230, 3, 4, 0, True),
+    (1000, 230, 33, 2, 0, False), (1000, 270, 33, 2, 0, True),
+    (1000, 150, 9, 1, 0, False), (1000, 170, 9, 1, 0, True),
+    (1000, 130, 3, 8, 0, False), (1000, 160, 3, 8, 0, True),
+    (1000, 100, 2, 8, 0, True), (1000, 120, 2, 8, 8, False),  # whole vectors
+    (100, 270, 21, 2, 0, True), (97, 230, 11, 4, 4, True),    # even heights
+])
+def test_wave_of_units_of_elements(a, mb, b, e, off, wave):
+    B = (mb << 20) // (a * b * e)
+    assert (_route(1, a, B, b, e, off) == WAVE) == wave
