@@ -432,9 +432,80 @@ static bool stash_preferred(const void *buf, uint64_t T, uint64_t a, uint64_t B,
   return p.feasible && (e != 4 || p.g * b * e >= 384);
 }
 
-// elements of one CTA's on-chip tile past which the form held in shared
-// memory is the faster one
-constexpr uint64_t kTileElems = 16 * 1024;
+// Whether a conversion in on-chip tiles by `p` is slower than what takes it
+// otherwise, in nanoseconds fitted to 2500 shapes of 4 KB to 28 MB (the choice
+// costs 0.4 to 0.8 % on average over the faster of the two, and 20 % in one of
+// a hundred).  A CTA moves its elements one by one, at about 0.32 ns each and
+// half that where the bands of a cluster do, tile after tile where there are more
+// than fit (a GPC has room for one cluster of 16): 41 x 1598 bytes 25.0 us, held in the
+// shared memory of all SMs 12.2, 362 x 362 half-words in a cluster of four 18.8
+// and 11.9, 9 tiles of 327 x 38 units of 210 bytes 52 and 39.  The held form
+// takes 6 to 10 us, and
+//  * for units of one element 0.3 to 0.6 us per MB (22 tiles of 246 x 74 doubles
+//    10.3 and 8.3, 66 of 363 x 17 8.3 and 10.4), but 0.4 to 2.6 us per MB where a
+//    column is a vector or two or a part of one (62 tiles of 8 x 8266 floats 8.8
+//    and 17.0, 27 of 4 x 107368 half-words 24.6 and 51.0);
+//  * for units of several, which it writes one element at a time too, the time
+//    of an SM's share of them and of the tiles' rows: 2 tiles of 92 x 30 units of
+//    45 bytes 49.5 and 10.1, but 148 of 91 x 2 of 163 bytes 16.5 and 24.7, 35 of
+//    3 x 2405 of 86 bytes 23.2 and 33.4.
+// Units of 64 bytes and more whose cycles are short go to those instead: 9 us
+// where their list is kept, 14.5 where not (4 x 40 units of 1536 bytes 8.3 and
+// 15.2), and 0.5 per MB; where it is kept with half of the SMs idle from 512 KB
+// on in any case (21 tiles of 8 x 2 units of 6776 bytes 8.3 and 7.4).
+static bool held_preferred(const void *buf, uint64_t T, uint64_t a, uint64_t B,
+                           uint64_t b, int e, const BsPlan &p) {
+  const DeviceInfo &di = device_info();
+  const uint64_t sms = (uint64_t)di.sms, C = (uint64_t)p.cluster;
+  const uint64_t chunks = (T + p.tiles_per_chunk - 1) / p.tiles_per_chunk;
+  const uint64_t all = T * a * B * b, bytes = all * (uint64_t)e;
+  const uint64_t rows = T * a / sms;
+  const bool vectors = ((uintptr_t)buf & 15) == 0;
+  // elements of a CTA, for as many rounds as the tiles take
+  const uint64_t at_once =
+      C == 1   ? sms * std::max<uint64_t>(1, (uint64_t)di.max_smem_per_sm /
+                                                 (p.smem_bytes + 1024))
+      : C == 2 ? sms * 75 / 152
+      : C == 4 ? sms * 36 / 152
+      : C == 8 ? sms * 15 / 152
+               : sms * 7 / 152;
+  const uint64_t rounds = chunks / std::max<uint64_t>(1, at_once) +
+                          (chunks % std::max<uint64_t>(1, at_once) != 0);
+  const uint64_t elems =
+      rounds * a * b * (C == 1 ? B * p.tiles_per_chunk : p.rows_per_cta);
+  if (b == 1) {
+    const uint64_t out = a * e;  // bytes of an output row
+    const uint64_t tile =
+        C == 1   ? 3800 + elems * 32 / 100
+        : e == 8 ? 4400 + elems * 28 / 100
+                 : 5300 + elems * (e > 1 && vectors && out % 16 == 0 ? 10 : 18) / 100;
+    if ((out <= 16 || out == 32) && out % 4 == 0 &&
+        ((uintptr_t)buf & 3) == 0 && (a >= 4 || e == 8))
+      return tile > (e == 1   ? 20000 + bytes / 450
+                     : e == 2 ? 12500 + bytes / 550
+                     : e == 4 ? 7500 + bytes / 1000
+                              : 9400 + bytes / 2500);
+    return tile > (e == 1   ? 8300 + bytes / 1700
+                   : e == 2 ? 7500 + bytes / 2000
+                   : e == 4 ? 6700 + bytes / 3000 + rows * 3
+                            : 6500 + bytes / 3300 + rows * 3);
+  }
+  const uint64_t tile = C == 1  ? 3400 + elems * 36 / 100
+                        : e < 8 ? 6500 + elems * 18 / 100
+                                : 4800 + elems * 26 / 100;
+  if (b * e >= 64 && !getenv("LM_NO_CYCLES") && a * B - 1 <= (1ull << 28) &&
+      tile > 7000 && cycle_order(a, B, kCycleMaxLen)) {
+    const bool kept = cycle_list_kept(a, B, 0);
+    return tile > (kept ? 9000u : 14500u) + bytes / 2000 ||
+           (kept && bytes >= (512ull << 10) && chunks * C * 2 < sms);
+  }
+  const uint64_t share = all / sms;
+  return tile > (e == 1   ? 10600 + share * 32 / 100 + bytes / 20000 + rows * 2
+                 : e == 2 ? 8300 + share * 33 / 100 + bytes / 10000 + rows * 6
+                 : e == 4 ? 7100 + share * 26 / 100 + bytes / 6000 + rows * 4
+                          : 6400 + bytes / 5000 + rows * 8 +
+                                share * (vectors && b % 2 == 0 ? 13 : 18) / 100);
+}
 
 enum class Method { Auto, BS, Pttwac, Stash, TwoPass, Cycles, Staged, Resident };
 
@@ -553,24 +624,13 @@ static bool do_0100(cudaStream_t s, void *buf, int e, uint64_t T, uint64_t a,
     const uint64_t sms = (uint64_t)device_info().sms;
     bool thin = m == Method::Auto && !t010 && bytes >= (1ull << 20) &&
                 ctas < sms;
-    // Where the form held in shared memory can take it (about 10 us and 0.25
-    // us per MB whatever the shape), the on-chip tile is the better one while
-    // a CTA has few elements to move one by one (about 5.3 us and 0.31 ns
-    // each): 41 x 1598 bytes in one CTA 25.0 us, 12.2 held; 1704 x 38
-    // half-words 24.8 and 10.4; 362 x 362 half-words in a cluster of four
-    // 18.8 and 11.9; but 66 tiles of 363 x 17 doubles 8.3 and 10.4, 100 of
-    // 129 x 129 12.2 and 13.9, 635 of 153 x 11 half-words 10.9 and 14.4.
-    // Clusters that leave SMs idle lose as well (15 tiles of 770 x 37 doubles
-    // 12.2 and 10.5).
-    const uint64_t elems = a * B * b * p.tiles_per_chunk / (uint64_t)p.cluster;
-    const bool held = elems > kTileElems + bytes / 1250 ||
-                      (p.cluster > 1 && ctas < sms);
-    if (m == Method::Auto && !t010 && p.feasible && !getenv("LM_NO_RESIDENT") &&
-        !planner_beside_other_work() && (thin || held) &&
-        resident0100_applies(T, a, B, b, e)) {
-      // (under stream capture the resident form does not run)
+    // (under stream capture the resident form does not run)
+    if (m == Method::Auto && !t010 && p.feasible &&
+        !planner_beside_other_work() && !getenv("LM_NO_RESIDENT")) {
+      const bool held = held_preferred(buf, T, a, B, b, e, p);
       cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-      if (cudaStreamIsCapturing(s, &cs) == cudaSuccess &&
+      if ((thin || held) && resident0100_applies(T, a, B, b, e) &&
+          cudaStreamIsCapturing(s, &cs) == cudaSuccess &&
           cs == cudaStreamCaptureStatusNone)
         thin = held;
     }

@@ -2006,13 +2006,15 @@ static bool staged_job(BJob &j, const lm_job &jb, const Normalized &nz,
   if (tune_params().square) Si = Sj = tune_params().square;
   Si = std::min<uint64_t>(Si, nz.a);
   Sj = std::min<uint64_t>(Sj, nz.B);
-  // units of several elements: blocks of even height down the rows, as a last
-  // one of a few rows costs the ordered form as much as a whole one (100 rows
-  // of 42-byte units in blocks of 32, 600 MB, 948 us, of 25 754; staged 819
-  // and 804)
-  if (nz.b > 1 && !tune_params().square) {
+  // units written one element at a time: where the last blocks down the rows
+  // hold little, all of even height, as such a block costs the ordered form as
+  // much as a whole one (100 rows of 42-byte units in blocks of 32, 600 MB, 948
+  // us, of 25 754; staged 819 and 804).  Not in the form held in shared memory
+  // (which sets its widths): 41 x 186 units of 140 bytes 11.6 us, even 12.6
+  if (nz.b > 1 && (unit % 16 || ((uintptr_t)jb.buf & 15)) &&
+      !tune_params().square && !tune_params().staged_wide) {
     const uint64_t n = (nz.a + Si - 1) / Si;
-    Si = (nz.a + n - 1) / n;
+    if ((n * Si - nz.a) * 16 > nz.a) Si = (nz.a + n - 1) / n;
   }
   j.ragged = j.extra = j.contig = 0;
   const uint64_t row = nz.B * unit;

@@ -54,3 +54,27 @@ def test_stash(a, B, b, e, off, stash):
 def test_wave_of_units_of_elements(a, mb, b, e, off, wave):
     B = (mb << 20) // (a * b * e)
     assert (_route(1, a, B, b, e, off) == WAVE) == wave
+
+
+@pytest.mark.parametrize("T,a,B,b,e,off,ran", [
+    # units of one element: long tiles held, short ones and vector columns not
+    (1, 41, 1598, 1, 1, 0, {"resident"}), (66, 363, 17, 1, 8, 0, {"bs_tile"}),
+    (22, 246, 74, 1, 8, 0, {"resident"}), (62, 8, 8266, 1, 4, 0, {"bs_cluster"}),
+    (1, 4, 17951, 1, 2, 0, {"bs_cluster"}),
+    # units of several, written one element at a time either way
+    (2, 92, 30, 45, 1, 0, {"resident"}), (148, 91, 2, 163, 1, 0, {"bs_tile"}),
+    (35, 3, 2405, 86, 1, 1, {"bs_cluster"}),
+    # clusters that do not fit at once
+    (9, 327, 38, 105, 2, 0, {"resident"}), (14, 15, 27, 706, 4, 0, {"bs_cluster"}),
+])
+def test_held_or_tiles(T, a, B, b, e, off, ran):
+    assert _route(T, a, B, b, e, off) == ran
+
+
+def test_tiles_or_short_cycles():
+    """Units whose cycles are short: whole cycles where their list is kept."""
+    lm.lib().lm_marshal_finalize()
+    assert _route(1, 4, 40, 768, 2) == {"bs_cluster"}
+    for _ in range(2):
+        ran = _route(21, 8, 2, 847, 8) - {"cycle_leaders"}
+        assert ran == {"cycle_move"}
