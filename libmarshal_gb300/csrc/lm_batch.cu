@@ -3100,6 +3100,12 @@ static bool plan_square(SqArgs &g, void *buf, uint64_t T, uint64_t a,
                     rounds(S / 2) * (S / 2 * unit >= 256 ? 1.2 : 2.2) <
                         rounds(S)))
     S /= 2;
+  // units of several bytes or half-words, which are written one element at a
+  // time: not where few CTAs have a pair of long blocks each (335^2 units of 31
+  // bytes 38.8 us, 26.5 held in shared memory; 280^2 of 13 20.6 and 16.8; but
+  // 430^2 of 15 level, 621^2 of 9 0.7 times)
+  if (b >= 8 && e <= 2 && pairs(S) * 16 < (uint64_t)device_info().sms * 9)
+    return false;
   const uint64_t nb = (a + S - 1) / S, RW = 16 / (uint64_t)e;
   S = ((a + nb - 1) / nb + RW - 1) / RW * RW;
   const TuneParams saved = tune_params();
@@ -3114,6 +3120,11 @@ static bool plan_square(SqArgs &g, void *buf, uint64_t T, uint64_t a,
       4 * stage + 4096 > (size_t)device_info().max_smem_optin)
     return false;
   if (e <= 2 && b == 1 && !g.job.vb1 && g.job.vbc < 8) return false;
+  // ... nor where an SM holds one CTA (1152^2 units of 31 bytes 157 us, staged
+  // 105; 3912^2 of 7 368 and 259, 2421^2 of 15 half-words 309 and 243)
+  if (b > 1 && e <= 2 &&
+      2 * (4 * stage + 6144) > (size_t)device_info().max_smem_per_sm)
+    return false;
   g.job.scratch = g.job.base;
   g.nb = g.job.nJ;
   const uint32_t per = g.nb * (g.nb + 1) / 2;

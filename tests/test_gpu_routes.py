@@ -78,3 +78,13 @@ def test_tiles_or_short_cycles():
     for _ in range(2):
         ran = _route(21, 8, 2, 847, 8) - {"cycle_leaders"}
         assert ran == {"cycle_move"}
+
+
+@pytest.mark.parametrize("T,a,b,e,off,square", [
+    (1, 335, 31, 1, 0, False), (1, 1152, 31, 1, 0, False),
+    (1, 280, 13, 1, 8, False), (1, 621, 9, 1, 0, True),
+    (1, 3912, 7, 1, 0, False), (1, 2421, 15, 2, 2, False),
+    (1, 1000, 13, 2, 0, True), (1, 335, 7, 4, 0, True), (3, 400, 3, 8, 8, True),
+])
+def test_squares_of_units(T, a, b, e, off, square):
+    assert (_route(T, a, a, b, e, off) == {"square"}) == square
