@@ -79,3 +79,13 @@ def test_calls_after_an_empty_one(off):
                                                y, pad, unpad, 0,
                                                1_000_000) is False
         _check(4, 1000, 600, 1010, off)
+
+
+@pytest.mark.parametrize("x,pad", [(0, 1), (1, 2), (1, 3), (2, 3), (3, 4),
+                                   (4, 5), (5, 9), (12, 14), (25, 26)])
+def test_short_rows_of_doubles(x, pad):
+    """A vector's two elements in one row, in two, or in a row's padding, over
+    many tasks and on both halves of a vector."""
+    for off in (0, 8):
+        for y in (1, 7, 40001):
+            _check(8, x, y, pad, off)
