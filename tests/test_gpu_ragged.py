@@ -84,3 +84,19 @@ def test_groups_of_rows(groups, e):
         for B in (7, 131, 517):
             _check(2, a, B, e, STAGED)
             _check(2, a, B, e, RESIDENT)
+
+
+@pytest.mark.parametrize("a,B", [(905, 1082), (323, 1243), (2111, 853),
+                                 (1217, 1213), (3301, 2503), (150, 9001)])
+@pytest.mark.parametrize("off", [0, 3, 8])
+def test_bytes_held_in_smaller_blocks(a, B, off):
+    """Ragged blocks of bytes of each size that the held form chooses among."""
+    n = a * B
+    raw = torch.randint(0, 256, (n + 64,), dtype=torch.uint8, device="cuda")
+    before = raw.clone()
+    lm.transpose_0100(raw.data_ptr() + off, 1, a, B, 1, method=7, elem_bytes=1)
+    torch.cuda.synchronize()
+    assert torch.equal(raw[off:off + n],
+                       before[off:off + n].view(a, B).t().reshape(-1))
+    assert torch.equal(raw[:off], before[:off])
+    assert torch.equal(raw[off + n:], before[off + n:])
