@@ -667,15 +667,22 @@ static bool do_0100(cudaStream_t s, void *buf, int e, uint64_t T, uint64_t a,
   }
   // a payload that fits the shared memory of all SMs: one cooperative
   // launch at 2 x payload (not beside other work, where it would wait for
-  // every SM to drain, nor under stream capture)
-  if (m == Method::Resident ||
-      (m == Method::Auto && !planner_beside_other_work() &&
-       !getenv("LM_NO_RESIDENT"))) {
+  // every SM to drain, nor under stream capture); where bytes would be written
+  // one by one, near that limit, the staged form first, if its scratch can be had
+  // (11675 x 2179 38.1 us and 29.3, 20854 x 1455 49.4 and 31.0)
+  const bool may_hold = m == Method::Auto && !planner_beside_other_work() &&
+                        !getenv("LM_NO_RESIDENT");
+  const bool hold_last = may_hold && !getenv("LM_NO_STAGED") &&
+                         T * a * B * b * e >= (16ull << 20) &&
+                         resident0100_by_elements(buf, T, a, B, b, e);
+  auto hold = [&]() {
     uint32_t *status = device_status_word();
-    const cudaError_t err =
-        status ? launch_resident0100(s, buf, e, T, a, B, b, status,
-                                     wait_timeout_ns())
-               : cudaErrorNotSupported;
+    return status ? launch_resident0100(s, buf, e, T, a, B, b, status,
+                                        wait_timeout_ns())
+                  : cudaErrorNotSupported;
+  };
+  if (m == Method::Resident || (may_hold && !hold_last)) {
+    const cudaError_t err = hold();
     if (err == cudaSuccess) return false;
     if (err != cudaErrorNotSupported) return cuda_fail(err, "resident launch");
     if (m == Method::Resident)
@@ -745,6 +752,11 @@ static bool do_0100(cudaStream_t s, void *buf, int e, uint64_t T, uint64_t a,
     } else if (m == Method::Staged) {
       return fail("staged: units above 32 KB or too many blocks");
     }
+  }
+  if (hold_last) {
+    const cudaError_t err = hold();
+    if (err == cudaSuccess) return false;
+    if (err != cudaErrorNotSupported) return cuda_fail(err, "resident launch");
   }
   // the stash plan moves 3 x payload with half the scratch, where the forms
   // above could not have theirs.  Its wavefront spreads rows over all CTAs:

@@ -3440,6 +3440,18 @@ bool resident0100_applies(uint64_t T, uint64_t a, uint64_t B, uint64_t b,
                               d->max_dyn);
 }
 
+bool resident0100_by_elements(void *buf, uint64_t T, uint64_t a, uint64_t B,
+                              uint64_t b, int e) {
+  if (e != 1 || b != 1 || T == 0 || a <= 1 || B <= 1) return false;
+  ResDevice *d = res_device();
+  ResArgs g{};
+  uint32_t grid = 0;
+  size_t dyn = 0;
+  return d &&
+         plan_resident_cached(g, &grid, &dyn, buf, T, a, B, b, e, d->max_dyn) &&
+         g.nper > 1 && !g.job.ragged && !g.job.vb1 && !g.job.vbc;
+}
+
 cudaError_t launch_resident0100(cudaStream_t s, void *buf, int e, uint64_t T,
                                 uint64_t a, uint64_t B, uint64_t b,
                                 uint32_t *status, uint64_t timeout_ns,

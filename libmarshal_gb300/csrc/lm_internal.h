@@ -256,6 +256,10 @@ cudaError_t launch_square0100(cudaStream_t s, void *buf, int e, uint64_t T,
 // arrivals more than there are CTAs).
 bool resident0100_applies(uint64_t T, uint64_t a, uint64_t B, uint64_t b,
                           int e);
+// Whether it would write the bytes of this buffer one by one, without room for
+// ragged blocks (more than a block per CTA).
+bool resident0100_by_elements(void *buf, uint64_t T, uint64_t a, uint64_t B,
+                              uint64_t b, int e);
 cudaError_t launch_resident0100(cudaStream_t s, void *buf, int e, uint64_t T,
                                 uint64_t a, uint64_t B, uint64_t b,
                                 uint32_t *status, uint64_t timeout_ns,

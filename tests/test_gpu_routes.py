@@ -88,3 +88,12 @@ def test_tiles_or_short_cycles():
 ])
 def test_squares_of_units(T, a, b, e, off, square):
     assert (_route(T, a, a, b, e, off) == {"square"}) == square
+
+
+@pytest.mark.parametrize("a,B,off,held", [
+    (11675, 2179, 0, False), (20854, 1455, 1, False), (3758, 7173, 0, False),
+    (15048, 1907, 8, True),   # 8-byte vectors
+    (13228, 1893, 0, True), (9148, 2673, 0, True), (4001, 4003, 1, True),
+])
+def test_bytes_near_the_limit_of_the_held_form(a, B, off, held):
+    assert (_route(1, a, B, 1, 1, off) == {"resident"}) == held
