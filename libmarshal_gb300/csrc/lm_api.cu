@@ -451,60 +451,59 @@ static bool stash_preferred(const void *buf, uint64_t T, uint64_t a, uint64_t B,
 //    3 x 2405 of 86 bytes 23.2 and 33.4.
 // Units of 64 bytes and more whose cycles are short go to those instead: 9 us
 // where their list is kept, 14.5 where not (4 x 40 units of 1536 bytes 8.3 and
-// 15.2), and 0.5 per MB; where it is kept with half of the SMs idle from 512 KB
-// on in any case (21 tiles of 8 x 2 units of 6776 bytes 8.3 and 7.4).
+// 15.2), and 0.5 per MB of doubles to 4 per MB of bytes (314 tiles of 5 x 38 units
+// of 347 bytes 56.9 and 70.5); where it is kept with half of the SMs idle from
+// 512 KB on in any case (21 tiles of 8 x 2 units of 6776 bytes 8.3 and 7.4).
 static bool held_preferred(const void *buf, uint64_t T, uint64_t a, uint64_t B,
                            uint64_t b, int e, const BsPlan &p) {
-  const DeviceInfo &di = device_info();
-  const uint64_t sms = (uint64_t)di.sms, C = (uint64_t)p.cluster;
+  const uint64_t sms = (uint64_t)device_info().sms, C = (uint64_t)p.cluster;
   const uint64_t chunks = (T + p.tiles_per_chunk - 1) / p.tiles_per_chunk;
   const uint64_t all = T * a * B * b, bytes = all * (uint64_t)e;
   const uint64_t rows = T * a / sms;
   const bool vectors = ((uintptr_t)buf & 15) == 0;
-  // elements of a CTA, for as many rounds as the tiles take
-  const uint64_t at_once =
-      C == 1   ? sms * std::max<uint64_t>(1, (uint64_t)di.max_smem_per_sm /
-                                                 (p.smem_bytes + 1024))
-      : C == 2 ? sms * 75 / 152
-      : C == 4 ? sms * 36 / 152
-      : C == 8 ? sms * 15 / 152
-               : sms * 7 / 152;
-  const uint64_t rounds = chunks / std::max<uint64_t>(1, at_once) +
-                          (chunks % std::max<uint64_t>(1, at_once) != 0);
+  // elements of an SM, or of a CTA of a cluster for as many rounds as it takes
+  // (one cluster of 16 to a GPC of about 20 SMs, two of 8, ...)
+  const uint64_t fit = std::max<uint64_t>(
+      1, sms * (C == 2 ? 75 : C == 4 ? 36 : C == 8 ? 15 : 7) / 152);
   const uint64_t elems =
-      rounds * a * b * (C == 1 ? B * p.tiles_per_chunk : p.rows_per_cta);
+      C == 1 ? a * B * b * p.tiles_per_chunk * std::max(chunks, sms) / sms
+             : a * b * p.rows_per_cta * ((chunks + fit - 1) / fit);
   if (b == 1) {
     const uint64_t out = a * e;  // bytes of an output row
-    const uint64_t tile =
-        C == 1   ? 3800 + elems * 32 / 100
-        : e == 8 ? 4400 + elems * 28 / 100
-                 : 5300 + elems * (e > 1 && vectors && out % 16 == 0 ? 10 : 18) / 100;
-    if ((out <= 16 || out == 32) && out % 4 == 0 &&
+    const uint64_t ps = !vectors || out % 16 ? 180 : e == 1 ? 50 : e == 2 ? 80 : 100;
+    const uint64_t tile = C == 1   ? 3800 + elems * 32 / 100
+                          : e == 8 ? 4400 + elems * 28 / 100 + a * 2
+                                   : 5300 + elems * ps / 1000 + a * 2;
+    if ((out == 4 || out == 8 || out == 16 || out == 32) &&
         ((uintptr_t)buf & 3) == 0 && (a >= 4 || e == 8))
       return tile > (e == 1   ? 20000 + bytes / 450
                      : e == 2 ? 12500 + bytes / 550
-                     : e == 4 ? 7500 + bytes / 1000
-                              : 9400 + bytes / 2500);
-    return tile > (e == 1   ? 8300 + bytes / 1700
-                   : e == 2 ? 7500 + bytes / 2000
+                     : e == 4 ? 9500 + bytes / 1000
+                              : 7400 + bytes / 1000);
+    return tile > (e == 1   ? 9300 + bytes / 1700
+                   : e == 2 ? 8200 + bytes / 2000
                    : e == 4 ? 6700 + bytes / 3000 + rows * 3
                             : 6500 + bytes / 3300 + rows * 3);
   }
   const uint64_t tile = C == 1  ? 3400 + elems * 36 / 100
-                        : e < 8 ? 6500 + elems * 18 / 100
-                                : 4800 + elems * 26 / 100;
-  if (b * e >= 64 && !getenv("LM_NO_CYCLES") && a * B - 1 <= (1ull << 28) &&
-      tile > 7000 && cycle_order(a, B, kCycleMaxLen)) {
-    const bool kept = cycle_list_kept(a, B, 0);
-    return tile > (kept ? 9000u : 14500u) + bytes / 2000 ||
-           (kept && bytes >= (512ull << 10) && chunks * C * 2 < sms);
-  }
-  const uint64_t share = all / sms;
-  return tile > (e == 1   ? 10600 + share * 32 / 100 + bytes / 20000 + rows * 2
-                 : e == 2 ? 8300 + share * 33 / 100 + bytes / 10000 + rows * 6
-                 : e == 4 ? 7100 + share * 26 / 100 + bytes / 6000 + rows * 4
-                          : 6400 + bytes / 5000 + rows * 8 +
-                                share * (vectors && b % 2 == 0 ? 13 : 18) / 100);
+                        : e < 8 ? 6500 + elems * 18 / 100 + a * 2
+                                : 4800 + elems * 26 / 100 + a * 2;
+  const uint64_t share = std::max<uint64_t>(all / sms, 8192 / (uint64_t)e);
+  if (tile <= (e == 1   ? 8000 + share * 32 / 100 + bytes / 20000 + rows * 2
+               : e == 2 ? 8300 + share * 33 / 100 + bytes / 10000 + rows * 6
+               : e == 4 ? 7100 + share * 26 / 100 + bytes / 6000 + rows * 4
+                        : 6400 + bytes / 5000 + rows * 8 +
+                              share * (vectors && b % 2 == 0 ? 13 : 18) / 100))
+    return false;
+  if (b * e < 64 || getenv("LM_NO_CYCLES") || a * B - 1 > (1ull << 28) ||
+      !cycle_order(a, B, kCycleMaxLen))
+    return true;
+  const bool kept = cycle_list_kept(a, B, 0);
+  return tile > (kept ? 9000 : 14500) + bytes / (e == 1   ? 500
+                                                 : e == 2 ? 900
+                                                 : e == 4 ? 1300
+                                                          : 2000) ||
+         (kept && bytes >= (512ull << 10) && chunks * C * 2 < sms);
 }
 
 enum class Method { Auto, BS, Pttwac, Stash, TwoPass, Cycles, Staged, Resident };

@@ -3339,9 +3339,10 @@ bool plan_resident(ResArgs &g, uint32_t *grid, size_t *dyn, void *buf,
         }
         // the largest block of this width that fits; of ragged bytes the
         // smaller ones as well, as their steps cost more (905 x 1082 14.1 us,
-        // in blocks of 16 KB 12.7; of half-words and of short rows the larger
-        // ones are better, 2261 x 1007 14.8 and 16.9)
-        if (j.ragged != 1 || j.contig || e > 1) break;
+        // in blocks of 16 KB 12.7; of half-words the larger ones are better,
+        // 2261 x 1007 14.8 and 16.9, and of short rows, where these are not few:
+        // 107087 x 2 13.9 and 11.5)
+        if (j.ragged != 1 || e > 1 || (j.contig && nblk > 32)) break;
       }
     }
   }
