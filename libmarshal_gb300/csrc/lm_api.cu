@@ -73,9 +73,13 @@ static bool fail(const char *fmt, ...) {
   return true;
 }
 
-bool set_error(const char *msg) { return fail("%s", msg); }
+bool set_error(const char *msg) {
+  cudaGetLastError();  // (as in cuda_fail)
+  return fail("%s", msg);
+}
 
 static bool cuda_fail(cudaError_t e, const char *what) {
+  cudaGetLastError();  // reported here, not by the next call's check
   return fail("%s: %s", what, cudaGetErrorString(e));
 }
 
@@ -157,8 +161,10 @@ uint32_t *device_status_word() {
   std::lock_guard<std::mutex> lock(mu);
   if (!words[dev]) {
     void *p = nullptr;
-    if (cudaMalloc(&p, 4) != cudaSuccess) return nullptr;
-    if (cudaMemset(p, 0, 4) != cudaSuccess) return nullptr;
+    if (cudaMalloc(&p, 4) != cudaSuccess || cudaMemset(p, 0, 4) != cudaSuccess) {
+      cudaGetLastError();  // the callers have other ways
+      return nullptr;
+    }
     words[dev] = (uint32_t *)p;
   }
   return words[dev];

@@ -3411,7 +3411,10 @@ ResDevice *res_device() {
   size_t max_dyn = (size_t)di.max_smem_optin;
   for (const void *k : kResidentKernels) {
     cudaFuncAttributes fa{};
-    if (cudaFuncGetAttributes(&fa, k) != cudaSuccess) return nullptr;
+    if (cudaFuncGetAttributes(&fa, k) != cudaSuccess) {
+      cudaGetLastError();
+      return nullptr;
+    }
     max_dyn = std::min(max_dyn, (size_t)di.max_smem_optin > fa.sharedSizeBytes
                                     ? ((size_t)di.max_smem_optin -
                                        fa.sharedSizeBytes) / 128 * 128
@@ -3419,8 +3422,10 @@ ResDevice *res_device() {
   }
   for (const void *k : kResidentKernels)
     if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)max_dyn) != cudaSuccess)
+                             (int)max_dyn) != cudaSuccess) {
+      cudaGetLastError();
       return nullptr;
+    }
   d = new ResDevice;
   d->max_dyn = max_dyn;
   g_res_dev[di.device] = d;
@@ -3483,6 +3488,7 @@ cudaError_t launch_resident0100(cudaStream_t s, void *buf, int e, uint64_t T,
       kResidentKernels[e == 1 ? 0 : e == 2 ? 1 : e == 4 ? 2 : 3], dim3(grid),
       dim3(kResThreads), args, dyn, s);
   if (err != cudaSuccess) {
+    cudaGetLastError();
     // no CTA arrives: the slot keeps the count it had
     std::lock_guard<std::mutex> lock(g_res_mu);
     d->arrivals[g.slot] -= grid;

@@ -23,7 +23,10 @@ cudaError_t grow_smem_limit(const void *kern, size_t smem) {
   if (limit >= smem) return cudaSuccess;
   const cudaError_t err = cudaFuncSetAttribute(
       kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  if (err == cudaSuccess) limit = smem;
+  if (err == cudaSuccess)
+    limit = smem;
+  else
+    cudaGetLastError();  // (not for the check after a later launch to find)
   return err;
 }
 
@@ -44,8 +47,10 @@ int prepare_launch(const void *kern, LaunchCache &c, size_t smem, int threads,
   if (key && (key >> 16) == (uint64_t)smem) return (int)(key & 0xffff);
   int occ = 0;
   if ((*err = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, threads,
-                                                            smem)) != cudaSuccess)
+                                                            smem)) != cudaSuccess) {
+    cudaGetLastError();
     return 0;
+  }
   c.occ_key[d].store(((uint64_t)smem << 16) | (uint64_t)(occ & 0xffff),
                      std::memory_order_release);
   return occ;

@@ -568,8 +568,10 @@ static int wave_occupancy(size_t smem) {
   if (grow_smem_limit((const void *)kern, smem) != cudaSuccess) return 0;
   int occ = 0;
   if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, kWaveThreads,
-                                                    smem) != cudaSuccess)
+                                                    smem) != cudaSuccess) {
+    cudaGetLastError();
     return 0;
+  }
   return occ;
 }
 

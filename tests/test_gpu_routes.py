@@ -97,3 +97,31 @@ def test_squares_of_units(T, a, b, e, off, square):
 ])
 def test_bytes_near_the_limit_of_the_held_form(a, B, off, held):
     assert (_route(1, a, B, 1, 1, off) == {"resident"}) == held
+
+
+@pytest.mark.parametrize("a,B,b,e", [(12684, 6629, 1, 1), (12700, 6629, 1, 1),
+                                     (12684, 947, 7, 1), (25000, 600, 3, 2),
+                                     (30100, 301, 9, 1)])
+def test_first_call_of_a_stash_plan(a, B, b, e):
+    """A plan that tries sizes beyond the limit of shared memory, in a thread
+    that has planned nothing yet: neither its call nor the next one finds the
+    refused size's error."""
+    import threading
+    n = a * B * b * e
+    raw = torch.randint(0, 256, (n,), dtype=torch.uint8, device="cuda")
+    want = raw.view(a, B, b * e).transpose(0, 1).reshape(-1)
+    failed = []
+
+    def work():
+        for method, x in ((3, raw), (0, raw.clone())):
+            try:
+                lm.transpose_0100(x, 1, a, B, b, method=method, elem_bytes=e)
+            except Exception as ex:  # noqa: BLE001
+                failed.append((method, str(ex)))
+        torch.cuda.synchronize()
+
+    t = threading.Thread(target=work)
+    t.start()
+    t.join()
+    assert not failed
+    assert torch.equal(raw, want)

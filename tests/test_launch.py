@@ -25,9 +25,16 @@ static std::map<std::pair<const void *, int>, int> g_limit;
 static std::atomic<int> g_sets{0}, g_hold{0}, g_applied{0};
 
 extern "C" cudaError_t cudaGetDevice(int *d) { *d = t_dev; return cudaSuccess; }
+static thread_local cudaError_t t_last = cudaSuccess;
+extern "C" cudaError_t cudaGetLastError() {
+  const cudaError_t e = t_last;
+  t_last = cudaSuccess;
+  return e;
+}
 extern "C" cudaError_t cudaFuncSetAttribute(const void *k, cudaFuncAttribute,
                                             int v) {
   g_sets++;
+  if (v > 227 << 10) return t_last = cudaErrorInvalidValue;
   // the call that is to lose: applied after the other thread's, if that one
   // comes through meanwhile
   if (v == g_hold)
@@ -120,3 +127,20 @@ def test_devices_have_their_own(tmp_path):
     t_dev = dev;
     launch(&k, c, 100 << 10);
   }""")
+
+
+def test_a_refused_limit_leaves_no_error(tmp_path):
+    """A size that the driver refuses is reported by its caller alone: the error
+    is not left for the check of the next launch to find."""
+    _run(tmp_path, r"""
+  static lm::LaunchCache c;
+  static char k;
+  cudaError_t err;
+  if (lm::prepare_launch(&k, c, 300 << 10, 256, &err) != 0 ||
+      err != cudaErrorInvalidValue || cudaGetLastError() != cudaSuccess)
+    return puts("an error is pending"), 1;
+  launch(&k, c, 100 << 10);
+  if (lm::grow_smem_limit(&k, 300 << 10) != cudaErrorInvalidValue ||
+      cudaGetLastError() != cudaSuccess)
+    return puts("an error is pending"), 1;
+  launch(&k, c, 200 << 10);""")
