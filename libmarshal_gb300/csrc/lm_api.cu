@@ -447,8 +447,9 @@ static bool stash_preferred(const void *buf, uint64_t T, uint64_t a, uint64_t B,
 // shared memory of all SMs 12.2, 362 x 362 half-words in a cluster of four 18.8
 // and 11.9, 9 tiles of 327 x 38 units of 210 bytes 52 and 39.  The held form
 // takes 6 to 10 us, and
-//  * for units of one element 0.3 to 0.6 us per MB (22 tiles of 246 x 74 doubles
-//    10.3 and 8.3, 66 of 363 x 17 8.3 and 10.4), but 0.4 to 2.6 us per MB where a
+//  * for units of one element 0.3 to 0.6 us per MB, and some for each tile and
+//    row (22 tiles of 246 x 74 doubles 10.3 and 8.3, 66 of 363 x 17 8.3 and 10.4,
+//    2108 of 2679 x 2 half-words 23.2 and 37.6), but 0.4 to 2.6 us per MB where a
 //    column is a vector or two or a part of one (62 tiles of 8 x 8266 floats 8.8
 //    and 17.0, 27 of 4 x 107368 half-words 24.6 and 51.0);
 //  * for units of several, which it writes one element at a time too, the time
@@ -470,7 +471,7 @@ static bool held_preferred(const void *buf, uint64_t T, uint64_t a, uint64_t B,
   // elements of an SM, or of a CTA of a cluster for as many rounds as it takes
   // (one cluster of 16 to a GPC of about 20 SMs, two of 8, ...)
   const uint64_t fit = std::max<uint64_t>(
-      1, sms * (C == 2 ? 75 : C == 4 ? 36 : C == 8 ? 15 : 7) / 152);
+      1, sms * (C == 2 ? 76 : C == 4 ? 36 : C == 8 ? 15 : 7) / 152);
   const uint64_t elems =
       C == 1 ? a * B * b * p.tiles_per_chunk * std::max(chunks, sms) / sms
              : a * b * p.rows_per_cta * ((chunks + fit - 1) / fit);
@@ -486,10 +487,10 @@ static bool held_preferred(const void *buf, uint64_t T, uint64_t a, uint64_t B,
                      : e == 2 ? 12500 + bytes / 550
                      : e == 4 ? 9500 + bytes / 1000
                               : 7400 + bytes / 1000);
-    return tile > (e == 1   ? 9300 + bytes / 1700
-                   : e == 2 ? 8200 + bytes / 2000
-                   : e == 4 ? 6700 + bytes / 3000 + rows * 3
-                            : 6500 + bytes / 3300 + rows * 3);
+    return tile > T * 350 / sms + (e == 1   ? 9300 + bytes / 1700 + rows * 35 / 100
+                                   : e == 2 ? 8200 + bytes / 2000 + rows * 35 / 100
+                                   : e == 4 ? 6700 + bytes / 3000 + rows * 3
+                                            : 6500 + bytes / 3300 + rows * 3);
   }
   const uint64_t tile = C == 1  ? 3400 + elems * 36 / 100
                         : e < 8 ? 6500 + elems * 18 / 100 + a * 2

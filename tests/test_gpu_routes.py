@@ -61,6 +61,7 @@ def test_wave_of_units_of_elements(a, mb, b, e, off, wave):
     (1, 41, 1598, 1, 1, 0, {"resident"}), (66, 363, 17, 1, 8, 0, {"bs_tile"}),
     (22, 246, 74, 1, 8, 0, {"resident"}), (62, 8, 8266, 1, 4, 0, {"bs_cluster"}),
     (1, 4, 17951, 1, 2, 0, {"bs_cluster"}),
+    (2108, 2679, 2, 1, 2, 2, {"bs_tile"}),  # many tiles of many rows
     # units of several, written one element at a time either way
     (2, 92, 30, 45, 1, 0, {"resident"}), (148, 91, 2, 163, 1, 0, {"bs_tile"}),
     (35, 3, 2405, 86, 1, 1, {"bs_cluster"}),
