@@ -407,35 +407,38 @@ static size_t wave_scratch(void *buf, uint64_t T, uint64_t a, uint64_t B,
 
 // The stash plan before the forms through scratch, where its wavefront has the
 // rows (kStashRowsPerSm).  Its writers go down a column of rows, the blocks of
-// the others write units of several elements one element at a time:
-//  * units of several bytes or half-words, at every size (us, stash and the
-//    better of staged and ordered, 60 / 130 / 400 MB): 15001 rows of 7-byte
-//    units 95 / 178 / 473 and 143 / 284 / 792; of 66-byte units 64 / 110 / 269
-//    and 85 / 176 / 493; 7400 rows of 9-byte units 120 / 237 / 672 and 141 / 284
-//    / 821;
-//  * units of several words from 128 MB on, where a step's strip holds 384 bytes
-//    of a row: 15001 rows of 12-byte units 60 / 102 / 235 and 57 / 115 / 309 (of
-//    8-byte elements never: 24-byte units 55 / 97 / 229 and 43 / 89 / 225);
-//  * half-words in tall matrices whose output rows are no whole vectors long:
-//    at 13529 columns level with the ordered form at 24000 rows, and faster above
-//    (28775 465 and 475, 31006 486 and 506, 38902 583 and 629).  With fewer
-//    columns it is the slower one, at 31001 rows by 4 % at 7003, 12 at 4005
-//    and 31 at 2005: none below 4000.  Rows 2 bytes past whole vectors take it
-//    13-20 % longer at every height, for no cause that could be shown; those of
-//    the seven other places do not differ.  (Bytes, 28775 x 27060: 657 and 514.)
+// the others write units of several elements one element at a time, if those are
+// no whole vectors.  Microseconds, stash and the better of staged and ordered (with
+// the row offsets of the stash kept; found on each call, as where 16 shapes are
+// kept already, they cost 12 more):
+//  * units of several bytes or half-words, at every size: 20000 rows of 9-byte
+//    units, 34 / 100 / 200 MB, 51 / 127 / 234 and 88 / 230 / 424, 7400 rows of
+//    10-byte ones 50 / 126 / 238 and 59 / 134 / 267;
+//  * of several words too: 15001 rows of 12-byte units, 48 / 112 / 300 MB, 43 / 79 /
+//    173 and 50 / 98 / 237, 8000 of 44-byte ones 41 / 79 / 177 and 50 / 98 / 234;
+//  * of several doubles from 128 MB on: 12298 rows of 40-byte units, 64 / 112 / 160 /
+//    600 MB, 51 / 76 / 99 / 316 and 45 / 76 / 112 / 338;
+//  * half-words in tall matrices whose output rows are no whole vectors long: at
+//    13530 columns level with the ordered form at 20000 rows, and faster above
+//    (23001 372 and 384, 28775 443 and 478, 38902 554 and 639); with fewer columns
+//    it loses some of that (28775 x 7003 239 and 254, 4005 152 and 155, 2005 92 and
+//    85).  Rows 2 bytes past whole vectors take it 13-15 % longer at every height,
+//    for no cause that could be shown; those of the seven other places do not
+//    differ.  (Bytes, 28775 x 27060: 657 and 514.)
+// Strips of fewer than 384 bytes, in very tall matrices, are for narrow elements.
 static bool stash_preferred(const void *buf, uint64_t T, uint64_t a, uint64_t B,
                             uint64_t b, int e) {
-  const uint64_t bytes = a * B * b * e;
   if (T != 1 || b * e >= 128 || a * B < (1ull << 20) ||
       a < kStashRowsPerSm * (uint64_t)device_info().sms)
     return false;
+  const bool vectors = b * e % 16 == 0 && ((uintptr_t)buf & 15) == 0;
   if (b == 1 ? e != 2 || a < 23000 || B < 4000 || B * 2 % 16 == 2 ||
                    a * 2 % 16 == 0 || !wave_preferred(buf, T, a, B, 1, 2)
-             : e > 4 || (e == 4 && bytes < (128ull << 20)))
+             : vectors || (e == 8 && a * B * b * e < (128ull << 20)))
     return false;
   if (getenv("LM_NO_STASH")) return false;
   const StashPlan p = plan_stash(a, B, (uint32_t)b, e);
-  return p.feasible && (e != 4 || p.g * b * e >= 384);
+  return p.feasible && (e < 4 || p.g * b * e >= 384);
 }
 
 // Whether a conversion in on-chip tiles by `p` is slower than what takes it

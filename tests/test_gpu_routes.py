@@ -35,8 +35,9 @@ def _route(T, a, B, b, e, off=0):
     (15001, 80, 33, 2, 0, True), (15001, 423, 33, 2, 2, True),
     (7400, 446, 127, 1, 0, True), (7000, 1214, 7, 1, 0, False),  # rows
     (15001, 420, 129, 1, 0, False),                    # units of 128 bytes
-    (15001, 2330, 3, 4, 0, True), (15001, 600, 3, 4, 0, False),
-    (30001, 600, 3, 8, 0, False),
+    (15001, 2330, 3, 4, 0, True), (15001, 230, 3, 4, 0, True),
+    (9001, 400, 3, 8, 0, False), (9001, 700, 3, 8, 0, True),
+    (9001, 3000, 4, 4, 4, True), (9001, 3000, 4, 4, 0, False),  # vectors
     (28775, 4005, 1, 2, 0, True), (28775, 3995, 1, 2, 0, False),
 ])
 def test_stash(a, B, b, e, off, stash):
