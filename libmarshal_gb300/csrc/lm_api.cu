@@ -548,15 +548,6 @@ static const TuneVariant kVariants[] = {
 };
 constexpr int kNumVariants = (int)(sizeof(kVariants) / sizeof(kVariants[0]));
 
-// Sets the thread's tuning overrides for the life of the object.
-struct TuneScope {
-  TuneParams saved;
-  explicit TuneScope(const TuneParams &p) : saved(tune_params()) {
-    tune_params() = p;
-  }
-  ~TuneScope() { tune_params() = saved; }
-};
-
 static bool check_launch(cudaError_t e, const char *what) {
   if (e != cudaSuccess) return cuda_fail(e, what);
   return false;

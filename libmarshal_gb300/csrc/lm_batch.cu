@@ -39,9 +39,6 @@ constexpr size_t kCounterBytes =
     (size_t)(5 + kBandGroups + 2 * kMaxWaves) * kCounterStride * 4;
 constexpr int kT010Counter = 2 + kBandGroups + 2 * kMaxWaves;
 constexpr uint64_t kDefaultArenaBytes = 1ull << 30;
-// jobs at least this large and with enough rows skip the waves: the planner
-// takes the ordered form (3 x payload, the staged form 4 x) where that pays
-constexpr uint64_t kStashPreferBytes = 64ull << 20;
 constexpr int kSideStreams = 6;      // streams of the large jobs
 constexpr int kGroupStreams = 8;     // streams of the item groups
 // jobs at least this large that go through scratch run as the planner's
@@ -2311,18 +2308,9 @@ static bool plan_batch(lm_batch_t bt, const lm_job *jobs, int n,
         bt->stats.big_bytes += bytes;
         continue;
       }
-      // a large 100 of many rows goes to the planner (whose ordered form moves
-      // 3 x payload instead of the staged form's 4)
-      if (nz.T == 1 && unit < 128 && bytes >= kStashPreferBytes &&
-          nz.a >= kStashRowsPerSm * (uint64_t)di.sms &&
-          nz.a * nz.B >= (1ull << 20) &&
-          plan_stash(nz.a, nz.B, (uint32_t)nz.b, e).feasible)
-        goto planner;
-      // large jobs of units of kStagedMaxUnit bytes and more: cycle
-      // following in the planner (2 x payload) is at least as fast
-      if (unit >= kStagedMaxUnit && bytes >= kStashPreferBytes) goto planner;
-      // a large job through scratch runs as the planner's own staged form
-      // (its gather and copy back overlap the other jobs on a side stream)
+      // a large job is the planner's: its forms at 2 and 3 x payload, or the
+      // staged form, whose gather and copy back overlap the other jobs on a
+      // side stream
       if (bytes >= kPlannerStagedBytes) goto planner;
       // staged: the job fits the arena (in the current wave or a new one)
       if (stageable) {
@@ -2339,9 +2327,12 @@ static bool plan_batch(lm_batch_t bt, const lm_job *jobs, int n,
           // (ragged blocks of 1- and 2-byte elements only: 28 MB of bytes in
           // 12 jobs 52 us without, 29 with; those of 4- and 8-byte elements
           // gain nothing beside other items, 245 MB 111 us either way)
-          tune_params().staged_plain = nz.e >= 4;
-          const bool fits = staged_job(j, jb, nz, &nblk, &stage);
-          tune_params().staged_plain = 0;
+          TuneParams tp = tune_params();
+          tp.staged_plain = nz.e >= 4;
+          const bool fits = [&]() {
+            TuneScope scope(tp);
+            return staged_job(j, jb, nz, &nblk, &stage);
+          }();
           if (!fits) goto planner;
           // same address modulo 16 as the buffer (see k_batch_copyback);
           // the arena base is set when the wave is enqueued
@@ -3108,15 +3099,13 @@ static bool plan_square(SqArgs &g, void *buf, uint64_t T, uint64_t a,
     return false;
   const uint64_t nb = (a + S - 1) / S, RW = 16 / (uint64_t)e;
   S = ((a + nb - 1) / nb + RW - 1) / RW * RW;
-  const TuneParams saved = tune_params();
-  tune_params() = TuneParams();
-  tune_params().square = (uint32_t)S;
-  tune_params().staged_plain = 1;
+  TuneParams tp;
+  tp.square = (uint32_t)S;
+  tp.staged_plain = 1;
+  TuneScope scope(tp);
   uint64_t nblk = 0;
   size_t stage = 0;
-  const bool ok = staged_job(g.job, jb, nz, &nblk, &stage);
-  tune_params() = saved;
-  if (!ok || pairs(S) >= 0xffffffffull ||
+  if (!staged_job(g.job, jb, nz, &nblk, &stage) || pairs(S) >= 0xffffffffull ||
       4 * stage + 4096 > (size_t)device_info().max_smem_optin)
     return false;
   if (e <= 2 && b == 1 && !g.job.vb1 && g.job.vbc < 8) return false;
@@ -3301,7 +3290,7 @@ bool plan_resident(ResArgs &g, uint32_t *grid, size_t *dyn, void *buf,
   nz.B = B;
   nz.b = b;
   if (T * a * B * b * (uint64_t)e > (uint64_t)di.sms * max_dyn) return false;
-  const TuneParams saved = tune_params();
+  TuneScope scope(tune_params());
   double best_cost = 0;
   bool ok = false;
   // (plain: blocks without the extra rows of unaligned narrow ones, whose
@@ -3346,7 +3335,6 @@ bool plan_resident(ResArgs &g, uint32_t *grid, size_t *dyn, void *buf,
       }
     }
   }
-  tune_params() = saved;
   return ok;
 }
 

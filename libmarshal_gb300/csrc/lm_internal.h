@@ -94,6 +94,15 @@ struct TuneParams {
   uint32_t square = 0;
 };
 TuneParams &tune_params();
+// Sets the thread's overrides for the life of the object, which may change
+// them meanwhile.
+struct TuneScope {
+  TuneParams saved;
+  explicit TuneScope(const TuneParams &p) : saved(tune_params()) {
+    tune_params() = p;
+  }
+  ~TuneScope() { tune_params() = saved; }
+};
 
 // True on a thread while the batch executor runs planner jobs beside its
 // other kernels: the planner then takes no whole-GPU cooperative form (its
