@@ -75,3 +75,55 @@ def test_forms_of_large_matrices(method):
 
     _threads(len(shapes), work)
     assert lm.lib().lm_device_status(None) == 0
+
+
+def test_padding_flags_of_many_threads():
+    """Twenty threads, more than blocks of flags are kept, pad and unpad their
+    own buffers with task counts that go up and down, on their own streams."""
+    shapes = [(1000, 600, 1010), (7, 9, 8), (300, 40000, 301), (50, 3001, 64),
+              (4000, 101, 4096)]
+
+    def work(k, s):
+        for i in range(6):
+            x, y, pad = shapes[(k + i) % len(shapes)]
+            src = torch.arange(k, k + y * x, dtype=torch.int32, device="cuda")
+            d = torch.full((y * pad,), -1, dtype=torch.int32, device="cuda")
+            d[:y * x] = src
+            lm.padding(d, x, y, pad, stream=s)
+            want = torch.zeros((y, pad), dtype=torch.int32, device="cuda")
+            want[:, :x] = src.view(y, x)
+            assert torch.equal(d.view(y, pad), want)
+            lm.unpadding(d, x, y, pad, stream=s)
+            assert torch.equal(d[:y * x], src)
+            assert not d[y * x:].any()
+
+    _threads(20, work)
+
+
+def test_padding_about_the_kept_flags():
+    """Calls with a task less and more than a kept block has words for, and
+    small ones between them; and the call after one that timed out, whose block
+    is not used again."""
+    task = 16 * 1024
+    small = torch.zeros(1010 * 600, dtype=torch.int32, device="cuda")
+    for tasks in (16 * 1024 - 2, 16 * 1024 - 1, 16 * 1024 - 2, 20000):
+        pad = 4096  # one row of floats is one task
+        x = pad - 3
+        d = torch.zeros(tasks * pad, dtype=torch.int32, device="cuda")
+        src = torch.randint(1, 1 << 30, (tasks * x,), dtype=torch.int32,
+                            device="cuda")
+        assert d.numel() * 4 == tasks * task
+        d[:tasks * x] = src
+        lm.padding(d, x, tasks, pad)
+        assert torch.equal(d.view(tasks, pad)[:, :x], src.view(tasks, x))
+        assert not d.view(tasks, pad)[:, x:].any()
+        small.fill_(7)
+        lm.padding(small, 1000, 600, 1010)
+        assert int(small.sum()) == 7 * 1000 * 600
+        assert lm.lib().lm_debug_pad_stall(None, small.data_ptr(), 4, 1000, 600,
+                                           1010, 0, 3, 20_000_000) is True
+        assert "timed out" in lm.last_error()
+        lm.unpadding(d, x, tasks, pad)
+        assert torch.equal(d[:tasks * x], src)
+        assert not d[tasks * x:].any()
+        del d, src
