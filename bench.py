@@ -41,11 +41,11 @@ CONFIG = {
     "l2": "inputs larger than L2 (805 MB vs 126 MB); no flush needed",
     "steps_alternate": "(16384,12289) then (12289,16384)",
 }
-# DRAM traffic of the dominant kernel per launch (dram__bytes_read.sum +
-# dram__bytes_write.sum), from one ncu capture of k_wave on the forward
-# 100(16384, 12289) fp32 call (profiles/wave_100_16384x12289_f32.txt): 809.6 MB
-# read + 751.3 MB written.
-NCU_TRAFFIC = {"wave": 1560905984}
+# DRAM traffic of each kernel of a step per launch (dram__bytes_read.sum +
+# dram__bytes_write.sum), from one ncu capture of the forward 100(16384, 12289)
+# fp32 call (profiles/wave_100_16384x12289_f32.txt): 809.6 MB read + 751.3 MB
+# written, and 428.1 MB + 373.9 MB.
+NCU_TRAFFIC = {"wave": 1560905984, "suffix_copy": 802000000}
 
 
 def peak_hbm():
@@ -328,13 +328,18 @@ def run_ours(args, ws, rank, local):
 
     value = aggregate_rate(ws, 2.0 * PAYLOAD, args.steps, ms)
     peak, peak_kind = peak_hbm()
-    dom = max(prof.items(), key=lambda kv: kv[1][1]) if prof else None
+    # a step is one conversion by all of its kernels together: their time is
+    # what the 2 x payload of a transposition is set against
     roof = None
-    if dom:
-        name, (n, tot) = dom
-        per = tot / n
+    if prof:
+        names = sorted(prof, key=lambda k: -prof[k][1])
+        n = sum(v[0] for v in prof.values())
+        per = sum(v[1] for v in prof.values()) / args.steps
         achieved = 2.0 * PAYLOAD / (per / 1e3) / 1e9
-        tr = NCU_TRAFFIC.get(name)
+        name = "+".join(names)
+        tr = None
+        if all(k in NCU_TRAFFIC and prof[k][0] == args.steps for k in names):
+            tr = sum(NCU_TRAFFIC[k] for k in names)
         roof = {"bound": "hbm", "achieved": round(achieved, 1),
                 "peak": peak, "unit": "GB/s",
                 "frac": round(achieved / peak, 4), "traffic": tr,
@@ -344,7 +349,7 @@ def run_ours(args, ws, rank, local):
                                  "same %d steps (%.4f ms per step with the "
                                  "events)" % (args.steps,
                                               ms_prof / args.steps),
-                "algorithmic_bytes_per_launch": 2 * PAYLOAD,
+                "algorithmic_bytes_per_step": 2 * PAYLOAD,
                 "peak_kind": peak_kind,
                 "kernels": {k: {"launches": v[0], "ms": round(v[1], 3)}
                             for k, v in prof.items()}}
