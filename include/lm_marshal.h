@@ -30,8 +30,12 @@
  *         transposed out of place, then copied back): the payload's size
  *         and a little more (the ordered form of several instances: one
  *         instance's size);
+ *       the stash plan (100s on units of several elements under 128 bytes that
+ *         are no whole 16-byte vectors, and tall matrices of half-words): about
+ *         half the payload, and 8 bytes per row kept for the first 16 shapes;
  *       walks (100s on units of 128 bytes and more): an eighth of the
- *         payload and a list of the cycles' segments;
+ *         payload, and a list of the cycles that hold no segment's start (2
+ *         bytes per unit) kept for the first 64 shapes and 256 MB;
  *       padding: 4 bytes per task of up to 16 KB, up to 16 blocks of 64 KB
  *         kept per device until lm_marshal_finalize;
  *     payloads that fit the shared memory of all SMs (about 30 MB on GB300)

@@ -82,14 +82,16 @@ struct BJob {
   // staged form, b == 1 and 1- or 2-byte elements: staged rows start on
   // 32-bit words and output vectors on 16 bytes (store_b1_vec applies);
   // else vbc = the widest output vector (16, 8 or 4 bytes; 16 for 4- and
-  // 8-byte elements) the output rows allow (store_b1_vecc), 0 for none; vrw = staged rows per output vector
-  // of either store (their groups are shifted in the stage), 0 for none
+  // 8-byte elements) the output rows allow (store_b1_vecc), 0 for none; vrw =
+  // staged rows per output vector of either store (their groups are shifted
+  // in the stage), 0 for none
   uint32_t vb1, vbc, vrw;
-  // 1- and 2-byte elements whose output rows start anywhere: ragged 1 =
-  // store_b1_ragged (blocks stage `extra` rows more than S), 2 =
-  // store_b1_flat (blocks of whole columns), 0 = none; contig = blocks of
-  // whole rows staged as the one range that they are, row r at r * row
-  // bytes (2: with 16 bytes after each 16/e rows); tab = words of a block's table of row offsets
+  // elements whose output rows start anywhere: ragged 1 = store_b1_ragged, or
+  // store_b1_ragw for 4 and 8 bytes (blocks stage `extra` rows more than S, one
+  // less than a vector holds), 2 = store_b1_flat (blocks of whole columns of
+  // 1- and 2-byte elements), 0 = none; contig = blocks of whole rows staged as
+  // the one range that they are, row r at r * row bytes (2: with 16 bytes after
+  // each 16/e rows); tab = words of a block's table of row offsets
   uint8_t ragged, contig;
   uint16_t extra;
   uint32_t tab;
@@ -1444,11 +1446,9 @@ __device__ void gather_store(const BJob &j, uint32_t q, const unsigned char *buf
 // Persistent: every CTA walks blocks (claimed item by item from the work
 // counter) with two shared-memory stages, loading block n+1 by bulk copies
 // (issued by all warps) while it writes block n.
-// MB: CTAs per SM the registers are sized for.  Three suit the mixed
-// batches and 1-, 4- and 8-byte blocks; 2-byte blocks run 0-3 % faster with
-// the registers of two (staged 100s of 2-byte elements, 4096 x 32768:
-// gather 0.0933 vs 0.0963 ms; 500 x 268435: 0.161 vs 0.167 ms; 1-byte
-// 16384 x 16384 the other way: 0.126 vs 0.121 ms).
+// MB: CTAs per SM the registers are sized for: three, which with the stores of
+// one element width alone (ES: one job's, from the parameters) hold all of them,
+// and with every width's suit the mixed batches.
 // RAG: with the code of ragged blocks and of rows staged as one range (in a
 // kernel of its own: alone it has the registers of three CTAs, but not beside
 // the other items of a batch: 697 us with two, 715 with three).
@@ -2714,8 +2714,12 @@ __global__ void __launch_bounds__(kStageThreads, MB) k_wave(const __grid_constan
       }
     __syncthreads();  // staged for everyone, and its place is free
     if (s_dead) break;
-    // (relaxed: the copies have completed, and a release would wait for this
-    // thread's stores of the last block)
+    // (relaxed: a release would wait for this thread's stores of the last block,
+    // 25 % slower.  What it has to order are this block's reads before another
+    // CTA's stores over the same place, and those reads are over: the bytes that
+    // they returned are in shared memory, as the barrier has seen, before this
+    // thread gets here, and no later store can change them.  No CTA reads what
+    // another has stored.)
     if (threadIdx.x == 0) red_relaxed_gpu(done + fdiv(s, g.div_group), 1u);
     const unsigned char *buf = smem + (size_t)st * g.stage_bytes;
     const GBlock k = gather_decode<RAG>(g.job, q);

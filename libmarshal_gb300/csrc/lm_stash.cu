@@ -7,10 +7,12 @@
 // payload bytes).  This file implements a streaming alternative that moves
 // 3 x payload bytes and only touches memory in >= 128-byte runs.  The ordered
 // form (k_wave, lm_batch.cu) moves as much with blocks by ticket and is as fast
-// or faster (16384 x 12289 floats 389 us here, 390 there; 32768 x 16000 doubles
-// 2555 and 1896), so the planner comes here where that form's scratch, the
-// payload's size, cannot be had (the stash is half of it), and for tall
-// matrices of unaligned half-words (28775 x 13530: 443 and 476 us).
+// or faster for units of one element and of whole vectors (16384 x 12289 floats
+// 389 us here, 390 there; 32768 x 16000 doubles 2555 and 1896).  The planner
+// comes here for other units of several elements, which its blocks write one
+// element at a time (15001 x 1704 of 12 bytes 173 us here, 237 there), for tall
+// matrices of unaligned half-words (28775 x 13530 443 and 478), and where that
+// form's scratch, the payload's size, cannot be had (the stash is half of it).
 //
 //   [A][B] units -> [B][A].  Destination rows are produced in groups of g
 //   (one group = g source columns, a column strip of the source) in order

@@ -24,8 +24,8 @@
 // Bound by DRAM at random lines: 100(24, 187500) of 128-byte units (576 MB)
 // 222 us = 5.2 TB/s (the staged form, 4 x payload: 368 us = 3.1), 100(24,
 // 20001) of 1 KB units 179 us = 5.5 TB/s (cycle following with done bits: 262
-// us).  m = 8: the starts cost 3/8 payload more (written, read back, mostly
-// from L2), but segments of 8 positions on average (their lengths are
+// us).  m = 8: the starts cost a quarter of the payload more (read and written
+// once more; the read back stands for that of their places), but segments of 8 positions on average (their lengths are
 // geometric, the longest about m * ln(segments)) leave a short tail: m = 4 /
 // 8 / 16 / 32 / 64 took 281 / 222 / 228 / 270 / 520 us on the first shape.
 // K = 8 loads in flight at 3 CTAs per SM (80 registers, no spills); K = 4, 6
@@ -276,7 +276,8 @@ bool walk_args(const void *buf, uint64_t T, uint64_t a, uint64_t B, uint64_t U,
   // units of whole 16-byte vectors.  Moved one at a time, smaller units or
   // ones that straddle lines fetch more than they hold: 64 bytes 2.4-3.1
   // TB/s, 80 1.8, 112 2.2, 144 2.5, 208 3.2, 128 and 192 and more in whole
-  // half lines 4.4-5.6, against 2.9-3.1 of the forms that take them else
+  // half lines 4.4-5.6, against 2.9-3.1 of the staged form (walk_by_lines has
+  // the line against the ordered one)
   if (T == 0 || a < 2 || B < 2 || (U != 128 && U < 192) || U % 16 ||
       ((uintptr_t)buf & 15))
     return false;
